@@ -205,6 +205,13 @@ int tape_prunable(const cc_optape* t) {
   return mode == CC_COMB_MIN ? 1 : 2;
 }
 
+// 1 for a tape without smooth minima: one primitive's value, negated or not, is the body's everywhere.
+int tape_select(const cc_optape* t) {
+  for (int i = 0; i < t->n_ops; ++i)
+    if (t->ops[i].combine == CC_COMB_SMIN) return 0;
+  return 1;
+}
+
 // A deeper slab keeps a few more spheres per cell but bounds the union less often. On the 64-sphere
 // cloud (radii U[0.02, 0.08]) the Float32 update was fastest at 16 layers at 512^3 (3.27 ms; 8:
 // 3.31, 32: 3.50) and at 8 at 256^3 (0.676 ms; 16: 0.696, 4: 0.698): the same thickness in space,
@@ -252,6 +259,7 @@ cc_status upload_tape(cc_handle* h, const cc_optape* t, int dim, cudaStream_t s,
   out->n_params = np;
   out->bytes_len = int(bytes);
   out->prunable = cci::tape_prunable(t);
+  out->select = cci::tape_select(t);
   return CC_OK;
 }
 

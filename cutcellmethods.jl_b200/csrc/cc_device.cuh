@@ -619,6 +619,226 @@ struct PruneSmem {
 };
 
 // ---------------------------------------------------------------------------------------------
+// The value and gradient of a body at a cell centroid, with the gradient formed only where it is
+// used. Evaluating the whole tape on duals pays every primitive's gradient (three divisions for a
+// sphere) at every point; a hard combinator (MIN, MAX, SUB, NEG) only ever selects one primitive's.
+
+// A sphere's offset from its centre and its length at one point, from which value and gradient follow.
+template <class T>
+struct SphereAt {
+  T d[3], s;
+};
+template <class T>
+__device__ __forceinline__ T sphere_at(const T* __restrict__ p, const T x[3], SphereAt<T>& h) {
+  T c[4];
+  ldq(p, c);
+  h.d[0] = x[0] - c[0];
+  h.d[1] = x[1] - c[1];
+  h.d[2] = x[2] - c[2];
+  T u = h.d[0] * h.d[0];
+  u = u + h.d[1] * h.d[1];
+  u = u + h.d[2] * h.d[2];
+  h.s = dsqrt(u);
+  return h.s - c[3];
+}
+// The dual arithmetic of tape_prim's sphere on unit seeds: u's gradient is d + d per axis (the
+// other axes add signed zeros, which change no bit of a sum with a value of +0 or larger magnitude;
+// x - c is never -0 for the centroid of a cell), over 2 s.
+template <class T>
+__device__ __forceinline__ void sphere_grad(const SphereAt<T>& h, T g[3]) {
+  const T two_s = T(2) * h.s;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) g[a] = (h.d[a] + h.d[a]) / two_s;
+}
+
+// A box's value and gradient, as tape_prim forms them on unit seeds: outside, the offset beyond the
+// box over its length (the final + 0 is the inside part's gradient); inside, 0 / 0 on every axis.
+template <class T>
+__device__ __forceinline__ Dual<T, 3> box_dual(const T* __restrict__ p, const T x[3]) {
+  T c[8];
+  ldq(p, c);
+  ldq(p + 4, c + 4);
+  T sg[3], q[3], qa[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const T d = x[a] - c[a];
+    sg[a] = d > T(0) ? T(1) : (d < T(0) ? T(-1) : T(0));
+    q[a] = dabs(d) - c[3 + a];
+    qa[a] = q[a] > T(0) ? q[a] : T(0);
+  }
+  T u = qa[0] * qa[0];
+  u = u + qa[1] * qa[1];
+  u = u + qa[2] * qa[2];
+  const T s = dsqrt(u), two_s = T(2) * s;
+  T m = q[0];
+  m = q[1] > m ? q[1] : m;
+  m = q[2] > m ? q[2] : m;
+  Dual<T, 3> r;
+  r.v = s + (m < T(0) ? m : T(0));
+#pragma unroll
+  for (int a = 0; a < 3; ++a) r.g[a] = (q[a] > T(0) ? sg[a] * qa[a] + qa[a] * sg[a] : T(0)) / two_s + T(0);
+  return r;
+}
+
+// One primitive's dual at the point x (unit seeds).
+template <class T>
+__device__ __forceinline__ Dual<T, 3> prim_dual(const cc_op op, const T* __restrict__ p, const T x[3]) {
+  if (op.opcode == CC_OP_SPHERE) {
+    SphereAt<T> h;
+    Dual<T, 3> r;
+    r.v = sphere_at<T>(p + op.poff, x, h);
+    sphere_grad<T>(h, r.g);
+    return r;
+  }
+  if (op.opcode == CC_OP_BOX) return box_dual<T>(p + op.poff, x);
+  Dual<T, 3> xd[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    xd[a].v = x[a];
+#pragma unroll
+    for (int b = 0; b < 3; ++b) xd[a].g[b] = a == b ? T(1) : T(0);
+  }
+  return tape_prim<T, 3, Dual<T, 3>>(op, p, xd);
+}
+
+// A tape without smooth minima: its value at x is one primitive's, negated or not, and so is its
+// gradient. The stack carries values with the op they came from; the dual of that one op is formed
+// at the end. The selections compare the same values as on duals, so the result is the same bits.
+template <class T>
+__device__ __forceinline__ Dual<T, 3> tape_eval_select(const STape<T>& t, const T x[3]) {
+  constexpr int NEG = 1 << 16;
+  T acc = T(0), sv[CC_TAPE_MAX_STACK];
+  int who = 0, sw[CC_TAPE_MAX_STACK], sp = 0;
+  bool have = false;
+  for (int i = 0; i < t.n_ops; ++i) {
+    const cc_op op = t.ops[i];
+    T v;
+    int w = i;
+    if (op.opcode == CC_OP_NONE) {
+      if (op.combine == CC_COMB_NEG) { acc = -acc; who ^= NEG; continue; }
+      v = acc;
+      w = who;
+      --sp;
+      acc = sv[sp];
+      who = sw[sp];
+    } else {
+      v = tape_prim<T, 3, T>(op, t.p, x);
+    }
+    bool take = true;
+    if (op.combine == CC_COMB_PUSH) {
+      if (have) { sv[sp] = acc; sw[sp] = who; ++sp; }
+      have = true;
+    } else if (op.combine == CC_COMB_MIN) {
+      take = v < acc;
+    } else if (op.combine == CC_COMB_MAX) {
+      take = v > acc;
+    } else {  // SUB
+      v = -v;
+      w ^= NEG;
+      take = v > acc;
+    }
+    if (take) { acc = v; who = w; }
+  }
+  Dual<T, 3> r = prim_dual<T>(t.ops[who & (NEG - 1)], t.p, x);
+  if (who & NEG) r = -r;
+  return r;
+}
+
+// ---------------------------------------------------------------------------------------------
+// One warp prunes a union (mode 1) or smooth union (mode 2) of spheres to a box of its own, as
+// prune_union does for a CTA: a sphere stays unless its smallest value over the box exceeds every
+// value the running minimum can take there (mode 2: by k, so that the smooth step returns its
+// input). Bounds are formed in Float32 whatever T is; the margin, 2^-18 of every magnitude involved
+// (`mag`: the grid's coordinates, plus the sphere's own), is at least eight times their rounding and
+// that of the coordinates and of T's evaluation. A NaN or infinite bound keeps its sphere. Writes the
+// kept spheres in op order, poff | kparam << 16, to `out` (n_ops entries) and returns their number;
+// low and up receive the smallest lower and upper bound over the spheres.
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float r;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+template <class T>
+__device__ __forceinline__ int prune_warp(const STape<T>& t, int mode, const float lo[3], const float hi[3], float mag,
+                                          unsigned* out, float& low, float& up) {
+  const int lane = threadIdx.x & 31, n = t.n_ops;
+  const float big = __int_as_float(0x7f800000);
+  auto bounds = [&](int i, float& l, float& u) {
+    T c[4];
+    ldq(t.p + t.ops[i].poff, c);
+    float dmin2 = 0.0f, dmax2 = 0.0f, m = mag + fabsf(float(c[3]));
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const float ca = float(c[a]);
+      const float below = lo[a] - ca, above = ca - hi[a];
+      const float dn = fmaxf(fmaxf(below, above), 0.0f), dx = fmaxf(fabsf(below), fabsf(above));
+      dmin2 += dn * dn;
+      dmax2 += dx * dx;
+      m += fabsf(ca);
+    }
+    const float far = sqrt_approx(dmax2), margin = 0x1p-18f * (m + far);
+    l = sqrt_approx(dmin2) - float(c[3]) - margin;
+    u = far - float(c[3]) + margin;
+  };
+  auto warp_min = [](float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+  };
+  int kept = 0;
+  float running = big;  // mode 1: the least upper bound of all; mode 2: of the spheres so far
+  low = big;
+  float l0 = big, u0 = big;
+  if (mode == 1) {
+    for (int i = lane; i < n; i += 32) {
+      float l, u;
+      bounds(i, l, u);
+      if (i < 32) { l0 = l; u0 = u; }
+      running = fminf(running, u);
+      low = fminf(low, l);
+    }
+    running = warp_min(running);
+  }
+  for (int base = 0; base < n; base += 32) {
+    const int i = base + lane;
+    float l = l0, u = u0;
+    if (i < n && (base > 0 || mode != 1)) bounds(i, l, u);
+    bool keep = false;
+    if (mode == 1) {
+      keep = i < n && !(l > running);
+    } else {
+      if (i >= n) { l = big; u = big; }
+      low = fminf(low, l);
+      float before = u;  // inclusive prefix minimum over the lanes, then made exclusive
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float v = __shfl_up_sync(0xffffffffu, before, o);
+        if (lane >= o) before = fminf(before, v);
+      }
+      const float all = __shfl_sync(0xffffffffu, before, 31);
+      before = __shfl_up_sync(0xffffffffu, before, 1);
+      before = fminf(lane == 0 ? big : before, running);
+      if (i < n) {
+        const float k = float(t.p[t.ops[i].kparam]);
+        const float km = 0x1p-18f * (fabsf(k) + fabsf(before) + fabsf(l) + mag);
+        keep = i == 0 || !(l >= before + k + km);
+      }
+      running = fminf(running, all);
+    }
+    const unsigned b = __ballot_sync(0xffffffffu, keep);
+    if (keep) {
+      const cc_op op = t.ops[i];
+      out[kept + __popc(b & ((1u << lane) - 1u))] = unsigned(op.poff) | (unsigned(op.kparam) << 16);
+    }
+    kept += __popc(b);
+  }
+  __syncwarp();
+  low = warp_min(low);
+  up = running;
+  return kept;
+}
+
+// ---------------------------------------------------------------------------------------------
 // CartesianMeshes stand-ins: node and centroid coordinates, the plane-cube clip.
 template <class T> __device__ __forceinline__ T node_coord(T x0, T d, long long i) { return x0 + T(i) * d; }
 template <class T> __device__ __forceinline__ T centroid_coord(T x0, T d, long long i) {

@@ -41,6 +41,7 @@ struct DevTape {
   int n_params;
   int bytes_len;
   int prunable = 0;  // 1: a union (MIN) of spheres, 2: a smooth union (SMIN) of spheres; see prune_union
+  int select = 0;    // no smooth minimum: value and gradient are one primitive's (tape_eval_select)
   int slab = 8;      // the 3D PLIC passes' pruning slab in cell layers (prune_slab)
 };
 
@@ -126,6 +127,7 @@ template <class T>
 size_t pack_tape(const cc_optape* t, int dim, unsigned char* out, int* n_params);
 size_t tape_pack_capacity();
 int tape_prunable(const cc_optape* t);
+int tape_select(const cc_optape* t);
 
 // Release the contour a marching-squares handle holds (ms_mesh.cu).
 void free_ms_mesh(cc_handle* h);

@@ -317,16 +317,6 @@ __global__ void __launch_bounds__(NT, 6) plic_face_kernel(const DevGrid<T> g, co
   }
 }
 
-// What the fit records per cell for the 3D face pass (cell_side): -1 when every face_area of the
-// cell's plane is 0, +1 when every one is the full face, 0 when they must be clipped. A valid plane
-// is classified by plane_side; an invalid one has face areas 0 (fraction < 1/2) or full (any other
-// fraction, NaN included), _face_area's rule for an invalid plane.
-template <class T>
-__device__ __forceinline__ int8_t cell_side(bool valid, const T n[3], T a, T frac) {
-  if (!valid) return frac < T(0.5) ? int8_t(-1) : int8_t(1);
-  return int8_t(plane_side<T>(n, a));
-}
-
 // The resolved faces in 3D, marching z: a CTA owns a column of FZ_X x FZ_Y cells and FZ_KZ slices.
 // Per slice it forms the next slice's one-sided fractions (area / full face, frac_of; whose -z face
 // is this slice's +z neighbour) and this slice's x and y halo, then resolves the slice and writes
@@ -513,57 +503,169 @@ __global__ void __launch_bounds__(NT, MX ? 4 : 5) plic_face_z_kernel(const DevGr
   }
 }
 
-// The fit pass in 3D, marching z: a CTA owns a column of FZ_X x FZ_Y cells and FZ_KZ slices, and
-// prunes a union of spheres once per slab of tape.slab slices (the box of the slab's centroids;
-// the depth is chosen on the host from the spheres' radii, prune_slab) instead of once per 256
-// cells. The pruning drops only spheres strictly above the minimum over the box and keeps op
-// order, so the planes are the same bits whatever the depth.
+// What the 3D centroid passes know of a tape: a union (SPHERES) or smooth union (SMOOTH) of spheres,
+// pruned per warp; a tape of hard combinators (SELECT), whose gradient is one primitive's; any other
+// (DUAL), evaluated on duals throughout.
+enum PlaneMode { DUAL = 0, SPHERES = 1, SMOOTH = 2, SELECT = 3 };
 
-// At Float32 a bound of 3 CTAs per SM lets the fit keep its values in registers (62, no spills;
-// 64-sphere cloud at 512^3: 3.64 -> 3.61 ms per update); Float64 keeps the compiler's own choice
-// (a bound of 1 CTA doubled its registers and cost 0.19 ms).
+// A cell plane's box of work for one warp: a row of FZ_X cells, `depth` layers deep.
+template <class T>
+struct RowBox {
+  float lo[3], hi[3], mag;
+  __device__ __forceinline__ RowBox(const DevGrid<T>& g, long long i0, int ni, long long j, long long k0, int nk) {
+    const long long first[3] = {i0, j, k0}, last[3] = {i0 + ni - 1, j, k0 + nk - 1};
+    mag = 0.0f;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      lo[a] = float(g.x0[a] + (T(first[a]) + T(0.5)) * g.d[a]);
+      hi[a] = float(g.x0[a] + (T(last[a]) + T(0.5)) * g.d[a]);
+      mag += fabsf(float(g.x0[a])) + float(g.n[a]) * float(g.d[a]);
+    }
+  }
+};
+
+// The body's value and gradient at the centroid x, by the tape's mode; `list`: the warp's m kept spheres.
+template <class T, int MODE>
+__device__ __forceinline__ Dual<T, 3> centroid_dual(const STape<T>& t, const unsigned* list, int m, const T x[3]) {
+  Dual<T, 3> r;
+  if constexpr (MODE == SPHERES) {
+    SphereAt<T> h;
+    r.v = sphere_at<T>(t.p + (list[0] & 0xffffu), x, h);
+    for (int i = 1; i < m; ++i) {
+      SphereAt<T> w;
+      const T v = sphere_at<T>(t.p + (list[i] & 0xffffu), x, w);
+      if (v < r.v) { r.v = v; h = w; }
+    }
+    sphere_grad<T>(h, r.g);
+  } else if constexpr (MODE == SMOOTH) {
+    // the smooth step returns the smaller value unchanged where the two are k or more apart: then
+    // no gradient is needed yet (`raw`: r is the sphere h, its gradient not formed)
+    SphereAt<T> h;
+    r.v = sphere_at<T>(t.p + (list[0] & 0xffffu), x, h);
+    r.g[0] = r.g[1] = r.g[2] = T(0);
+    bool raw = true;
+    for (int i = 1; i < m; ++i) {
+      const unsigned e = list[i];
+      SphereAt<T> w;
+      Dual<T, 3> v;
+      v.v = sphere_at<T>(t.p + (e & 0xffffu), x, w);
+      const T k = t.p[e >> 16];
+      if (k - dabs(r.v - v.v) > T(0)) {
+        if (raw) sphere_grad<T>(h, r.g);
+        raw = false;
+        sphere_grad<T>(w, v.g);
+        r = tape_combine<T, Dual<T, 3>>(CC_COMB_SMIN, r, v, k);
+      } else if (v.v < r.v) {
+        r.v = v.v;
+        h = w;
+        raw = true;
+      }
+    }
+    if (raw) sphere_grad<T>(h, r.g);
+  } else if constexpr (MODE == SELECT) {
+    r = tape_eval_select<T>(t, x);
+  } else {
+    Dual<T, 3> xd[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      xd[a].v = x[a];
+#pragma unroll
+      for (int b = 0; b < 3; ++b) xd[a].g[b] = a == b ? T(1) : T(0);
+    }
+    r = tape_eval<T, 3, Dual<T, 3>>(t, xd);
+  }
+  return r;
+}
+
+// cell_plane (src/plic/plic.jl:72-88) from the body's dual at the centroid, with the cell's side
+// (cell_side). Where plane_side says that a valid plane misses the cell, gvf3 returns 1 or 0: its
+// alpha is then beyond s or below 0 by far more than the few roundings of its sums.
 template <class T, bool MX>
-__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 3 : 0) plic_fit_z_kernel(const DevGrid<T> g, const DevTape tape, const Cols cols,
-                                                        T* normals, T* intercepts, uint8_t* valid, int8_t* sides) {
+__device__ __forceinline__ PlaneFit<T, 3> plane_of(const Dual<T, 3>& r, T h, int& side) {
+  T s = r.g[0];
+  s = s + r.g[1];
+  s = s + r.g[2];
+  const T a = T(0.5) * s - r.v / h;
+  PlaneFit<T, 3> pl;
+  pl.valid = !(isnan(a) || (r.g[0] == T(0) && r.g[1] == T(0) && r.g[2] == T(0)));
+  if (!pl.valid) {
+    pl.n[0] = pl.n[1] = pl.n[2] = pl.a = T(0);
+    pl.fraction = r.v <= T(0) ? T(1) : T(0);
+    side = T(1) - pl.fraction < T(0.5) ? -1 : 1;
+    return pl;
+  }
+  pl.n[0] = r.g[0];
+  pl.n[1] = r.g[1];
+  pl.n[2] = r.g[2];
+  pl.a = a;
+  side = plane_side<T>(pl.n, a);
+  if (side != 0) pl.fraction = side < 0 ? T(1) : T(0);
+  else pl.fraction = gvf3m<T, MX>(r.g[0], r.g[1], r.g[2], a);
+  return pl;
+}
+
+// The fit pass in 3D: a warp owns a row of FZ_X cells and `depth` layers of it, prunes a union of
+// spheres to that box by itself (no CTA barrier after the tape is loaded) and marches up the layers.
+// Only the selected sphere's gradient is formed. Normals leave through the warp's own staging row so
+// that each store covers whole sectors. Bound by instruction issue (about half of what it was: three
+// divisions and two square roots a cell are left). Fit at 512^3, 64 spheres, against a CTA-wide prune
+// and duals throughout: Float32 1.89 -> 1.04 ms, Float64 3.00 -> 1.68, mixed 1.98 -> 1.07; at 128^3
+// 227 -> 39 us; a smooth blob at 256^3 1.04 -> 0.39 ms; a CSG body at 150 x 97 x 131, Float64, 156 -> 70 us.
+template <class T, bool MX, int MODE>
+__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 2)
+    plic_fit_z_kernel(const DevGrid<T> g, const DevTape tape, const Cols cols, T* __restrict__ normals,
+                      T* __restrict__ intercepts, uint8_t* __restrict__ valid, int8_t* __restrict__ sides, int depth) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ int s_count;
+  __shared__ T s_nrm[NT / 32][3 * FZ_X];
   const STape<T> t = load_tape<T>(tape.bytes, tape.n_ops, tape.n_params, smem);
   __syncthreads();
-  constexpr int X = FZ_X, Y = FZ_Y;
-  const long long n[3] = {g.n[0], g.n[1], g.n[2]};
-  const unsigned ntx = unsigned((n[0] + X - 1) / X), nty = unsigned((n[1] + Y - 1) / Y);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const long long n0 = g.n[0], n1 = g.n[1], n2 = g.n[2];
+  const unsigned ntx = unsigned((n0 + FZ_X - 1) / FZ_X), nty = unsigned((n1 + FZ_Y - 1) / FZ_Y);
   unsigned b = blockIdx.x;
-  const unsigned bx = b % ntx;
+  const long long i0 = (long long)(b % ntx) * FZ_X;
   b /= ntx;
-  const unsigned by = b % nty;
-  b /= nty;
-  const long long i0 = (long long)bx * X, j0 = (long long)by * Y, k0 = (long long)b * FZ_KZ;
-  const long long k1 = k0 + FZ_KZ < n[2] ? k0 + FZ_KZ : n[2];
-  const int q = threadIdx.x;
-  const long long ix = i0 + q % X, jy = j0 + q / X;
-  const bool inxy = ix < n[0] && jy < n[1];
+  const long long j = (long long)(b % nty) * FZ_Y + w, k0 = (long long)(b / nty) * depth;
+  if (j >= n1) return;
+  const int nk = n2 - k0 < depth ? int(n2 - k0) : depth, ni = n0 - i0 < FZ_X ? int(n0 - i0) : FZ_X;
+  unsigned* list = reinterpret_cast<unsigned*>(smem + ((tape.bytes_len + 15) / 16) * 16) + w * tape.n_ops;
+  int m = 0;
+  if constexpr (MODE == SPHERES || MODE == SMOOTH) {
+    const RowBox<T> box(g, i0, ni, j, k0, nk);
+    float low, up;
+    m = prune_warp<T>(t, MODE, box.lo, box.hi, box.mag, list, low, up);
+  }
+  const bool in = lane < ni;
+  T x[3] = {centroid_coord(g.x0[0], g.d[0], i0 + lane), centroid_coord(g.x0[1], g.d[1], j), T(0)};
+  const T kf = T(k0);
+  T* const nrm = s_nrm[w];
   T* vf = static_cast<T*>(cols.vf);
-  const int fit_s = tape.slab > 0 ? tape.slab : 8;
-  for (long long ks = k0; ks < k1; ks += fit_s) {
-    const long long first[3] = {i0, j0, ks};
-    const int ext[3] = {X, Y, fit_s};
-    const STape<T> u = box_tape<T, 3>(t, tape, g, first, ext, smem, &s_count);
-    const long long ke = ks + fit_s < k1 ? ks + fit_s : k1;
-    for (long long k = ks; k < ke; ++k) {
-      if (!inxy) continue;
-      const long long idx[3] = {ix, jy, k};
-      const long long ci = ix + n[0] * (jy + n[1] * k);
-      const PlaneFit<T, 3> pl = cell_plane<T, 3, MX>(u, g, idx);
-      const T frac = T(1) - pl.fraction;
+  const long long nxy = n0 * n1;
+  long long row = i0 + n0 * j + nxy * k0;
+  for (int kk = 0; kk < nk; ++kk, row += nxy) {
+    // T(k) + T(0.5) is T(double(k) + 0.5) while k + 0.5 fits T's mantissa
+    if (sizeof(T) == 8 || k0 < (1 << 22) - FZ_KZ) x[2] = g.x0[2] + ((kf + T(kk)) + T(0.5)) * g.d[2];
+    else x[2] = centroid_coord(g.x0[2], g.d[2], k0 + kk);
+    int side;
+    const PlaneFit<T, 3> pl = plane_of<T, MX>(centroid_dual<T, MODE>(t, list, m, x), g.d[0], side);
+    const T frac = T(1) - pl.fraction;
+    nrm[3 * lane] = pl.n[0];
+    nrm[3 * lane + 1] = pl.n[1];
+    nrm[3 * lane + 2] = pl.n[2];
+    __syncwarp();
+    T* const np = normals + 3 * row;
 #pragma unroll
-      for (int a = 0; a < 3; ++a) normals[3 * ci + a] = pl.n[a];
+    for (int e = 0; e < 3; ++e)
+      if (lane + 32 * e < 3 * ni) np[lane + 32 * e] = nrm[lane + 32 * e];
+    __syncwarp();  // read before the next layer's normals are staged
+    if (in) {
+      const long long ci = row + lane;
       intercepts[ci] = pl.a;
-      valid[ci] = pl.valid ? 1 : 0;
       vf[ci] = frac;
+      valid[ci] = pl.valid ? 1 : 0;
       cols.kind[ci] = frac == T(0) ? 0 : (frac == T(1) ? 1 : 2);
-      sides[ci] = cell_side<T>(pl.valid, pl.n, pl.a, frac);
+      sides[ci] = int8_t(side);
     }
-    __syncthreads();  // the next slab's pruning overwrites the ops this one read
   }
 }
 
@@ -816,39 +918,70 @@ cudaError_t launch_monte_carlo(const DevTape& tape, const double lo[3], const do
   return cudaGetLastError();
 }
 
+namespace {
+
+// Layers per warp of the 3D fit: the pruning slab of a union of spheres, else 16; halved while the
+// launch would leave SMs without their eight CTAs, so that a small grid is not a few long columns.
+template <class T>
+int fit_depth(const DevGrid<T>& g, const DevTape& tape) {
+  int depth = tape.prunable && tape.slab > 0 && tape.slab <= FZ_KZ ? tape.slab : 16;
+  const long long tiles = ((g.n[0] + FZ_X - 1) / FZ_X) * ((g.n[1] + FZ_Y - 1) / FZ_Y);
+  while (depth > 2 && tiles * ((g.n[2] + depth - 1) / depth) < 148 * 8) depth /= 2;
+  return depth;
+}
+
+template <class T, int MODE>
+cudaError_t launch_fit_z(const DevGrid<T>& g, const DevTape& tape, const Cols& cols, T* normals, T* intercepts,
+                         uint8_t* valid, int8_t* sides, bool mx, cudaStream_t s) {
+  const int depth = fit_depth(g, tape);
+  const long long blocks = ((g.n[0] + FZ_X - 1) / FZ_X) * ((g.n[1] + FZ_Y - 1) / FZ_Y) * ((g.n[2] + depth - 1) / depth);
+  if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+  // the tape, then each warp's list of kept spheres
+  const int lists = MODE == SPHERES || MODE == SMOOTH ? (NT / 32) * tape.n_ops * int(sizeof(unsigned)) : 0;
+  const int sm = ((tape.bytes_len + 15) / 16) * 16 + lists;
+  auto run = [&](auto kernel) {
+    if (sm > 40 * 1024) {
+      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+      if (e != cudaSuccess) return e;
+    }
+    kernel<<<unsigned(blocks), NT, sm, s>>>(g, tape, cols, normals, intercepts, valid, sides, depth);
+    return cudaSuccess;
+  };
+  if constexpr (sizeof(T) == 4) {
+    if (mx) return run(plic_fit_z_kernel<T, true, MODE>);
+  }
+  return run(plic_fit_z_kernel<T, false, MODE>);
+}
+
+}  // namespace
+
 template <class T, int D>
 cudaError_t launch_plic(const DevGrid<T>& g, const DevTape& tape, const Cols& cols, T* normals, T* intercepts,
                         uint8_t* valid, int8_t* sides, cudaStream_t s, bool mixed) {
-  if (D == 3 && !sides) return cudaErrorInvalidValue;
   const long long total = g.n[0] * g.n[1] * (D == 3 ? g.n[2] : 1);
-  const int sm = CentroidSmem::of(tape).bytes;
-  if (sm > 48 * 1024) {
+  if constexpr (D == 3) {
+    if (!sides) return cudaErrorInvalidValue;
+    const bool mx = mixed && sizeof(T) == 4;
     cudaError_t e;
-    if constexpr (D == 3) {
-      e = cudaFuncSetAttribute(plic_fit_z_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-      if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(plic_fit_z_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    } else {
-      e = cudaFuncSetAttribute(plic_fit_kernel<T, D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    if (tape.prunable == 1) e = launch_fit_z<T, SPHERES>(g, tape, cols, normals, intercepts, valid, sides, mx, s);
+    else if (tape.prunable == 2) e = launch_fit_z<T, SMOOTH>(g, tape, cols, normals, intercepts, valid, sides, mx, s);
+    else if (tape.select) e = launch_fit_z<T, SELECT>(g, tape, cols, normals, intercepts, valid, sides, mx, s);
+    else e = launch_fit_z<T, DUAL>(g, tape, cols, normals, intercepts, valid, sides, mx, s);
+    if (e != cudaSuccess) return e;
+    const long long zcols = ((g.n[0] + FZ_X - 1) / FZ_X) * ((g.n[1] + FZ_Y - 1) / FZ_Y) * ((g.n[2] + FZ_KZ - 1) / FZ_KZ);
+    if (mx) plic_face_z_kernel<T, true><<<unsigned(zcols), NT, 0, s>>>(g, cols, normals, intercepts, sides);
+    else plic_face_z_kernel<T, false><<<unsigned(zcols), NT, 0, s>>>(g, cols, normals, intercepts, sides);
+  } else {  // 2D works in tiles
+    const int sm = CentroidSmem::of(tape).bytes;
+    if (sm > 48 * 1024) {
+      cudaError_t e = cudaFuncSetAttribute(plic_fit_kernel<T, D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
       if (e == cudaSuccess)
         e = cudaFuncSetAttribute(plic_fit_kernel<T, D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+      if (e != cudaSuccess) return e;
     }
-    if (e != cudaSuccess) return e;
-  }
-  // 3D fit and faces march z, one CTA per FZ_X x FZ_Y x FZ_KZ column; 2D works in tiles
-  const long long zcols = ((g.n[0] + FZ_X - 1) / FZ_X) * ((g.n[1] + FZ_Y - 1) / FZ_Y) * ((g.n[2] + FZ_KZ - 1) / FZ_KZ);
-  if (mixed && sizeof(T) == 4) {
-    if constexpr (D == 3) {
-      plic_fit_z_kernel<T, true><<<unsigned(zcols), NT, sm, s>>>(g, tape, cols, normals, intercepts, valid, sides);
-      plic_face_z_kernel<T, true><<<unsigned(zcols), NT, 0, s>>>(g, cols, normals, intercepts, sides);
-    } else {
+    if (mixed && sizeof(T) == 4) {
       plic_fit_kernel<T, D, true><<<blocks_for(total, 16), NT, sm, s>>>(g, tape, cols, normals, intercepts, valid);
       plic_face_kernel<T, D, true><<<blocks_for(total, 16), NT, 0, s>>>(g, cols, normals, intercepts, valid);
-    }
-  } else {
-    if constexpr (D == 3) {
-      plic_fit_z_kernel<T, false><<<unsigned(zcols), NT, sm, s>>>(g, tape, cols, normals, intercepts, valid, sides);
-      plic_face_z_kernel<T, false><<<unsigned(zcols), NT, 0, s>>>(g, cols, normals, intercepts, sides);
     } else {
       plic_fit_kernel<T, D, false><<<blocks_for(total, 16), NT, sm, s>>>(g, tape, cols, normals, intercepts, valid);
       plic_face_kernel<T, D, false><<<blocks_for(total, 16), NT, 0, s>>>(g, cols, normals, intercepts, valid);
