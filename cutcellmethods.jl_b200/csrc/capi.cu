@@ -386,7 +386,7 @@ cc_status cc_handle_create(int32_t device, int32_t method, int32_t dim, int32_t 
     if (e == cudaSuccess) e = cudaMalloc(&h->cut_count, sizeof(unsigned));
   }
   if (e == cudaSuccess && method == CC_PLIC && dim == 3 && !tree)
-    e = cudaMalloc(&h->plic_sides, size_t(h->n[0] * h->n[1] * h->n[2]));
+    e = cudaMalloc(&h->plic_sides, size_t(h->n[0] * h->n[1]) * size_t(h->n[2] + 1) + 64);  // see plic_resolve_kernel
   if (e != cudaSuccess) {
     cc_handle_destroy(h);
     return cuda_fail(e, "cc_handle_create");

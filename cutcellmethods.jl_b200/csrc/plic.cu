@@ -317,198 +317,15 @@ __global__ void __launch_bounds__(NT, 6) plic_face_kernel(const DevGrid<T> g, co
   }
 }
 
-// The resolved faces in 3D, marching z: a CTA owns a column of FZ_X x FZ_Y cells and FZ_KZ slices.
-// Per slice it forms the next slice's one-sided fractions (area / full face, frac_of; whose -z face
-// is this slice's +z neighbour) and this slice's x and y halo, then resolves the slice and writes
-// its rows; this slice's +z fractions are kept as the next slice's -z neighbours. A cell's six
-// one-sided fractions come from its side byte alone (all 0 or all 1) unless the fit marked its
-// plane as crossing the cell, and only then is the plane read and clipped. Every side byte is read
-// once (the column's first slice also reads the one below it), in one barrier per slice, and each
-// one-sided fraction is formed once rather than by both cells of its face. The areas, fractions
-// and resolve expression are plic_face_kernel's, so the faces are the same bits.
+// The 3D passes' row of cells (a warp), rows per CTA, and most layers per warp.
 constexpr int FZ_X = 32, FZ_Y = 8, FZ_KZ = 32;
-
-template <class T, bool MX>
-__global__ void __launch_bounds__(NT, MX ? 4 : 5) plic_face_z_kernel(const DevGrid<T> g, const Cols cols,
-                                                            const T* __restrict__ normals,
-                                                            const T* __restrict__ intercepts,
-                                                            const int8_t* __restrict__ sides) {
-  constexpr int X = FZ_X, Y = FZ_Y, NF = 6;
-  static_assert(X * Y == NT, "one cell of the slice per thread");
-  // One-sided fractions of the slices k % 3, warp-blocked: row w (one warp) keeps its six faces
-  // over its 32 lanes, [w][f][lane], so a warp's own writes stay in its own block.
-  __shared__ __align__(16) T bufs[3][Y][NF][X];
-  __shared__ T prev5[NT];                    // the slice below's +z fractions (own slot only)
-  __shared__ T hx[2][2][Y], hy[2][2][X];     // the x and y halo of slices of each parity
-  const long long n[3] = {g.n[0], g.n[1], g.n[2]};
-  T* ff = static_cast<T*>(cols.ff);
-  const T cs[3] = {g.d[0], g.d[1], g.d[2]};
-  const unsigned ntx = unsigned((n[0] + X - 1) / X), nty = unsigned((n[1] + Y - 1) / Y);
-  unsigned b = blockIdx.x;
-  const unsigned bx = b % ntx;
-  b /= ntx;
-  const unsigned by = b % nty;
-  b /= nty;
-  const long long i0 = (long long)bx * X, j0 = (long long)by * Y, k0 = (long long)b * FZ_KZ;
-  const long long k1 = k0 + FZ_KZ < n[2] ? k0 + FZ_KZ : n[2];
-  const int q = threadIdx.x, lx = q % X, ly = q / X;
-  const long long ix = i0 + lx, jy = j0 + ly;
-  const bool inxy = ix < n[0] && jy < n[1];
-  // the full area of a face of direction f
-  auto full_of = [&](int f) {
-    const int c = f >> 1;
-    return (T(1) * cs[c == 0 ? 1 : 0]) * cs[c == 2 ? 1 : 2];
-  };
-  // the clipped one-sided fraction of face f of cell ci, whose plane crosses it (side 0, so valid)
-  auto clip_frac = [&](const T nn[3], T a, int f) {
-    return frac_of(face_area<T, 3, MX>(nn, a, T(0), true, cs, f), full_of(f));
-  };
-  auto own6 = [&](T (*buf)[NF][X], int side, long long ci) {  // this thread's cell: six one-sided fractions
-    if (side != 0) {
-      const T v = side > 0 ? T(1) : T(0);
-#pragma unroll
-      for (int f = 0; f < NF; ++f) buf[ly][f][lx] = v;
-    } else {
-      const T nn[3] = {normals[3 * ci], normals[3 * ci + 1], normals[3 * ci + 2]};
-      const T a = intercepts[ci];
-#pragma unroll
-      for (int f = 0; f < NF; ++f) buf[ly][f][lx] = clip_frac(nn, a, f);
-    }
-  };
-  // The x and y halo of a slice: 2Y + 2X faces, one on every third thread (all eight warps share
-  // them). Item h: the cell beyond the tile's -x / +x edge at row h (h < 2Y), or beyond its -y / +y
-  // edge at column h - 2Y; the face it shows the tile.
-  constexpr int NH = 2 * Y + 2 * X;
-  static_assert(3 * (NH - 1) < NT, "one halo face per third thread");
-  const int hitem = (q % 3 == 0) ? q / 3 : NH;
-  long long hcell = -1;
-  int hface = 0;
-  if (hitem < 2 * Y) {
-    const int side = hitem / Y, y = hitem % Y;
-    const long long ii = side == 0 ? i0 - 1 : i0 + X, jj = j0 + y;
-    if (ii >= 0 && ii < n[0] && jj < n[1]) hcell = ii + n[0] * jj;
-    hface = side == 0 ? 1 : 0;
-  } else if (hitem < NH) {
-    const int side = (hitem - 2 * Y) / X, x = (hitem - 2 * Y) % X;
-    const long long ii = i0 + x, jj = side == 0 ? j0 - 1 : j0 + Y;
-    if (jj >= 0 && jj < n[1] && ii < n[0]) hcell = ii + n[0] * jj;
-    hface = side == 0 ? 3 : 2;
-  }
-  // a halo cell's face hface (one of the x and y directions), clipped with a constant direction
-  auto halo_frac = [&](int side, long long ci) -> T {
-    if (side != 0) return side > 0 ? T(1) : T(0);
-    const T nn[3] = {normals[3 * ci], normals[3 * ci + 1], normals[3 * ci + 2]};
-    const T a = intercepts[ci];
-    switch (hface) {
-      case 0: return clip_frac(nn, a, 0);
-      case 1: return clip_frac(nn, a, 1);
-      case 2: return clip_frac(nn, a, 2);
-      default: return clip_frac(nn, a, 3);
-    }
-  };
-  const long long nxy = n[0] * n[1];
-  const long long cxy = ix + n[0] * jy;
-  // One barrier per slice. Slice k's fractions live in bufs[(k - k0) % 3]: the next slice's are
-  // written (own slots) while this one's are read, and the buffer they overwrite was last read in
-  // slice k - 2, whose readers all passed the previous barrier. The halo alternates by slice
-  // parity on the same argument. The third buffer, free during slice k (it was slice k - 1's and
-  // becomes slice k + 2's), takes each warp's resolved row in the warp's own block: only that
-  // warp writes or reads its block until it fills it with slice k + 2's fractions itself, and it
-  // copies the row out in between. Side bytes are read a slice ahead of their use.
-  if (inxy) own6(bufs[0], sides[cxy + nxy * k0], cxy + nxy * k0);
-  if (inxy && k0 >= 1) {
-    const long long cb = cxy + nxy * (k0 - 1);
-    const int sb = sides[cb];
-    T v;
-    if (sb != 0) {
-      v = sb > 0 ? T(1) : T(0);
-    } else {
-      const T nn[3] = {normals[3 * cb], normals[3 * cb + 1], normals[3 * cb + 2]};
-      v = clip_frac(nn, intercepts[cb], 5);
-    }
-    prev5[q] = v;
-  }
-  // Slice bookkeeping in 32-bit counters and running offsets: kk = k - k0, kn = n[2] - k0 slices
-  // to the grid's top; the offsets advance one slice (nxy cells) per step.
-  const int nk = int(k1 - k0), kn = int(n[2] - k0);
-  const bool x_lo = ix >= 1, x_hi = ix <= n[0] - 2, y_lo = jy >= 1, y_hi = jy <= n[1] - 2;
-  long long cn = cxy + nxy * (k0 + 1);  // the cell own6 builds next (slice k + 1)
-  long long hc = hcell + nxy * k0;      // this slice's halo cell
-  int snext = (inxy && kn > 1) ? sides[cn] : 0;
-  int hsnext = hcell >= 0 ? sides[hc] : 0;
-  const int lane = q & 31, wrow = q >> 5;
-  static_assert(X == 32, "a warp is one row of the slice");
-  const int rowcells = (int)(n[0] - i0 < X ? n[0] - i0 : X);
-  T* frow = ff + NF * (i0 + n[0] * (jy + n[1] * k0));
-  const long long fstep = NF * nxy;
-  int r3 = 0;
-  for (int kk = 0; kk < nk; ++kk) {
-    const int par = kk & 1;
-    T (*cur)[NF][X] = bufs[r3];
-    T (*nxt)[NF][X] = bufs[r3 == 2 ? 0 : r3 + 1];
-    T* const res = &bufs[r3 == 0 ? 2 : r3 - 1][wrow][0][0];  // this warp's row, cell-major
-    T (*hxp)[Y] = hx[par];
-    T (*hyp)[X] = hy[par];
-    const int scur = snext, hscur = hsnext;
-    if (inxy && kk + 2 < kn) snext = sides[cn + nxy];
-    if (hcell >= 0 && kk + 1 < nk) hsnext = sides[hc + nxy];
-    if (inxy && kk + 1 < kn) own6(nxt, scur, cn);
-    if (hcell >= 0) {
-      const T v = halo_frac(hscur, hc);
-      if (hitem < 2 * Y) hxp[hitem / Y][hitem % Y] = v;
-      else hyp[(hitem - 2 * Y) / X][(hitem - 2 * Y) % X] = v;
-    }
-    cn += nxy;
-    hc += nxy;
-    __syncthreads();
-    if (inxy) {
-      const bool lo[3] = {x_lo, y_lo, k0 + kk >= 1}, hi[3] = {x_hi, y_hi, kk + 1 < kn};
-#pragma unroll
-      for (int f = 0; f < NF; ++f) {
-        const int c = f >> 1;
-        const T mine = cur[ly][f][lx];
-        T r;
-        if ((f & 1) == 0) {
-          const bool has = lo[c];
-          T below = T(0);
-          if (has) below = c == 0 ? (lx > 0 ? cur[ly][1][lx - 1] : hxp[0][ly])
-                                  : c == 1 ? (ly > 0 ? cur[ly - 1][3][lx] : hyp[0][lx]) : prev5[q];
-          r = has ? (below + mine) * T(0.5) : mine;
-        } else {
-          const bool has = hi[c];
-          T above = T(0);
-          if (has) above = c == 0 ? (lx < X - 1 ? cur[ly][0][lx + 1] : hxp[1][ly])
-                                  : c == 1 ? (ly < Y - 1 ? cur[ly + 1][2][lx] : hyp[1][lx]) : nxt[ly][4][lx];
-          r = has ? (mine + above) * T(0.5) : mine;
-        }
-        res[lx * NF + f] = r;
-      }
-    }
-    __syncwarp();
-    // the warp's row leaves whole (16-byte vectors where the row is full and aligned)
-    if (jy < n[1]) {
-      constexpr int RV = X * NF * int(sizeof(T)) / 16;
-      const T* src = res;
-      if (rowcells == X && (reinterpret_cast<uintptr_t>(frow) & 15u) == 0) {
-        for (int v = lane; v < RV; v += 32)
-          reinterpret_cast<uint4*>(frow)[v] = reinterpret_cast<const uint4*>(src)[v];
-      } else {
-        for (int e = lane; e < rowcells * NF; e += 32) frow[e] = src[e];
-      }
-    }
-    frow += fstep;
-    if (inxy) prev5[q] = cur[ly][5][lx];
-    __syncwarp();  // every lane has copied the row out before any writes the next slice's fractions here
-    r3 = r3 == 2 ? 0 : r3 + 1;
-  }
-}
 
 // What the 3D centroid passes know of a tape: a union (SPHERES) or smooth union (SMOOTH) of spheres,
 // pruned per warp; a tape of hard combinators (SELECT), whose gradient is one primitive's; any other
 // (DUAL), evaluated on duals throughout.
 enum PlaneMode { DUAL = 0, SPHERES = 1, SMOOTH = 2, SELECT = 3 };
 
-// A cell plane's box of work for one warp: a row of FZ_X cells, `depth` layers deep.
+// The box of one warp's centroids: a row of ni cells, nk layers.
 template <class T>
 struct RowBox {
   float lo[3], hi[3], mag;
@@ -524,58 +341,91 @@ struct RowBox {
   }
 };
 
-// The body's value and gradient at the centroid x, by the tape's mode; `list`: the warp's m kept spheres.
+// The body's value and gradient at the points of a row's march in z, by the tape's mode; `list`: the
+// warp's m kept spheres. A row that keeps one sphere holds it, with the x and y part of its distance,
+// in registers (ONE).
 template <class T, int MODE>
-__device__ __forceinline__ Dual<T, 3> centroid_dual(const STape<T>& t, const unsigned* list, int m, const T x[3]) {
-  Dual<T, 3> r;
-  if constexpr (MODE == SPHERES) {
-    SphereAt<T> h;
-    r.v = sphere_at<T>(t.p + (list[0] & 0xffffu), x, h);
-    for (int i = 1; i < m; ++i) {
-      SphereAt<T> w;
-      const T v = sphere_at<T>(t.p + (list[i] & 0xffffu), x, w);
-      if (v < r.v) { r.v = v; h = w; }
-    }
-    sphere_grad<T>(h, r.g);
-  } else if constexpr (MODE == SMOOTH) {
-    // the smooth step returns the smaller value unchanged where the two are k or more apart: then
-    // no gradient is needed yet (`raw`: r is the sphere h, its gradient not formed)
-    SphereAt<T> h;
-    r.v = sphere_at<T>(t.p + (list[0] & 0xffffu), x, h);
-    r.g[0] = r.g[1] = r.g[2] = T(0);
-    bool raw = true;
-    for (int i = 1; i < m; ++i) {
-      const unsigned e = list[i];
-      SphereAt<T> w;
-      Dual<T, 3> v;
-      v.v = sphere_at<T>(t.p + (e & 0xffffu), x, w);
-      const T k = t.p[e >> 16];
-      if (k - dabs(r.v - v.v) > T(0)) {
-        if (raw) sphere_grad<T>(h, r.g);
-        raw = false;
-        sphere_grad<T>(w, v.g);
-        r = tape_combine<T, Dual<T, 3>>(CC_COMB_SMIN, r, v, k);
-      } else if (v.v < r.v) {
-        r.v = v.v;
-        h = w;
-        raw = true;
+struct RowBody {
+  const STape<T>& t;
+  const unsigned* list;
+  int m;
+  T x[3];
+
+  __device__ __forceinline__ Dual<T, 3> at(T z) {
+    x[2] = z;
+    Dual<T, 3> r;
+    if constexpr (MODE == SPHERES) {
+      SphereAt<T> h;
+      r.v = sphere_at<T>(t.p + (list[0] & 0xffffu), x, h);
+      for (int i = 1; i < m; ++i) {
+        SphereAt<T> w;
+        const T v = sphere_at<T>(t.p + (list[i] & 0xffffu), x, w);
+        if (v < r.v) { r.v = v; h = w; }
       }
-    }
-    if (raw) sphere_grad<T>(h, r.g);
-  } else if constexpr (MODE == SELECT) {
-    r = tape_eval_select<T>(t, x);
-  } else {
-    Dual<T, 3> xd[3];
+      sphere_grad<T>(h, r.g);
+    } else if constexpr (MODE == SMOOTH) {
+      // the smooth step returns the smaller value unchanged where the two are k or more apart: then
+      // no gradient is needed yet (`raw`: r is the sphere h, its gradient not formed)
+      SphereAt<T> h;
+      r.v = sphere_at<T>(t.p + (list[0] & 0xffffu), x, h);
+      r.g[0] = r.g[1] = r.g[2] = T(0);
+      bool raw = true;
+      for (int i = 1; i < m; ++i) {
+        const unsigned e = list[i];
+        SphereAt<T> w;
+        Dual<T, 3> v;
+        v.v = sphere_at<T>(t.p + (e & 0xffffu), x, w);
+        const T k = t.p[e >> 16];
+        if (k - dabs(r.v - v.v) > T(0)) {
+          if (raw) sphere_grad<T>(h, r.g);
+          raw = false;
+          sphere_grad<T>(w, v.g);
+          r = tape_combine<T, Dual<T, 3>>(CC_COMB_SMIN, r, v, k);
+        } else if (v.v < r.v) {
+          r.v = v.v;
+          h = w;
+          raw = true;
+        }
+      }
+      if (raw) sphere_grad<T>(h, r.g);
+    } else if constexpr (MODE == SELECT) {
+      r = tape_eval_select<T>(t, x);
+    } else {
+      Dual<T, 3> xd[3];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      xd[a].v = x[a];
+      for (int a = 0; a < 3; ++a) {
+        xd[a].v = x[a];
 #pragma unroll
-      for (int b = 0; b < 3; ++b) xd[a].g[b] = a == b ? T(1) : T(0);
+        for (int b = 0; b < 3; ++b) xd[a].g[b] = a == b ? T(1) : T(0);
+      }
+      r = tape_eval<T, 3, Dual<T, 3>>(t, xd);
     }
-    r = tape_eval<T, 3, Dual<T, 3>>(t, xd);
+    return r;
   }
-  return r;
-}
+};
+template <class T>
+struct OneSphere {  // sphere_at's arithmetic, the part that z does not change formed once
+  SphereAt<T> h;
+  T cz, rad, u01;
+  __device__ __forceinline__ OneSphere(const T* p, T x, T y) {
+    T c[4];
+    ldq(p, c);
+    h.d[0] = x - c[0];
+    h.d[1] = y - c[1];
+    u01 = h.d[0] * h.d[0];
+    u01 = u01 + h.d[1] * h.d[1];
+    cz = c[2];
+    rad = c[3];
+  }
+  __device__ __forceinline__ Dual<T, 3> at(T z) {
+    Dual<T, 3> r;
+    h.d[2] = z - cz;
+    h.s = dsqrt(u01 + h.d[2] * h.d[2]);
+    r.v = h.s - rad;
+    sphere_grad<T>(h, r.g);
+    return r;
+  }
+};
 
 // cell_plane (src/plic/plic.jl:72-88) from the body's dual at the centroid, with the cell's side
 // (cell_side). Where plane_side says that a valid plane misses the cell, gvf3 returns 1 or 0: its
@@ -604,19 +454,55 @@ __device__ __forceinline__ PlaneFit<T, 3> plane_of(const Dual<T, 3>& r, T h, int
   return pl;
 }
 
+__device__ __forceinline__ void put_pair(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
+__device__ __forceinline__ void put_pair(double* p, double a, double b) { *reinterpret_cast<double2*>(p) = make_double2(a, b); }
+
+// A cell that its plane crosses, kept until the warp clips its faces; `at`: its first face fraction
+// from the warp's first.
+template <class T>
+struct CrossedCell {
+  T n[3], a;
+  long long at;
+};
+constexpr int CROSSED_MAX = 64;
+
+// The one-sided fractions (face_area over the full face, frac_of) of n crossed cells, one face per lane.
+template <class T, bool MX>
+__device__ __forceinline__ void clip_crossed(const CrossedCell<T>* cells, int n, const DevGrid<T>& g, T* ff) {
+  const T full = (T(1) * g.d[0]) * g.d[0];  // PLIC grids are isotropic
+  for (int e = threadIdx.x & 31; e < 6 * n; e += 32) {
+    const int q = e / 6, f = e - 6 * q;
+    const CrossedCell<T>& c = cells[q];
+    const T np = c.n[f < 2 ? 1 : 0], nq = c.n[f < 4 ? 2 : 1];
+    const T base = c.n[f >> 1] * ((f & 1) ? T(1) : T(0)) - c.a;
+    T area;
+    if (np == T(0) && nq == T(0)) area = base >= T(0) ? full : T(0);
+    else area = full * (T(1) - gvf2m<T, MX>(np, nq, -base));
+    ff[c.at + f] = frac_of(area, full);
+  }
+  __syncwarp();  // the list is filled again
+}
+
 // The fit pass in 3D: a warp owns a row of FZ_X cells and `depth` layers of it, prunes a union of
 // spheres to that box by itself (no CTA barrier after the tape is loaded) and marches up the layers.
 // Only the selected sphere's gradient is formed. Normals leave through the warp's own staging row so
-// that each store covers whole sectors. Bound by instruction issue (about half of what it was: three
-// divisions and two square roots a cell are left). Fit at 512^3, 64 spheres, against a CTA-wide prune
-// and duals throughout: Float32 1.89 -> 1.04 ms, Float64 3.00 -> 1.68, mixed 1.98 -> 1.07; at 128^3
-// 227 -> 39 us; a smooth blob at 256^3 1.04 -> 0.39 ms; a CSG body at 150 x 97 x 131, Float64, 156 -> 70 us.
+// that each store covers whole sectors. A cell's faces are written here too, one-sided: of a cell that
+// its plane misses, all open or all closed; a crossed cell's are clipped from a list, full warps at a
+// time. plic_resolve_kernel then joins the two sides. (A face pass that read every cell's side and
+// resolved all six faces through shared memory took as long as the fit.) Near both its bounds: 85% of
+// the issue slots and 4.6 TB/s of stores. Boxes of 8 x 4 and 16 x 2 columns keep fewer spheres (1.3 and
+// 1.6 instead of 2.0 at 512^3) but their stores cost more: 1.44 and 1.41 against 1.33 ms. CTAs per SM: 4
+// at Float32 (3: 1.36 ms), at Float64 2 with spheres (3: 2.46 against 2.38 ms), else 3 (CSG body at
+// 150 x 97 x 131: 101 against 111 us).
+// Update at 512^3, 64 spheres, kernels: Float32 2.50 -> 1.43 ms, Float64 3.92 -> 2.50, mixed 2.75 -> 1.55;
+// a smooth blob at 256^3 714 -> 455 us; a CSG body at 150 x 97 x 131, Float64, 281 -> 112 us.
 template <class T, bool MX, int MODE>
-__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 2)
+__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : (MODE == SPHERES || MODE == SMOOTH ? 2 : 3))
     plic_fit_z_kernel(const DevGrid<T> g, const DevTape tape, const Cols cols, T* __restrict__ normals,
                       T* __restrict__ intercepts, uint8_t* __restrict__ valid, int8_t* __restrict__ sides, int depth) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ T s_nrm[NT / 32][3 * FZ_X];
+  __shared__ CrossedCell<T> s_crossed[NT / 32][CROSSED_MAX];
   const STape<T> t = load_tape<T>(tape.bytes, tape.n_ops, tape.n_params, smem);
   __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -636,36 +522,200 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 2)
     m = prune_warp<T>(t, MODE, box.lo, box.hi, box.mag, list, low, up);
   }
   const bool in = lane < ni;
-  T x[3] = {centroid_coord(g.x0[0], g.d[0], i0 + lane), centroid_coord(g.x0[1], g.d[1], j), T(0)};
-  const T kf = T(k0);
+  const T x = centroid_coord(g.x0[0], g.d[0], i0 + lane), y = centroid_coord(g.x0[1], g.d[1], j);
+  const T kf = T(k0), z0 = g.x0[2], dz = g.d[2];
+  // T(k) + T(0.5) is T(double(k) + 0.5) while k + 0.5 fits T's mantissa
+  const bool exact_z = sizeof(T) == 8 || k0 < (1 << 22) - FZ_KZ;
   T* const nrm = s_nrm[w];
-  T* vf = static_cast<T*>(cols.vf);
-  const long long nxy = n0 * n1;
-  long long row = i0 + n0 * j + nxy * k0;
-  for (int kk = 0; kk < nk; ++kk, row += nxy) {
-    // T(k) + T(0.5) is T(double(k) + 0.5) while k + 0.5 fits T's mantissa
-    if (sizeof(T) == 8 || k0 < (1 << 22) - FZ_KZ) x[2] = g.x0[2] + ((kf + T(kk)) + T(0.5)) * g.d[2];
-    else x[2] = centroid_coord(g.x0[2], g.d[2], k0 + kk);
-    int side;
-    const PlaneFit<T, 3> pl = plane_of<T, MX>(centroid_dual<T, MODE>(t, list, m, x), g.d[0], side);
-    const T frac = T(1) - pl.fraction;
-    nrm[3 * lane] = pl.n[0];
-    nrm[3 * lane + 1] = pl.n[1];
-    nrm[3 * lane + 2] = pl.n[2];
-    __syncwarp();
-    T* const np = normals + 3 * row;
+  CrossedCell<T>* const crossed = s_crossed[w];
+  int ncrossed = 0;
+  const int cell_of[3] = {lane / 3, (lane + 32) / 3, (lane + 64) / 3};  // the cells of this lane's face pairs
+  const long long nxy = n0 * n1, row = i0 + n0 * j + nxy * k0;
+  // this lane's place in each column, moved up a layer at a time
+  T* np = normals + 3 * row + lane;
+  T* ap = intercepts + row + lane;
+  T* vp = static_cast<T*>(cols.vf) + row + lane;
+  T* fp = static_cast<T*>(cols.ff) + 6 * row;
+  int8_t* kp = cols.kind + row + lane;
+  int8_t* sp = sides + row + lane;
+  uint8_t* okp = valid + row + lane;
+  T* const ff0 = fp;
+  const bool pairs = (reinterpret_cast<uintptr_t>(cols.ff) & (2 * sizeof(T) - 1)) == 0;
+  auto march = [&](auto&& body) {
+    for (int kk = 0; kk < nk; ++kk) {
+      const T z = exact_z ? z0 + ((kf + T(kk)) + T(0.5)) * dz : centroid_coord(z0, dz, k0 + kk);
+      int side;
+      const PlaneFit<T, 3> pl = plane_of<T, MX>(body.at(z), g.d[0], side);
+      const T frac = T(1) - pl.fraction;
+      nrm[3 * lane] = pl.n[0];
+      nrm[3 * lane + 1] = pl.n[1];
+      nrm[3 * lane + 2] = pl.n[2];
+      __syncwarp();
 #pragma unroll
-    for (int e = 0; e < 3; ++e)
-      if (lane + 32 * e < 3 * ni) np[lane + 32 * e] = nrm[lane + 32 * e];
-    __syncwarp();  // read before the next layer's normals are staged
-    if (in) {
-      const long long ci = row + lane;
-      intercepts[ci] = pl.a;
-      vf[ci] = frac;
-      valid[ci] = pl.valid ? 1 : 0;
-      cols.kind[ci] = frac == T(0) ? 0 : (frac == T(1) ? 1 : 2);
-      sides[ci] = int8_t(side);
+      for (int e = 0; e < 3; ++e)
+        if (lane + 32 * e < 3 * ni) np[32 * e] = nrm[lane + 32 * e];
+      __syncwarp();  // read before the next layer's normals are staged
+      if (in) {
+        *ap = pl.a;
+        *vp = frac;
+        *okp = pl.valid ? 1 : 0;
+        *kp = frac == T(0) ? 0 : (frac == T(1) ? 1 : 2);
+        *sp = int8_t(side);
+      }
+      // every face of a cell that its plane misses is open (1) or closed (0), all of it
+      const unsigned open = __ballot_sync(0xffffffffu, side > 0);
+      if (pairs) {
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+          const T v = (open >> cell_of[e]) & 1u ? T(1) : T(0);
+          if (cell_of[e] < ni) put_pair(fp + 2 * (lane + 32 * e), v, v);
+        }
+      } else {
+        for (int e = lane; e < 6 * ni; e += 32) fp[e] = (open >> (e / 6)) & 1u ? T(1) : T(0);
+      }
+      // crossed cells wait until there are enough to clip their faces on full warps
+      const unsigned cross = __ballot_sync(0xffffffffu, in && side == 0);
+      if (cross) {
+        if (in && side == 0) {
+          CrossedCell<T>& c = crossed[ncrossed + __popc(cross & ((1u << lane) - 1u))];
+          c.n[0] = pl.n[0];
+          c.n[1] = pl.n[1];
+          c.n[2] = pl.n[2];
+          c.a = pl.a;
+          c.at = 6 * (lane + nxy * kk);
+        }
+        ncrossed += __popc(cross);
+        __syncwarp();  // also orders the layer's open / closed faces before the clipped ones
+        if (ncrossed > CROSSED_MAX - 32) {
+          clip_crossed<T, MX>(crossed, ncrossed, g, ff0);
+          ncrossed = 0;
+        }
+      }
+      np += 3 * nxy;
+      ap += nxy;
+      vp += nxy;
+      fp += 6 * nxy;
+      kp += nxy;
+      sp += nxy;
+      okp += nxy;
     }
+    clip_crossed<T, MX>(crossed, ncrossed, g, ff0);
+  };
+  if (MODE == SPHERES && m == 1) march(OneSphere<T>(t.p + (list[0] & 0xffffu), x, y));
+  else march(RowBody<T, MODE>{t, list, m, {x, y, T(0)}});
+}
+
+// 0x80 in each byte of x that is zero, nothing elsewhere (no carry crosses a byte: (b & 0x7f) +
+// 0x7f <= 0xfe).
+__device__ __forceinline__ unsigned zero_bytes(unsigned x) {
+  return ~(((x & 0x7f7f7f7fu) + 0x7f7f7f7fu) | x | 0x7f7f7f7fu);
+}
+
+// The resolved faces in 3D (src/plic/cache.jl:118-162). The fit has written every cell's one-sided
+// fractions into its faces; a face between two cells takes their mean, (lower + upper) / 2, which only
+// changes it where one of the two is crossed by its plane (side 0) or their sides differ, about the
+// interface's area. A warp reads 512 side bytes and their +x, +y, +z neighbours' sixteen a lane, lists
+// the cells that own such a face (the upper faces of a cell are its own) in shared memory, and forms
+// the means, one cell per lane, written to both cells. Each face is resolved by its lower cell alone,
+// with the expression and order of the reference, so it is single-valued bit for bit. Bytes compared
+// across a row's or a layer's end, or past the grid (the array is padded by a layer), only list a
+// cell that then turns out to own nothing.
+template <class T>
+__global__ void __launch_bounds__(NT) plic_resolve_kernel(const DevGrid<T> g, T* __restrict__ ff,
+                                                          const int8_t* __restrict__ sides, long long total) {
+  __shared__ uint16_t s_list[NT / 32][512];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const long long n0 = g.n[0], n1 = g.n[1], nxy = n0 * n1;
+  const long long step[3] = {1, n0, nxy};
+  for (long long base = 512 * ((long long)blockIdx.x * (NT / 32) + w); base < total; base += 512LL * gridDim.x * (NT / 32)) {
+    const long long c = base + 16 * lane;
+    unsigned act[4] = {0, 0, 0, 0};
+    int mine = 0;
+    if (c < total) {
+      auto sixteen = [&](long long at, unsigned v[5]) {  // the word-aligned bytes from `at` (a multiple of 16) on
+        const uint4 a = *reinterpret_cast<const uint4*>(sides + at);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+      };
+      unsigned o[5], yz[2][4];
+      sixteen(c, o);
+      o[4] = *reinterpret_cast<const unsigned*>(sides + c + 16);
+#pragma unroll
+      for (int d = 0; d < 2; ++d) {
+        const long long at = c + step[d + 1];
+        const int r = int(at & 15);  // the same for every lane
+        if (r == 0) {
+          sixteen(at, yz[d]);
+        } else {
+          unsigned u[8];
+          sixteen(at - r, u);
+          sixteen(at - r + 16, u + 4);
+          const int q0 = r >> 2, sh = (r & 3) * 8;
+          unsigned v[5];
+#pragma unroll
+          for (int q = 0; q < 5; ++q)
+            v[q] = q0 == 0 ? u[q] : q0 == 1 ? u[q + 1] : q0 == 2 ? u[q + 2 < 8 ? q + 2 : 7] : u[q + 3 < 8 ? q + 3 : 7];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) yz[d][q] = __funnelshift_r(v[q], v[q + 1], sh);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const unsigned x = __funnelshift_r(o[q], o[q + 1], 8);
+        const unsigned differ = (o[q] ^ x) | (o[q] ^ yz[0][q]) | (o[q] ^ yz[1][q]);
+        act[q] = (zero_bytes(differ) ^ 0x80808080u) | zero_bytes(o[q]);
+        mine += __popc(act[q]);
+      }
+    }
+    if (__ballot_sync(0xffffffffu, mine != 0) == 0) continue;
+    int at = mine;  // inclusive sum over the lanes, then this lane's first entry
+#pragma unroll
+    for (int s = 1; s < 32; s <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, at, s);
+      if (lane >= s) at += v;
+    }
+    const int count = __shfl_sync(0xffffffffu, at, 31);
+    at -= mine;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      for (unsigned m = act[q]; m; m &= m - 1) s_list[w][at++] = uint16_t(16 * lane + 4 * q + ((__ffs(m) - 1) >> 3));
+    __syncwarp();
+    for (int e = lane; e < count; e += 32) {
+      const long long ci = base + s_list[w][e];
+      if (ci >= total) continue;
+      long long idx[3];
+      if (total < (1LL << 32)) {
+        const unsigned u = unsigned(ci), a = u / unsigned(n0);
+        idx[0] = u - a * unsigned(n0);
+        const unsigned k = a / unsigned(n1);
+        idx[1] = a - k * unsigned(n1);
+        idx[2] = k;
+      } else {
+        idx[0] = ci % n0;
+        idx[1] = (ci / n0) % n1;
+        idx[2] = ci / nxy;
+      }
+      const int sc = sides[ci];
+      bool own[3];
+      T lower[3], upper[3];
+#pragma unroll
+      for (int ax = 0; ax < 3; ++ax) {
+        own[ax] = idx[ax] + 1 < g.n[ax];
+        if (own[ax]) own[ax] = sc == 0 || sides[ci + step[ax]] != sc;
+        lower[ax] = upper[ax] = T(0);
+        if (own[ax]) {
+          lower[ax] = ff[6 * ci + 2 * ax + 1];
+          upper[ax] = ff[6 * (ci + step[ax]) + 2 * ax];
+        }
+      }
+#pragma unroll
+      for (int ax = 0; ax < 3; ++ax)
+        if (own[ax]) {
+          const T r = (lower[ax] + upper[ax]) * T(0.5);
+          ff[6 * ci + 2 * ax + 1] = r;
+          ff[6 * (ci + step[ax]) + 2 * ax] = r;
+        }
+    }
+    __syncwarp();  // the next 512 cells reuse the list
   }
 }
 
@@ -785,12 +835,6 @@ __device__ __forceinline__ void report_cell(int k, int a, T v, unsigned long lon
   out += k == 1;
   am += a != 0;
   if (k == 2 && v > T(0) && v < vmin) vmin = v;
-}
-
-// 0x80 in each byte of x that is zero, nothing elsewhere (no carry crosses a byte: (b & 0x7f) +
-// 0x7f <= 0xfe).
-__device__ __forceinline__ unsigned zero_bytes(unsigned x) {
-  return ~(((x & 0x7f7f7f7fu) + 0x7f7f7f7fu) | x | 0x7f7f7f7fu);
 }
 
 template <class T>
@@ -968,9 +1012,9 @@ cudaError_t launch_plic(const DevGrid<T>& g, const DevTape& tape, const Cols& co
     else if (tape.select) e = launch_fit_z<T, SELECT>(g, tape, cols, normals, intercepts, valid, sides, mx, s);
     else e = launch_fit_z<T, DUAL>(g, tape, cols, normals, intercepts, valid, sides, mx, s);
     if (e != cudaSuccess) return e;
-    const long long zcols = ((g.n[0] + FZ_X - 1) / FZ_X) * ((g.n[1] + FZ_Y - 1) / FZ_Y) * ((g.n[2] + FZ_KZ - 1) / FZ_KZ);
-    if (mx) plic_face_z_kernel<T, true><<<unsigned(zcols), NT, 0, s>>>(g, cols, normals, intercepts, sides);
-    else plic_face_z_kernel<T, false><<<unsigned(zcols), NT, 0, s>>>(g, cols, normals, intercepts, sides);
+    const long long rows = (total + 512 * (NT / 32) - 1) / (512 * (NT / 32));
+    const unsigned rb = unsigned(rows < 148 * 8 ? rows : 148 * 8);
+    plic_resolve_kernel<T><<<rb, NT, 0, s>>>(g, static_cast<T*>(cols.ff), sides, total);
   } else {  // 2D works in tiles
     const int sm = CentroidSmem::of(tape).bytes;
     if (sm > 48 * 1024) {
