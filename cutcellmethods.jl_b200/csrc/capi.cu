@@ -9,6 +9,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <limits>
 #include <string>
 #include <vector>
 #include <cuda_runtime.h>
@@ -210,6 +211,45 @@ int tape_select(const cc_optape* t) {
   for (int i = 0; i < t->n_ops; ++i)
     if (t->ops[i].combine == CC_COMB_SMIN) return 0;
   return 1;
+}
+
+// A combinator takes one operand's value or a smooth blend whose gradient is a convex combination, so a
+// body's bounds are its primitives' largest. A sphere's and a box's gradient has length 1 (or none,
+// inside a box), a torus's at most its matrix's (Frobenius) norm, a plane's its normal's.
+TapeBounds tape_bounds(const cc_optape* t) {
+  TapeBounds b;
+  const double root3 = std::sqrt(3.0), inf = std::numeric_limits<double>::infinity();
+  for (int i = 0; i < t->n_ops; ++i) {
+    const cc_op& op = t->ops[i];
+    const double* p = t->params + op.poff;
+    double lip = 0, g1 = 0, mag = 0;
+    for (int q = 0; q < prim_params(op.opcode, 3); ++q) mag += std::fabs(p[q]);
+    switch (op.opcode) {
+      case CC_OP_NONE:
+      case CC_OP_CONST: break;
+      case CC_OP_SPHERE:
+      case CC_OP_BOX: lip = 1; g1 = root3; break;
+      case CC_OP_TORUS:
+        for (int q = 3; q < 12; ++q) lip += p[q] * p[q];
+        lip = std::sqrt(lip);
+        g1 = root3 * lip;
+        break;
+      case CC_OP_PLANE:
+        lip = std::sqrt(p[3] * p[3] + p[4] * p[4] + p[5] * p[5]);
+        g1 = std::fabs(p[3]) + std::fabs(p[4]) + std::fabs(p[5]);
+        break;
+      case CC_OP_TRIG:
+        g1 = std::fabs(p[0]) * (std::fabs(p[1]) + std::fabs(p[2]) + std::fabs(p[3]));
+        lip = g1;
+        break;
+      default: lip = g1 = inf;
+    }
+    if (!(lip < inf) || !(g1 < inf) || !(mag < inf)) lip = g1 = inf;  // a NaN parameter too
+    b.lipschitz = lip > b.lipschitz ? lip : b.lipschitz;
+    b.grad1 = g1 > b.grad1 ? g1 : b.grad1;
+    b.mag = mag > b.mag ? mag : b.mag;
+  }
+  return b;
 }
 
 // A deeper slab keeps a few more spheres per cell but bounds the union less often. On the 64-sphere
@@ -590,35 +630,35 @@ cc_status cc_calc_volume(cc_handle* h, const cc_grid* g, const cc_optape* body, 
   if (st != CC_OK) return st;
   DeviceGuard dg(h->device);
   const cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // calc_volume prunes over slabs of 8 layers whatever the body: deeper slabs, which the update's fit
-  // takes for small cells, made the Float64 sum slower (512^3 64-sphere cloud: 3.55 -> 6.37 ms at 16)
   cci::DevTape tape{nullptr, 0, 0, 0};
   double* partial = h->vol_scratch;
   double* res = h->vol_scratch + 2 * cci::calc_volume_blocks();
   cudaError_t e;
   double pd;
+  const cci::TapeBounds tb = g->dim == 3 ? cci::tape_bounds(body) : cci::TapeBounds();
   if (h->prec == CC_F64) {
     if ((st = upload_tape<double>(h, body, g->dim, s, &tape)) != CC_OK) return st;
     const cci::DevGrid<double> dg2 = dev_grid<double>(g);
-    e = g->dim == 3 ? cci::launch_calc_volume<double, 3>(dg2, tape, partial, res, s)
-                    : cci::launch_calc_volume<double, 2>(dg2, tape, partial, res, s);
+    e = g->dim == 3 ? cci::launch_calc_volume<double, 3>(dg2, tape, tb, partial, res, s)
+                    : cci::launch_calc_volume<double, 2>(dg2, tape, tb, partial, res, s);
     pd = dg2.d[0] * dg2.d[1];
     if (g->dim == 3) pd = pd * dg2.d[2];
   } else {
     if ((st = upload_tape<float>(h, body, g->dim, s, &tape)) != CC_OK) return st;
     const cci::DevGrid<float> dg2 = dev_grid<float>(g);
     const bool mx = h->prec == CC_MIXED;
-    e = g->dim == 3 ? cci::launch_calc_volume<float, 3>(dg2, tape, partial, res, s, mx)
-                    : cci::launch_calc_volume<float, 2>(dg2, tape, partial, res, s, mx);
+    e = g->dim == 3 ? cci::launch_calc_volume<float, 3>(dg2, tape, tb, partial, res, s, mx)
+                    : cci::launch_calc_volume<float, 2>(dg2, tape, tb, partial, res, s, mx);
     float pf = dg2.d[0] * dg2.d[1];
     if (g->dim == 3) pf = pf * dg2.d[2];
     pd = pf;
   }
   if (e != cudaSuccess) return cuda_fail(e, "calc_volume launch");
   double sum = 0.0;
-  e = cudaMemcpyAsync(&sum, res, sizeof(double), cudaMemcpyDeviceToHost, s);
+  e = cudaMemcpyAsync(h->rep_host, res, sizeof(double), cudaMemcpyDeviceToHost, s);  // pinned
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_fail(e, "calc_volume");
+  std::memcpy(&sum, h->rep_host, sizeof(double));
   *out = sum * pd;
   return CC_OK;
 }

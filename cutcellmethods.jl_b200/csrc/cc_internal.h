@@ -45,6 +45,14 @@ struct DevTape {
   int slab = 8;      // the 3D PLIC passes' pruning slab in cell layers (prune_slab)
 };
 
+// Bounds of a 3D body over all space: how fast its value can change (the Lipschitz constant), the
+// largest sum of |gradient components|, and the size of its parameters (for rounding margins).
+// Infinite where a primitive has none.
+struct TapeBounds {
+  double lipschitz = 0, grad1 = 0, mag = 0;
+};
+TapeBounds tape_bounds(const cc_optape* t);
+
 // The slab depth, in cell layers, over which the 3D PLIC fit and calc_volume prune a union of
 // spheres of cell size h: about 0.6 of the median radius, rounded to 4, 8, 16 or 32 layers.
 int prune_slab(const cc_optape* t, double h);
@@ -119,7 +127,7 @@ int calc_volume_blocks();
 cudaError_t launch_monte_carlo(const DevTape& tape, const double lo[3], const double hi[3], long long npts,
                                unsigned long long seed, unsigned long long* out, cudaStream_t s);
 template <class T, int D>
-cudaError_t launch_calc_volume(const DevGrid<T>& g, const DevTape& tape, double* partial,
+cudaError_t launch_calc_volume(const DevGrid<T>& g, const DevTape& tape, const TapeBounds& tb, double* partial,
                                double* out, cudaStream_t s, bool mixed = false);
 
 // Op-tape packing (capi.cu): pack a validated host tape for the device (see pack_tape).

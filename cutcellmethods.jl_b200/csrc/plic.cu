@@ -6,6 +6,7 @@
 // (_plic_face_fraction_kernel!, src/plic/cache.jl:118-162): per cell, per face, the mean of the
 // two one-sided candidates evaluated from the two cells' stored planes by the same _face_area
 // (src/plic/apertures.jl:112-125), so both cells of a face compute identical bits.
+#include <cmath>
 #include <cstdint>
 #include "cc_device.cuh"
 #include "cc_internal.h"
@@ -16,6 +17,7 @@ using namespace ccd;
 using cci::Cols;
 using cci::DevGrid;
 using cci::DevTape;
+using cci::TapeBounds;
 
 constexpr int NT = 256;
 constexpr int VOL_BLOCKS = 148 * 8;
@@ -351,6 +353,21 @@ struct RowBody {
   int m;
   T x[3];
 
+  // the value alone
+  __device__ __forceinline__ T value(T z) {
+    x[2] = z;
+    if constexpr (MODE == SPHERES || MODE == SMOOTH) {
+      SphereAt<T> h;
+      T v = sphere_at<T>(t.p + (list[0] & 0xffffu), x, h);
+      for (int i = 1; i < m; ++i) {
+        const T u = sphere_at<T>(t.p + (list[i] & 0xffffu), x, h);
+        v = tape_combine<T, T>(MODE == SPHERES ? CC_COMB_MIN : CC_COMB_SMIN, v, u, MODE == SPHERES ? T(0) : t.p[list[i] >> 16]);
+      }
+      return v;
+    } else {
+      return tape_eval<T, 3, T>(t, x);
+    }
+  }
   __device__ __forceinline__ Dual<T, 3> at(T z) {
     x[2] = z;
     Dual<T, 3> r;
@@ -730,7 +747,30 @@ struct KSum {
   }
 };
 
-// calc_volume, src/volume.jl:29-40: every cell's cell_plane solid fraction, summed.
+// The CTA's sums into out[0..1] (sum, compensation): a butterfly per warp, then the warps in order.
+__device__ __forceinline__ void block_ksum(KSum a, double* out) {
+  __shared__ double s_part[NT / 32][2];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double s = __shfl_down_sync(0xffffffffu, a.s, o), c = __shfl_down_sync(0xffffffffu, a.c, o);
+    a.add(s);
+    a.c += c;
+  }
+  if ((threadIdx.x & 31) == 0) {
+    s_part[threadIdx.x >> 5][0] = a.s;
+    s_part[threadIdx.x >> 5][1] = a.c;
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int w = 1; w < NT / 32; ++w) {
+    a.add(s_part[w][0]);
+    a.c += s_part[w][1];
+  }
+  out[0] = a.s;
+  out[1] = a.c;
+}
+
+// calc_volume, src/volume.jl:29-40: every cell's cell_plane solid fraction, summed (2D).
 template <class T, int D, bool MX>
 __global__ void __launch_bounds__(NT) calc_volume_kernel(const DevGrid<T> g, const DevTape tape, double* partial) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -751,77 +791,147 @@ __global__ void __launch_bounds__(NT) calc_volume_kernel(const DevGrid<T> g, con
     if (idx[0] < n0 && idx[1] < n1 && idx[2] < n2) acc.add(double(cell_plane<T, D, MX>(u, g, idx).fraction));
     __syncthreads();
   }
-  __shared__ double ss[NT], sc[NT];
-  ss[threadIdx.x] = acc.s;
-  sc[threadIdx.x] = acc.c;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    KSum b{0.0, 0.0};
-    double cc = 0.0;
-    for (int i = 0; i < NT; ++i) { b.add(ss[i]); cc += sc[i]; }
-    partial[2 * blockIdx.x] = b.s;
-    partial[2 * blockIdx.x + 1] = b.c + cc;
-  }
+  block_ksum(acc, partial + 2 * blockIdx.x);
 }
 
-// calc_volume in 3D, marching z: persistent CTAs take FZ_X x FZ_Y x FZ_KZ columns and prune a union
-// of spheres once per slab of tape.slab slices, as the 3D fit pass does (the same fractions; the sum
-// is the same compensated accumulation, in another order).
-template <class T, bool MX>
-__global__ void __launch_bounds__(NT) calc_volume_z_kernel(const DevGrid<T> g, const DevTape tape, double* partial) {
+// calc_volume in 3D. Only cells near the interface have a fraction other than 0 or 1: with |grad|_1 <=
+// L1 (the tape's bound), a plane whose value exceeds thr = h L1 / 2 (and 0.1% for rounding) misses its
+// cell, and gvf3 returns 0 or 1; a cell without a valid plane takes its fraction from the value's sign,
+// the same 0 or 1. So the grid is taken in boxes of VX x VY x VZ cells: a warp first evaluates the body at
+// the centres of `group` boxes, a lane each, and settles every box whose value is beyond thr plus what
+// the body can change over the box (its Lipschitz constant, and `margin` for the rounding of values and
+// coordinates); the boxes left are evaluated cell by cell, and the gradient and the clip are formed only
+// where |value| <= thr. Whole cells are counted, partial ones summed compensated in Float64. A tape
+// without a Lipschitz bound settles nothing and every cell takes its plane.
+// Before: every cell's plane on duals, 32 layers of a column one after another (the time of a 64^3
+// grid was that of 256^3), and one thread adding up the CTAs' partials (80 us). 64 spheres, kernels:
+// 256^3 Float64 687 -> 103 us, 64^3 Float64 667 -> 27 us, 512^3 Float32 1906 -> 150 us. Centres in Float32
+// on all lanes, and listing the near cells, took the 256^3 time from 244 to 103 us.
+constexpr int VX = 8, VY = 4, VZ = 8;
+
+template <class T, bool MX, int MODE>
+__global__ void __launch_bounds__(NT) calc_volume_z_kernel(const DevGrid<T> g, const DevTape tape, double* partial,
+                                                           T thr, T beyond, int group) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ int s_count;
   const STape<T> t = load_tape<T>(tape.bytes, tape.n_ops, tape.n_params, smem);
   __syncthreads();
-  constexpr int X = FZ_X, Y = FZ_Y;
-  const long long n[3] = {g.n[0], g.n[1], g.n[2]};
-  const unsigned ntx = unsigned((n[0] + X - 1) / X), nty = unsigned((n[1] + Y - 1) / Y);
-  const unsigned ncol = ntx * nty * unsigned((n[2] + FZ_KZ - 1) / FZ_KZ);
-  const int q = threadIdx.x;
+  __shared__ uint8_t s_near[NT / 32][VX * VY * VZ];
+  static_assert(VX * VY == 32 && VX * VY * VZ <= 256, "a box's cells are numbered in a byte");
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  unsigned* list = reinterpret_cast<unsigned*>(smem + ((tape.bytes_len + 15) / 16) * 16) + w * tape.n_ops;
+  const long long nx = (g.n[0] + VX - 1) / VX, ny = (g.n[1] + VY - 1) / VY, nz = (g.n[2] + VZ - 1) / VZ;
+  const long long boxes = nx * ny * nz;
+  const T h = g.d[0];
   KSum acc{0.0, 0.0};
-  for (unsigned col = blockIdx.x; col < ncol; col += gridDim.x) {
-    unsigned b = col;
-    const unsigned bx = b % ntx;
-    b /= ntx;
-    const unsigned by = b % nty;
-    b /= nty;
-    const long long i0 = (long long)bx * X, j0 = (long long)by * Y, k0 = (long long)b * FZ_KZ;
-    const long long k1 = k0 + FZ_KZ < n[2] ? k0 + FZ_KZ : n[2];
-    const long long ix = i0 + q % X, jy = j0 + q / X;
-    const bool inxy = ix < n[0] && jy < n[1];
-    const int fit_s = tape.slab > 0 ? tape.slab : 8;
-    for (long long ks = k0; ks < k1; ks += fit_s) {
-      const long long first[3] = {i0, j0, ks};
-      const int ext[3] = {X, Y, fit_s};
-      const STape<T> u = box_tape<T, 3>(t, tape, g, first, ext, smem, &s_count);
-      const long long ke = ks + fit_s < k1 ? ks + fit_s : k1;
-      if (inxy)
-        for (long long k = ks; k < ke; ++k) {
-          const long long idx[3] = {ix, jy, k};
-          acc.add(double(cell_plane<T, 3, MX>(u, g, idx).fraction));
+  long long whole = 0;
+  for (long long first = ((long long)blockIdx.x * (NT / 32) + w) * group; first < boxes;
+       first += (long long)gridDim.x * (NT / 32) * group) {
+    // the lane's box: its first cell, and its extents in the grid. Of a union of spheres, all 32 lanes
+    // take part whatever the group, `share` of them on the spheres of one box, in Float32 (the margin
+    // covers that); the first of them answers for the box
+    const int share = MODE == SPHERES ? 32 / group : 1, mine = lane / share;
+    long long i0[3] = {0, 0, 0};
+    int ext[3] = {0, 0, 0};
+    bool open = false;
+    T v = T(0);
+    const bool any = mine < group && first + mine < boxes;
+    if (any) {
+      const long long bx = first + mine, r = bx / nx;
+      i0[0] = (bx - r * nx) * VX;
+      i0[2] = r / ny;
+      i0[1] = (r - i0[2] * ny) * VY;
+      i0[2] *= VZ;
+      const int full[3] = {VX, VY, VZ};
+      T x[3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        ext[a] = g.n[a] - i0[a] < full[a] ? int(g.n[a] - i0[a]) : full[a];
+        x[a] = g.x0[a] + (T(i0[a]) + T(0.5) * T(full[a])) * g.d[a];
+      }
+      if constexpr (MODE == SPHERES) {
+        float least = __int_as_float(0x7f800000);
+        bool nan = false;
+        for (int i = lane % share; i < t.n_ops; i += share) {
+          T c[4];
+          ldq(t.p + t.ops[i].poff, c);
+          const float d0 = float(x[0]) - float(c[0]), d1 = float(x[1]) - float(c[1]), d2 = float(x[2]) - float(c[2]);
+          const float u = sqrt_approx(d0 * d0 + d1 * d1 + d2 * d2) - float(c[3]);
+          nan = nan || !(u == u);
+          least = fminf(least, u);
         }
-      __syncthreads();  // the next slab's pruning overwrites the ops this one read
+        v = nan ? qnan<T>() : T(least);
+      } else {
+        v = tape_eval<T, 3, T>(t, x);
+      }
+    }
+    if constexpr (MODE == SPHERES) {
+      for (int o = share / 2; o > 0; o >>= 1) {
+        const T u = __shfl_xor_sync(0xffffffffu, v, o);
+        v = u < v || !(u == u) ? u : v;  // the least, or NaN
+      }
+    }
+    if (any && lane % share == 0) {
+      if (v < -beyond) whole += ext[0] * ext[1] * ext[2];
+      open = !(v > beyond) && !(v < -beyond);
+    }
+    for (unsigned left = __ballot_sync(0xffffffffu, open); left; left &= left - 1) {
+      const int src = __ffs(left) - 1;
+      long long c0[3];
+      int ce[3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        c0[a] = __shfl_sync(0xffffffffu, i0[a], src);
+        ce[a] = __shfl_sync(0xffffffffu, ext[a], src);
+      }
+      int m = 0;
+      if constexpr (MODE == SPHERES || MODE == SMOOTH) {
+        float lo[3], hi[3], mag = 0.0f, low, up;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          lo[a] = float(g.x0[a] + (T(c0[a]) + T(0.5)) * g.d[a]);
+          hi[a] = float(g.x0[a] + (T(c0[a] + ce[a] - 1) + T(0.5)) * g.d[a]);
+          mag += fabsf(float(g.x0[a])) + float(g.n[a]) * float(g.d[a]);
+        }
+        m = prune_warp<T>(t, MODE, lo, hi, mag, list, low, up);
+      }
+      // cells near enough to need their plane are listed, then taken on full warps
+      const bool in = lane % VX < ce[0] && lane / VX < ce[1];
+      RowBody<T, MODE> body{t, list, m,
+                            {centroid_coord(g.x0[0], g.d[0], c0[0] + lane % VX),
+                             centroid_coord(g.x0[1], g.d[1], c0[1] + lane / VX), T(0)}};
+      int count = 0;
+      for (int k = 0; k < ce[2]; ++k) {
+        const T vc = body.value(centroid_coord(g.x0[2], g.d[2], c0[2] + k));
+        const bool near = in && !(vc > thr) && !(vc < -thr);
+        whole += in && vc < -thr ? 1 : 0;
+        const unsigned b = __ballot_sync(0xffffffffu, near);
+        if (near) s_near[w][count + __popc(b & ((1u << lane) - 1u))] = uint8_t(k * 32 + lane);
+        count += __popc(b);
+      }
+      __syncwarp();
+      for (int e = lane; e < count; e += 32) {
+        const int q = s_near[w][e] & 31, k = s_near[w][e] >> 5;
+        body.x[0] = centroid_coord(g.x0[0], g.d[0], c0[0] + q % VX);
+        body.x[1] = centroid_coord(g.x0[1], g.d[1], c0[1] + q / VX);
+        int side;
+        acc.add(double(plane_of<T, MX>(body.at(centroid_coord(g.x0[2], g.d[2], c0[2] + k)), h, side).fraction));
+      }
+      __syncwarp();  // the next box reuses the lists
     }
   }
-  __shared__ double ss[NT], sc[NT];
-  ss[threadIdx.x] = acc.s;
-  sc[threadIdx.x] = acc.c;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    KSum r{0.0, 0.0};
-    double cc = 0.0;
-    for (int i = 0; i < NT; ++i) { r.add(ss[i]); cc += sc[i]; }
-    partial[2 * blockIdx.x] = r.s;
-    partial[2 * blockIdx.x + 1] = r.c + cc;
-  }
+  acc.add(double(whole));
+  block_ksum(acc, partial + 2 * blockIdx.x);
 }
 
-__global__ void calc_volume_final(const double* partial, int nb, double* out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  KSum b{0.0, 0.0};
-  double cc = 0.0;
-  for (int i = 0; i < nb; ++i) { b.add(partial[2 * i]); cc += partial[2 * i + 1]; }
-  out[0] = b.s + (b.c + cc);
+__global__ void __launch_bounds__(NT) calc_volume_final(const double* partial, int nb, double* out) {
+  KSum a{0.0, 0.0};
+  for (int i = threadIdx.x; i < nb; i += NT) {
+    a.add(partial[2 * i]);
+    a.c += partial[2 * i + 1];
+  }
+  __shared__ double s_sum[2];
+  block_ksum(a, s_sum);
+  if (threadIdx.x == 0) out[0] = s_sum[0] + s_sum[1];
 }
 
 // cut_cell_report, src/cut_cell.jl:302-319: counts by kind, ambiguous, smallest cut fraction.
@@ -1036,30 +1146,66 @@ cudaError_t launch_plic(const DevGrid<T>& g, const DevTape& tape, const Cols& co
 
 int calc_volume_blocks() { return VOL_BLOCKS; }
 
-template <class T, int D>
-cudaError_t launch_calc_volume(const DevGrid<T>& g, const DevTape& tape, double* partial, double* out,
-                               cudaStream_t s, bool mixed) {
-  const int sm = CentroidSmem::of(tape).bytes;
-  if constexpr (D == 3) {
-    if (sm > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(calc_volume_z_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-      if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(calc_volume_z_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+namespace {
+
+template <class T, int MODE>
+cudaError_t launch_volume_z(const DevGrid<T>& g, const DevTape& tape, const TapeBounds& tb, double* partial, int* nb,
+                            bool mx, cudaStream_t s) {
+  const double h = double(g.d[0]);
+  double mag = tb.mag;
+  for (int a = 0; a < 3; ++a) mag += std::fabs(double(g.x0[a])) + double(g.n[a]) * double(g.d[a]);
+  const double thr = 0.5 * tb.grad1 * h * 1.001;
+  const double half = 0.5 * h * std::sqrt(double(VX * VX + VY * VY + VZ * VZ));
+  const double margin = (sizeof(T) == 4 || MODE == SPHERES ? 0x1p-16 : 0x1p-40) * (1.0 + tb.lipschitz) * mag;
+  const double beyond = (thr + tb.lipschitz * half) * 1.001 + margin;
+  const long long boxes = ((g.n[0] + VX - 1) / VX) * ((g.n[1] + VY - 1) / VY) * ((g.n[2] + VZ - 1) / VZ);
+  // boxes per warp at a time: few enough that every resident warp has some
+  int group = 32;
+  while (group > 1 && boxes < (long long)group * VOL_BLOCKS * (NT / 32)) group /= 2;
+  const long long ctas = (boxes + group * (NT / 32) - 1) / (group * (NT / 32));
+  *nb = int(ctas < VOL_BLOCKS ? ctas : VOL_BLOCKS);
+  const int lists = MODE == SPHERES || MODE == SMOOTH ? (NT / 32) * tape.n_ops * int(sizeof(unsigned)) : 0;
+  const int sm = ((tape.bytes_len + 15) / 16) * 16 + lists;
+  auto run = [&](auto kernel) {
+    if (sm > 40 * 1024) {
+      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
       if (e != cudaSuccess) return e;
     }
-    if (mixed && sizeof(T) == 4) calc_volume_z_kernel<T, true><<<VOL_BLOCKS, NT, sm, s>>>(g, tape, partial);
-    else calc_volume_z_kernel<T, false><<<VOL_BLOCKS, NT, sm, s>>>(g, tape, partial);
+    kernel<<<*nb, NT, sm, s>>>(g, tape, partial, T(thr), T(beyond), group);
+    return cudaSuccess;
+  };
+  if constexpr (sizeof(T) == 4) {
+    if (mx) return run(calc_volume_z_kernel<T, true, MODE>);
+  }
+  return run(calc_volume_z_kernel<T, false, MODE>);
+}
+
+}  // namespace
+
+template <class T, int D>
+cudaError_t launch_calc_volume(const DevGrid<T>& g, const DevTape& tape, const TapeBounds& tb, double* partial,
+                               double* out, cudaStream_t s, bool mixed) {
+  int nb = VOL_BLOCKS;
+  cudaError_t e;
+  if constexpr (D == 3) {
+    const bool mx = mixed && sizeof(T) == 4;
+    if (tape.prunable == 1) e = launch_volume_z<T, SPHERES>(g, tape, tb, partial, &nb, mx, s);
+    else if (tape.prunable == 2) e = launch_volume_z<T, SMOOTH>(g, tape, tb, partial, &nb, mx, s);
+    else if (tape.select) e = launch_volume_z<T, SELECT>(g, tape, tb, partial, &nb, mx, s);
+    else e = launch_volume_z<T, DUAL>(g, tape, tb, partial, &nb, mx, s);
+    if (e != cudaSuccess) return e;
   } else {
+    const int sm = CentroidSmem::of(tape).bytes;
     if (sm > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(calc_volume_kernel<T, D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+      e = cudaFuncSetAttribute(calc_volume_kernel<T, D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
       if (e == cudaSuccess)
         e = cudaFuncSetAttribute(calc_volume_kernel<T, D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
       if (e != cudaSuccess) return e;
     }
-    if (mixed && sizeof(T) == 4) calc_volume_kernel<T, D, true><<<VOL_BLOCKS, NT, sm, s>>>(g, tape, partial);
-    else calc_volume_kernel<T, D, false><<<VOL_BLOCKS, NT, sm, s>>>(g, tape, partial);
+    if (mixed && sizeof(T) == 4) calc_volume_kernel<T, D, true><<<nb, NT, sm, s>>>(g, tape, partial);
+    else calc_volume_kernel<T, D, false><<<nb, NT, sm, s>>>(g, tape, partial);
   }
-  calc_volume_final<<<1, 32, 0, s>>>(partial, VOL_BLOCKS, out);
+  calc_volume_final<<<1, NT, 0, s>>>(partial, nb, out);
   return cudaGetLastError();
 }
 
@@ -1080,8 +1226,8 @@ cudaError_t launch_report(long long ncell, const int8_t* kind, const uint8_t* am
 #define INST(T, D)                                                                                      \
   template cudaError_t launch_plic<T, D>(const DevGrid<T>&, const DevTape&, const Cols&, T*, T*, uint8_t*, int8_t*, \
                                          cudaStream_t, bool);                                           \
-  template cudaError_t launch_calc_volume<T, D>(const DevGrid<T>&, const DevTape&, double*, double*, cudaStream_t, \
-                                                bool);
+  template cudaError_t launch_calc_volume<T, D>(const DevGrid<T>&, const DevTape&, const TapeBounds&, double*, double*, \
+                                                cudaStream_t, bool);
 INST(float, 2)
 INST(float, 3)
 INST(double, 2)

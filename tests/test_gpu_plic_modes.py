@@ -2,6 +2,8 @@
 pruned per warp, hard combinators whose gradient is one primitive's, smooth minima on duals), at
 sizes around the row of 32 cells, the 8 rows of a CTA and the layers of a warp, bit for bit against
 the oracle in every precision."""
+import math
+
 import numpy as np
 import pytest
 import torch
@@ -53,3 +55,33 @@ def test_plic_update_bitwise(name, pname, prec):
         assert np.array_equal(bits(c.normals.cpu().numpy()), bits(rn)), n
         assert np.array_equal(bits(c.intercepts.cpu().numpy()), bits(ri)), n
         assert np.array_equal(c.is_valid.cpu().numpy(), rv), n
+
+
+VOLUME_BODIES = dict(_bodies(), inside=cc.Const(-1.0), zero=cc.Const(0.0),
+                     steep=cc.Plane((0.4, 0.3, 0.5), (3.0, -4.0, 12.0)),
+                     stretched=cc.Torus((0.5, 0.4, 0.3), 0.25, 0.08, 2.5 * np.eye(3)),
+                     waves=cc.Union(cc.Trig(0.4, (9.0, 7.0, 5.0), 0.05), cc.Sphere((0.1, 0.2, 0.2), 0.1)))
+
+
+@pytest.mark.parametrize("name", sorted(VOLUME_BODIES))
+@pytest.mark.parametrize("pname,prec", PREC)
+def test_calc_volume_is_the_sum_of_the_cell_fractions(name, pname, prec):
+    """Boxes settled by the body's bounds count as their cells do: the compensated sum of the oracle's
+    fractions, at sizes around the box of 8 x 4 x 8 cells and the 32 boxes a warp looks at, and on a
+    grid far from the origin, where rounding is a cell's size at Float32. A sum of n fractions in
+    [0, 1], compensated in Float64, is within 2 u of exact, plus n u^2; the product with the cell's
+    volume rounds twice more."""
+    dtype = torch.float64 if prec == 1 else torch.float32
+    T = np.float64 if prec == 1 else np.float32
+    tape = cc.flatten(VOLUME_BODIES[name], 3)
+    for n, x0, h in [((1, 1, 1), 0.0, 0.7), ((9, 5, 17), -0.1, 0.08), ((70, 33, 41), -0.05, 1.0 / 64),
+                     ((40, 40, 40), 0.0, 1.0 / 40), ((33, 9, 20), 2.0 ** 17, 0.01)]:
+        g = cc.CartesianGrid((x0, -0.03, 0.02), n, (h,) * 3)
+        frac = po.plic_fractions(g, tape, prec)
+        if name == "waves":  # sin differs from the host's by an ulp: a fraction moves by about u / h
+            tol = 64 * np.finfo(T).eps / h * max(n) * len(frac) ** (2 / 3)
+        else:
+            tol = 4 * 2.0 ** -53 * max(1.0, math.fsum(frac.tolist()))
+        pd = float(T(h) * T(h) * T(h))
+        v = cc.calc_volume(tape, g, dtype=dtype, precision="mixed" if prec == 2 else "plain")
+        assert abs(v / pd - math.fsum(frac.tolist())) <= tol, (name, n)
