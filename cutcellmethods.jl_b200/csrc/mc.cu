@@ -126,10 +126,6 @@ __device__ __forceinline__ constexpr int col_offset(int col) {
   return col == 0 ? Layout<T>::kind : col == 1 ? Layout<T>::amb : col == 2 ? Layout<T>::vf : col == 3 ? Layout<T>::c
        : col == 4 ? Layout<T>::ff : col == 5 ? Layout<T>::fcl : Layout<T>::ic;
 }
-__device__ __forceinline__ constexpr int col_elem(int col, int tsize) {
-  return col < 2 ? 1 : (col == 2 ? 1 : col == 3 ? 3 : col == 4 ? 6 : col == 5 ? 12 : 3) * tsize;
-}
-
 template <class T>
 __device__ __forceinline__ Stage<T> stage_at(unsigned char* base) {
   using L = Layout<T>;
@@ -188,7 +184,18 @@ __device__ __forceinline__ void put_uncut_z(const Stage<float>& st, int lc, floa
   d4[1] = make_float4(hx, hz, hx, hz);
 }
 
-template <class T, bool SAMPLE, bool PRUNED>
+// A warp copies n <= MOST contiguous elements.
+template <class E, int MOST>
+__device__ __forceinline__ void copy_row(E* __restrict__ dst, const E* __restrict__ src, int n, int lane) {
+#pragma unroll
+  for (int v = 0; v < MOST; v += 32)
+    if (v + lane < n) dst[v + lane] = src[v + lane];
+}
+
+// ALL_TMA: every column leaves by TMA (the common case, x extents that are multiples of 16); the
+// instantiation then carries none of the thread copies (update at 512^3 Float32 2.70 -> 2.65 ms, at
+// 256^3 Float64 with the report 775 -> 749 us).
+template <class T, bool SAMPLE, bool PRUNED, bool ALL_TMA>
 __global__ void __launch_bounds__(Tile<T>::NT, Tile<T>::MINB) mc_fill_kernel(const McArgs<T> A,
                                                                             const __grid_constant__ ColumnMaps maps) {
   using TL = Tile<T>;
@@ -293,7 +300,7 @@ __global__ void __launch_bounds__(Tile<T>::NT, Tile<T>::MINB) mc_fill_kernel(con
   const T cx = xa + T(0.5) * dx, cy = ya + T(0.5) * dy;
   const int lc = ty * TX + tx;
   const int s00 = ty * NSX + tx;
-  const bool fast = A.tma_mask != 0;
+  const bool fast = ALL_TMA || A.tma_mask != 0;
   const int rows = (int)((n1 - j0) < TY ? (n1 - j0) : TY);
   const int cnt = (int)((n0 - i0) < TX ? (n0 - i0) : TX);
   unsigned char* gcol[7] = {reinterpret_cast<unsigned char*>(A.cols.kind), A.cols.amb,
@@ -372,16 +379,16 @@ __global__ void __launch_bounds__(Tile<T>::NT, Tile<T>::MINB) mc_fill_kernel(con
     if (fast && tid == 0) {
       // one thread stores the TMA-addressable columns: one box each (clipped at the grid's edge)
       const int ci0 = (int)i0, cj0 = (int)j0, ck = (int)k;
-      if (A.tma_mask & 1) tma_store3(&maps.m[0], sbase + col_offset<T>(0), ci0, cj0, ck);
-      if (A.tma_mask & 2) tma_store3(&maps.m[1], sbase + col_offset<T>(1), ci0, cj0, ck);
-      if (A.tma_mask & 4) tma_store3(&maps.m[2], sbase + col_offset<T>(2), ci0, cj0, ck);
-      if (A.tma_mask & 8) tma_store3(&maps.m[3], sbase + col_offset<T>(3), 3 * ci0, cj0, ck);
-      if (A.tma_mask & 16) tma_store3(&maps.m[4], sbase + col_offset<T>(4), 6 * ci0, cj0, ck);
-      if (A.tma_mask & 32) tma_store4(&maps.m[5], sbase + col_offset<T>(5), 0, ci0, cj0, ck);
-      if (A.tma_mask & 64) tma_store3(&maps.m[6], sbase + col_offset<T>(6), 3 * ci0, cj0, ck);
+      if (ALL_TMA || (A.tma_mask & 1)) tma_store3(&maps.m[0], sbase + col_offset<T>(0), ci0, cj0, ck);
+      if (ALL_TMA || (A.tma_mask & 2)) tma_store3(&maps.m[1], sbase + col_offset<T>(1), ci0, cj0, ck);
+      if (ALL_TMA || (A.tma_mask & 4)) tma_store3(&maps.m[2], sbase + col_offset<T>(2), ci0, cj0, ck);
+      if (ALL_TMA || (A.tma_mask & 8)) tma_store3(&maps.m[3], sbase + col_offset<T>(3), 3 * ci0, cj0, ck);
+      if (ALL_TMA || (A.tma_mask & 16)) tma_store3(&maps.m[4], sbase + col_offset<T>(4), 6 * ci0, cj0, ck);
+      if (ALL_TMA || (A.tma_mask & 32)) tma_store4(&maps.m[5], sbase + col_offset<T>(5), 0, ci0, cj0, ck);
+      if (ALL_TMA || (A.tma_mask & 64)) tma_store3(&maps.m[6], sbase + col_offset<T>(6), 3 * ci0, cj0, ck);
       bulk_commit();
     }
-    if (A.tma_mask != 0x7f) {
+    if constexpr (!ALL_TMA) {
       // the columns TMA cannot address, copied by every thread: kind / ambiguous as one 32-bit word
       // per thread where every row starts on a 4-byte boundary (rows x 2 columns x TX/4 words fit
       // in the CTA), else bytes; T columns by element
@@ -395,25 +402,22 @@ __global__ void __launch_bounds__(Tile<T>::NT, Tile<T>::MINB) mc_fill_kernel(con
               reinterpret_cast<const uint32_t*>(sbase + col_offset<T>(col) + r * col_bytes<T>(col))[w];
         }
       }
-      // the rest element by element; most grids have none (every float column TMA-addressed and
-      // the byte columns copied as words), and the row loop is then skipped whole (200^3: 31.4 ->
-      // 18.3 warp instructions per cell, 0.383 -> 0.244 ms per update)
-      for (int r = 0; A.thread_cols && r < rows; ++r) {
-        const long long rowc = row0 + (long long)r * n0;
-#pragma unroll
-        for (int col = 0; col < 7; ++col) {
-          if (!(A.thread_cols & (1 << col))) continue;
-          const int es = col_elem(col, int(sizeof(T)));
-          const unsigned char* src = sbase + col_offset<T>(col) + r * col_bytes<T>(col);
-          unsigned char* dst = gcol[col] + rowc * es;
-          if (col >= 2) {
-            const T* s2 = reinterpret_cast<const T*>(src);
-            T* d2 = reinterpret_cast<T*>(dst);
-            const int ne = cnt * es / int(sizeof(T));
-            for (int v = tid; v < ne; v += NT) d2[v] = s2[v];
-          } else {
-            for (int v = tid; v < cnt; v += NT) dst[v] = src[v];
-          }
+      // the rest row by row, a warp taking the rows it staged itself: a column's part of a row is
+      // contiguous, so lane-strided elements are full-width stores whatever the row's alignment. (A CTA
+      // stepping through every row and column with all its threads ran mostly idle: 301 x 187 x 130
+      // mixed: fill 581 -> 228 us; 203^3 Float64: 1126 -> 434 us.) Most grids have none.
+      if (A.thread_cols) {
+        const int lane = tid & 31;
+        for (int r = tid >> 5; r < rows; r += NT / 32) {
+          const long long rowc = row0 + (long long)r * n0;
+          const int sr = r * TX;
+          if (A.thread_cols & 1) copy_row<int8_t, TX>(A.cols.kind + rowc, reinterpret_cast<const int8_t*>(sbase + L::kind) + sr, cnt, lane);
+          if (A.thread_cols & 2) copy_row<uint8_t, TX>(A.cols.amb + rowc, sbase + L::amb + sr, cnt, lane);
+          if (A.thread_cols & 4) copy_row<T, TX>(static_cast<T*>(A.cols.vf) + rowc, reinterpret_cast<const T*>(sbase + L::vf) + sr, cnt, lane);
+          if (A.thread_cols & 8) copy_row<T, 3 * TX>(static_cast<T*>(A.cols.c) + 3 * rowc, reinterpret_cast<const T*>(sbase + L::c) + 3 * sr, 3 * cnt, lane);
+          if (A.thread_cols & 16) copy_row<T, 6 * TX>(static_cast<T*>(A.cols.ff) + 6 * rowc, reinterpret_cast<const T*>(sbase + L::ff) + 6 * sr, 6 * cnt, lane);
+          if (A.thread_cols & 32) copy_row<T, 12 * TX>(static_cast<T*>(A.cols.fcl) + 12 * rowc, reinterpret_cast<const T*>(sbase + L::fcl) + 12 * sr, 12 * cnt, lane);
+          if (A.thread_cols & 64) copy_row<T, 3 * TX>(static_cast<T*>(A.cols.ic) + 3 * rowc, reinterpret_cast<const T*>(sbase + L::ic) + 3 * sr, 3 * cnt, lane);
         }
       }
     }
@@ -626,10 +630,14 @@ namespace {
 // every size: 500^3 2.85 against 3.18 ms, 260^3 0.468 against 0.496.)
 template <class T, bool SAMPLE, bool PRUNED>
 cudaError_t launch_fill(const McArgs<T>& a, const ColumnMaps& maps, unsigned blocks, int sm, cudaStream_t s) {
-  cudaError_t e = cudaFuncSetAttribute(mc_fill_kernel<T, SAMPLE, PRUNED>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-  if (e != cudaSuccess) return e;
-  mc_fill_kernel<T, SAMPLE, PRUNED><<<blocks, Tile<T>::NT, sm, s>>>(a, maps);
-  return cudaSuccess;
+  auto run = [&](auto kernel) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    if (e != cudaSuccess) return e;
+    kernel<<<blocks, Tile<T>::NT, sm, s>>>(a, maps);
+    return cudaSuccess;
+  };
+  if (a.tma_mask == 0x7f) return run(mc_fill_kernel<T, SAMPLE, PRUNED, true>);
+  return run(mc_fill_kernel<T, SAMPLE, PRUNED, false>);
 }
 }  // namespace
 
