@@ -44,7 +44,10 @@ template <class T> struct Tile {
 };
 constexpr int NS = 4;   // node slabs sampled per round (one op-major tape pass per thread)
 constexpr int KZ = 31;  // most z slices marched per CTA: KZ + 1 = 32 node slabs, 8 sampling rounds
-constexpr int CUT_NT = 256;  // 512^3 CSG body, Float32 update: 2.73 ms at 128, 2.71-2.72 at 256, 2.75 at 64
+// The cut kernel: 128 threads, bounded to 5 CTAs per SM at Float32 and 3 at Float64 (its registers: 111
+// and 239 unbounded). Kernel time in us of 128 (5, 3), 256 (3, 2) and 64 (8, 4): 512^3 Float32 80, 87, 81;
+// 256^3 Float64 40, 49, 46; a wave field at 192 x 160 x 129, Float64, 136, 138, 164.
+constexpr int CUT_NT = 128;
 
 template <class T>
 struct McArgs {
@@ -426,7 +429,7 @@ __global__ void __launch_bounds__(Tile<T>::NT, Tile<T>::MINB) mc_fill_kernel(con
 }
 
 template <class T, bool SAMPLE, bool MX>
-__global__ void __launch_bounds__(CUT_NT) mc_cut_kernel(const McArgs<T> A) {
+__global__ void __launch_bounds__(CUT_NT, sizeof(T) == 4 ? 5 : 3) mc_cut_kernel(const McArgs<T> A) {
   const long long n0 = A.g.n[0], n1 = A.g.n[1];
   const long long nx = n0 + 1, ny = n1 + 1;
   const T* phi = SAMPLE ? A.phi_out : A.phi_in;
@@ -441,8 +444,9 @@ __global__ void __launch_bounds__(CUT_NT) mc_cut_kernel(const McArgs<T> A) {
   const T cs[3] = {A.g.d[0], A.g.d[1], A.g.d[2]};
   const unsigned total = *A.cut_count;
   for (unsigned q = blockIdx.x * CUT_NT + threadIdx.x; q < total; q += gridDim.x * CUT_NT) {
-    const long long ci = A.cut_list[q];
-    const long long i = ci % n0, j = (ci / n0) % n1, k = ci / (n0 * n1);
+    const unsigned ci = A.cut_list[q];  // a cache has fewer than 2^32 cells: 32-bit quotients
+    const unsigned row = ci / unsigned(n0), k = row / unsigned(n1);
+    const unsigned i = ci - row * unsigned(n0), j = row - k * unsigned(n1);
     const long long b0 = i + nx * (j + ny * k);
     const long long bz = nx * ny;
     const T ph[8] = {phi[b0], phi[b0 + 1], phi[b0 + nx + 1], phi[b0 + nx],
@@ -685,7 +689,7 @@ cudaError_t launch_mc(const DevGrid<T>& g, const DevTape& tape, const T* phi_in,
     a.pruned_count = cnt;
   }
   const int sm = smem_bytes<T>(sample ? tape.bytes_len : 0);
-  const int cut_blocks = 148 * 8;
+  const int cut_blocks = 148 * 16;
   // the FP64 islands of mixed precision exist for Float32 caches only
   const bool mx = mixed && sizeof(T) == 4;
   if (sample && a.pruned_ops) {

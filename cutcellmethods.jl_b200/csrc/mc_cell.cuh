@@ -62,17 +62,6 @@ __device__ __forceinline__ bool test_face(const T* cb, int face) {
   if (fabs(det) < R(Eps<T>::v())) return face >= 0;
   return (R(face) * A) * det >= R(0);
 }
-// The same decider for a face code known at compile time (face_outside_connected, :421-422).
-template <class T, int FACE, bool MX = false>
-__device__ __forceinline__ bool test_face_c(const T* cb) {
-  using R = typename std::conditional<MX, double, T>::type;
-  constexpr int q[6][4] = {{0, 4, 5, 1}, {1, 5, 6, 2}, {2, 6, 7, 3}, {3, 7, 4, 0}, {0, 3, 2, 1}, {4, 7, 6, 5}};
-  const R A = cb[q[FACE - 1][0]], B = cb[q[FACE - 1][1]], C = cb[q[FACE - 1][2]], D = cb[q[FACE - 1][3]];
-  const R det = A * C - B * D;
-  if (fabs(det) < R(Eps<T>::v())) return true;
-  return (R(FACE) * A) * det >= R(0);
-}
-
 // _test_interior, :427-504. With MX every step runs in FP64 (R) from the FP32 corner values; the
 // thresholds stay eps(T).
 template <class T, bool MX = false>
@@ -110,60 +99,83 @@ __device__ bool test_interior(int itype, int edge, const T* cbt, int s) {
   return s < 0;
 }
 
-// The open polygon of one cube face in its own (p, q) frame: cell_boundary_walk
-// (src/marching_squares/marching_squares.jl:240-251) then _face_polygon
-// (src/marching_cubes/moments.jl:111-139) with _chord_target (:91-98).
-template <class T, bool MX = false>
-__device__ __forceinline__ void face_polygon(const T fn[4][2], const T fphi[4], bool connect, T& area2,
-                                             T& m0, T& m1) {
-  T sa[4][2], sb[4][2];
-  bool present[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int k1 = (k + 1) & 3;
-    const T fa = fphi[k], fb = fphi[k1];
-    const T frac = open_fraction<T, MX>(fa, fb);
-    present[k] = fa >= T(0) || fb >= T(0);
-    if (fa >= T(0) && fb >= T(0)) {
-      sa[k][0] = fn[k][0]; sa[k][1] = fn[k][1]; sb[k][0] = fn[k1][0]; sb[k][1] = fn[k1][1];
-    } else if (fa >= T(0)) {
-      sa[k][0] = fn[k][0]; sa[k][1] = fn[k][1];
-      sb[k][0] = fn[k][0] + frac * (fn[k1][0] - fn[k][0]);
-      sb[k][1] = fn[k][1] + frac * (fn[k1][1] - fn[k][1]);
-    } else {
-      sa[k][0] = fn[k1][0] + frac * (fn[k][0] - fn[k1][0]);
-      sa[k][1] = fn[k1][1] + frac * (fn[k][1] - fn[k1][1]);
-      sb[k][0] = fn[k1][0]; sb[k][1] = fn[k1][1];
+// The cube edge (MC_EDGE_NODES) between two corners.
+__host__ __device__ constexpr int edge_between(int a, int b) {
+  for (int e = 0; e < 12; ++e)
+    if ((edge_node(e, 0) == a && edge_node(e, 1) == b) || (edge_node(e, 0) == b && edge_node(e, 1) == a)) return e;
+  return -1;
+}
+__host__ __device__ constexpr int edge_axis(int e) { return e >= 8 ? 2 : (e & 1); }
+// Of a face's corner mask (bit k: corner k open), the first edge leaving the open part (corner k open,
+// k + 1 not) and the one entering it (k not, k + 1 open), two bits per mask.
+__host__ __device__ constexpr unsigned face_edges(bool leaving) {
+  unsigned t = 0;
+  for (unsigned m = 0; m < 16; ++m)
+    for (int k = 3; k >= 0; --k) {
+      const bool o = (m >> k) & 1, n = (m >> ((k + 1) & 3)) & 1;
+      if (leaving ? (o && !n) : (!o && n)) t = (t & ~(3u << (2 * m))) | (unsigned(k) << (2 * m));
     }
-  }
+  return t;
+}
+
+// The open part of a cut cube face in its own (p, q) frame, corners (0,0), (lp,0), (lp,lq), (0,lq) and
+// corner mask m (bits open): cell_boundary_walk (src/marching_squares/marching_squares.jl:240-251) then
+// _face_polygon (src/marching_cubes/moments.jl:111-139) with _chord_target (:91-98), from the cube edges'
+// crossings x[k] (the coordinate that varies along edge k). Twice its area and three times its first
+// moments, in the reference's order: the boundary segments of edges 0..3 (those of edges 0 and 3 lie
+// on the axes through the frame's origin and add exact zeros), then a chord per crossing out of the open
+// part. `connect`: the decider of a face with opposite corners open.
+template <class T, class Connect>
+__device__ __forceinline__ void face_polygon(unsigned m, T lp, T lq, const T x[4], Connect&& connect, T& area2, T& m0,
+                                             T& m1) {
+  const bool o1 = m & 2, o2 = m & 4, o3 = m & 8;
   area2 = T(0); m0 = T(0); m1 = T(0);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    if (present[k]) {
-      const T cr = sa[k][0] * sb[k][1] - sa[k][1] * sb[k][0];
-      area2 = area2 + cr;
-      m0 = m0 + (sa[k][0] + sb[k][0]) * cr;
-      m1 = m1 + (sa[k][1] + sb[k][1]) * cr;
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    if (!(fphi[k] >= T(0) && fphi[(k + 1) & 3] < T(0))) continue;
-    int j = k, hit = -1;
-#pragma unroll
-    for (int it = 0; it < 4; ++it) {
-      j = connect ? ((j + 1) & 3) : ((j + 3) & 3);
-      if (hit < 0 && fphi[j] < T(0) && fphi[(j + 1) & 3] >= T(0)) hit = j;
-    }
-    if (hit < 0) continue;
-    const T lb0 = hit == 0 ? sa[0][0] : hit == 1 ? sa[1][0] : hit == 2 ? sa[2][0] : sa[3][0];
-    const T lb1 = hit == 0 ? sa[0][1] : hit == 1 ? sa[1][1] : hit == 2 ? sa[2][1] : sa[3][1];
-    const T la0 = sb[k][0], la1 = sb[k][1];
-    const T cr = la0 * lb1 - la1 * lb0;
+  if (o1 || o2) {
+    const T a = o1 ? T(0) : x[1], b = o2 ? lq : x[1];
+    const T cr = lp * b - a * lp;
     area2 = area2 + cr;
-    m0 = m0 + (la0 + lb0) * cr;
-    m1 = m1 + (la1 + lb1) * cr;
+    m0 = m0 + (lp + lp) * cr;
+    m1 = m1 + (a + b) * cr;
   }
+  if (o2 || o3) {
+    const T a = o2 ? lp : x[2], b = o3 ? T(0) : x[2];
+    const T cr = a * lq - lq * b;
+    area2 = area2 + cr;
+    m0 = m0 + (a + b) * cr;
+    m1 = m1 + (lq + lq) * cr;
+  }
+  auto chord = [&](unsigned k, unsigned j) {
+    const T k0 = (k & 1) ? ((k & 2) ? T(0) : lp) : ((k & 2) ? x[2] : x[0]);
+    const T k1 = (k & 1) ? ((k & 2) ? x[3] : x[1]) : ((k & 2) ? lq : T(0));
+    const T j0 = (j & 1) ? ((j & 2) ? T(0) : lp) : ((j & 2) ? x[2] : x[0]);
+    const T j1 = (j & 1) ? ((j & 2) ? x[3] : x[1]) : ((j & 2) ? lq : T(0));
+    const T cr = k0 * j1 - k1 * j0;
+    area2 = area2 + cr;
+    m0 = m0 + (k0 + j0) * cr;
+    m1 = m1 + (k1 + j1) * cr;
+  };
+  constexpr unsigned LEAVING = face_edges(true), ENTERING = face_edges(false);
+  const unsigned k = (LEAVING >> (2 * m)) & 3u;
+  if (m == 5u || m == 10u) {
+    const unsigned j = connect() ? k + 1 : (k + 3) & 3u;
+    chord(k, j);
+    chord(k + 2, j ^ 2u);
+  } else {
+    chord(k, (ENTERING >> (2 * m)) & 3u);
+  }
+}
+
+// x / 3 and x / 6 for x >= 0, correctly rounded without a division: q = x RN(1/D), then one step q + (x -
+// D q) RN(1/D) whose residual is exact in an FMA. x / D lies at least ulp / 12 from any rounding boundary
+// (a boundary times D has more significant bits than x), far beyond the step's error of 2^-48 (2^-106)
+// relative. Below 2^-96 (2^-900) the residual could underflow, and x divides.
+template <class T, int D>
+__device__ __forceinline__ T div_const(T x) {
+  constexpr T R = T(1) / T(D);
+  if (!(x > (sizeof(T) == 4 ? T(0x1p-96) : T(0x1p-900)) || x == T(0))) return x / T(D);
+  const T q = x * R;
+  if constexpr (sizeof(T) == 4) return __fmaf_rn(__fmaf_rn(-float(D), q, x), R, q);
+  else return __fma_rn(__fma_rn(-double(D), q, x), R, q);
 }
 
 // Shared-memory staging of one tile's output columns.
@@ -234,18 +246,45 @@ __device__ __forceinline__ int mc_tile(const T phi[8], const DevTable& tb) {
 // raw corner values in MC_NODE_BITS order, `l` the cell's lattice edge lengths
 // (x_{i+1} - x_i per axis: every corner's cell-local coordinate is 0 or l exactly), `org` the
 // lower corner and `cs` the grid's cell size.
+//
+// A crossing belongs to two faces and to the triangles: it is formed once, one division per cut
+// edge, and the faces take their segments and chords from the coordinate that varies along it.
+// (Each face formed its own crossings and searched its chords over all four edges: 5300 warp instructions
+// for 32 cells. Bound by latency and issue. The cut kernel at 512^3 Float32 137 -> 80 us, at 64^3 23 -> 10,
+// at 256^3 Float64 75 -> 40; a wave field at 192 x 160 x 129, Float64, 244 -> 136.)
 template <class T, bool MX = false>
-__device__ __noinline__ void mc_cut_cell(const T phr[8], const T l[3], const T org[3], const T cs[3],
-                                         const DevTable tb, const Stage<T> st, long long lc) {
+__device__ __forceinline__ void mc_cut_cell(const T phr[8], const T l[3], const T org[3], const T cs[3],
+                                            const DevTable& tb, const Stage<T>& st, long long lc) {
   T phi[8];
+  unsigned lut = 0;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) phi[k] = nudge(phr[k]);
+  for (int k = 0; k < 8; ++k) {
+    phi[k] = nudge(phr[k]);
+    lut |= phi[k] >= T(0) ? 1u << k : 0u;
+  }
   T centre[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) centre[a] = org[a] + T(0.5) * cs[a];
   const T vol_cell = (cs[0] * cs[1]) * cs[2];
 
   const cc_mc_tile tl = tb.tiles[mc_tile<T, MX>(phi, tb)];
+
+  // edge_crossings (marching_cubes.jl:306-330)
+  T pts[13][3], xc[12];
+#pragma unroll
+  for (int e = 0; e < 12; ++e) {
+    const int a = edge_node(e, 0), b = edge_node(e, 1), ax = edge_axis(e);
+    xc[e] = T(0);
+    pts[e][0] = T(0); pts[e][1] = T(0); pts[e][2] = T(0);
+    if (((lut >> a) ^ (lut >> b)) & 1u) {
+      const T s = open_fraction<T, MX>(phi[a], phi[b]);
+      // a is the edge's end at 0, b the one at l
+      xc[e] = (lut >> a) & 1u ? T(0) + s * l[ax] : l[ax] + s * (T(0) - l[ax]);
+      const T z = s * T(0);  // the other two coordinates: the corner's plus this (a NaN value spreads)
+#pragma unroll
+      for (int x = 0; x < 3; ++x) pts[e][x] = x == ax ? xc[e] : (cbit(a, x) ? l[x] : T(0)) + z;
+    }
+  }
 
   // the six face clips (cut_cell_faces / _cut_cell_face, moments.jl:150-257)
   T ff[6], fcl[12];
@@ -255,35 +294,23 @@ __device__ __noinline__ void mc_cut_cell(const T phr[8], const T l[3], const T o
     const int ax = dir >> 1;
     const int p = ax == 0 ? 1 : 0;
     const int q = ax == 2 ? 1 : 2;
-    T fn[4][2], fphi[4];
-    int nout = 0;
+    unsigned m = 0;
+    T x[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const int c = face_node(dir, k);
-      fn[k][0] = cbit(c, p) ? l[p] : T(0);
-      fn[k][1] = cbit(c, q) ? l[q] : T(0);
-      fphi[k] = phi[c];
-      nout += fphi[k] >= T(0) ? 1 : 0;
+      m |= ((lut >> face_node(dir, k)) & 1u) << k;
+      x[k] = xc[edge_between(face_node(dir, k), face_node(dir, (k + 1) & 3))];
     }
-    amb_face = amb_face || ((nout == 2) && ((fphi[0] >= T(0)) == (fphi[2] >= T(0))));
-    const T avg0 = T(0.25) * (((fn[0][0] + fn[1][0]) + fn[2][0]) + fn[3][0]);
-    const T avg1 = T(0.25) * (((fn[0][1] + fn[1][1]) + fn[2][1]) + fn[3][1]);
+    amb_face = amb_face || m == 5u || m == 10u;
+    const T avg0 = T(0.25) * (l[p] + l[p]);
+    const T avg1 = T(0.25) * (l[q] + l[q]);
     T frac, c0, c1;
-    if (nout == 4 || nout == 0) {
-      frac = nout == 4 ? T(1) : T(0);
+    if (m == 15u || m == 0u) {
+      frac = m == 15u ? T(1) : T(0);
       c0 = avg0; c1 = avg1;
     } else {
-      bool connect;
-      switch (dir) {
-        case 0: connect = test_face_c<T, face_test_code(0), MX>(phi); break;
-        case 1: connect = test_face_c<T, face_test_code(1), MX>(phi); break;
-        case 2: connect = test_face_c<T, face_test_code(2), MX>(phi); break;
-        case 3: connect = test_face_c<T, face_test_code(3), MX>(phi); break;
-        case 4: connect = test_face_c<T, face_test_code(4), MX>(phi); break;
-        default: connect = test_face_c<T, face_test_code(5), MX>(phi); break;
-      }
       T area2, m0, m1;
-      face_polygon<T, MX>(fn, fphi, connect, area2, m0, m1);
+      face_polygon<T>(m, l[p], l[q], x, [&]() { return test_face<T, MX>(phi, face_test_code(dir)); }, area2, m0, m1);
       const T full = (T(1) * cs[p]) * cs[q];
       frac = (T(0.5) * area2) / full;
       if (area2 != T(0)) { const T den = T(3) * area2; c0 = m0 / den; c1 = m1 / den; }
@@ -293,32 +320,6 @@ __device__ __noinline__ void mc_cut_cell(const T phr[8], const T l[3], const T o
     fcl[2 * dir] = c0;
     fcl[2 * dir + 1] = c1;
   }
-
-  // edge_crossings (marching_cubes.jl:306-330)
-  T pts[13][3];
-  T acc0 = T(0), acc1 = T(0), acc2 = T(0);
-  int ncr = 0;
-#pragma unroll
-  for (int e = 0; e < 12; ++e) {
-    const int a = edge_node(e, 0), b = edge_node(e, 1);
-    const T fa = phi[a], fb = phi[b];
-    if ((fa >= T(0)) != (fb >= T(0))) {
-      const T s = open_fraction<T, MX>(fa, fb);
-#pragma unroll
-      for (int x = 0; x < 3; ++x) {
-        const T pa = cbit(a, x) ? l[x] : T(0);
-        const T pb = cbit(b, x) ? l[x] : T(0);
-        pts[e][x] = fa >= T(0) ? pa + s * (pb - pa) : pb + s * (pa - pb);
-      }
-      acc0 = acc0 + pts[e][0]; acc1 = acc1 + pts[e][1]; acc2 = acc2 + pts[e][2];
-      ++ncr;
-    } else {
-      pts[e][0] = T(0); pts[e][1] = T(0); pts[e][2] = T(0);
-    }
-  }
-  pts[12][0] = ncr > 0 ? acc0 / T(ncr) : T(0);
-  pts[12][1] = ncr > 0 ? acc1 / T(ncr) : T(0);
-  pts[12][2] = ncr > 0 ? acc2 / T(ncr) : T(0);
 
   // divergence theorem over the closed polyhedron (moments.jl:304-336)
   T vol3 = T(0);
@@ -339,8 +340,23 @@ __device__ __noinline__ void mc_cut_cell(const T phr[8], const T l[3], const T o
   }
   T iarea = T(0), ic0 = T(0), ic1 = T(0), ic2 = T(0);
   const uint8_t* codes = tb.codes + tl.code_off;
+  bool have_centre = false;
   for (int t = 0; t < tl.ntris; ++t) {
     const int ca = codes[3 * t] - 1, cb = codes[3 * t + 1] - 1, cd = codes[3 * t + 2] - 1;
+    if (!have_centre && (ca == 12 || cb == 12 || cd == 12)) {  // the crossings' mean, where a tile uses it
+      T acc0 = T(0), acc1 = T(0), acc2 = T(0);
+      int ncr = 0;
+#pragma unroll
+      for (int e = 0; e < 12; ++e)
+        if (((lut >> edge_node(e, 0)) ^ (lut >> edge_node(e, 1))) & 1u) {
+          acc0 = acc0 + pts[e][0]; acc1 = acc1 + pts[e][1]; acc2 = acc2 + pts[e][2];
+          ++ncr;
+        }
+      pts[12][0] = ncr > 0 ? acc0 / T(ncr) : T(0);
+      pts[12][1] = ncr > 0 ? acc1 / T(ncr) : T(0);
+      pts[12][2] = ncr > 0 ? acc2 / T(ncr) : T(0);
+      have_centre = true;
+    }
     const T A0 = pts[ca][0], A1 = pts[ca][1], A2 = pts[ca][2];
     const T B0 = pts[cb][0], B1 = pts[cb][1], B2 = pts[cb][2];
     const T D0 = pts[cd][0], D1 = pts[cd][1], D2 = pts[cd][2];
@@ -349,13 +365,13 @@ __device__ __noinline__ void mc_cut_cell(const T phr[8], const T l[3], const T o
     const T w0 = T(0.5) * (u1 * v2 - u2 * v1);
     const T w1 = T(0.5) * (u2 * v0 - u0 * v2);
     const T w2 = T(0.5) * (u0 * v1 - u1 * v0);
-    const T x0 = ((A0 + B0) + D0) / T(3);
-    const T x1 = ((A1 + B1) + D1) / T(3);
-    const T x2 = ((A2 + B2) + D2) / T(3);
+    const T x0 = div_const<T, 3>((A0 + B0) + D0);
+    const T x1 = div_const<T, 3>((A1 + B1) + D1);
+    const T x2 = div_const<T, 3>((A2 + B2) + D2);
     vol3 = vol3 - ((w0 * x0 + w1 * x1) + w2 * x2);
-    const T q0 = (((((A0 * A0 + B0 * B0) + D0 * D0) + A0 * B0) + B0 * D0) + D0 * A0) / T(6);
-    const T q1 = (((((A1 * A1 + B1 * B1) + D1 * D1) + A1 * B1) + B1 * D1) + D1 * A1) / T(6);
-    const T q2 = (((((A2 * A2 + B2 * B2) + D2 * D2) + A2 * B2) + B2 * D2) + D2 * A2) / T(6);
+    const T q0 = div_const<T, 6>(((((A0 * A0 + B0 * B0) + D0 * D0) + A0 * B0) + B0 * D0) + D0 * A0);
+    const T q1 = div_const<T, 6>(((((A1 * A1 + B1 * B1) + D1 * D1) + A1 * B1) + B1 * D1) + D1 * A1);
+    const T q2 = div_const<T, 6>(((((A2 * A2 + B2 * B2) + D2 * D2) + A2 * B2) + B2 * D2) + D2 * A2);
     cm0 = cm0 - w0 * q0;
     cm1 = cm1 - w1 * q1;
     cm2 = cm2 - w2 * q2;
@@ -378,9 +394,6 @@ __device__ __noinline__ void mc_cut_cell(const T phr[8], const T l[3], const T o
   } else {
     ic[0] = centre[0]; ic[1] = centre[1]; ic[2] = centre[2];
   }
-  int lut = 0;
-#pragma unroll
-  for (int p = 0; p < 8; ++p) lut |= (phi[p] >= T(0) ? 1 : 0) << p;
   const int lc_case = tb.luts[lut].lcase;
   const bool amb_case = lc_case == 5 || lc_case == 7 || lc_case == 8 || lc_case == 11 || lc_case == 13 || lc_case == 14;
   put_cell<T>(st, lc, 2, (amb_face || amb_case) ? 1 : 0, volume / vol_cell, c, ff, fcl, ic);
