@@ -274,7 +274,8 @@ def update_cache(cache, geo, domain, stream=None, sync=True):
     """Recompute every cell of ``cache`` from ``geo`` over ``domain``; blocks until done
     (src/marching_squares/cache.jl:55-64, src/plic/cache.jl:77-92)."""
     dev = cache.cells.kind.device
-    s = C.c_void_p(stream) if stream is not None else _stream(dev)
+    current = torch.cuda.current_stream(dev) if stream is None else None
+    s = C.c_void_p(stream if current is None else current.cuda_stream)
     L = cache.handle.lib
     cells = cache.cells.struct()
     if isinstance(domain, QuadTree):
@@ -315,7 +316,7 @@ def update_cache(cache, geo, domain, stream=None, sync=True):
                 fn = L.cc_mc_update if mc else L.cc_ms_update
                 _check(fn(cache.handle.h, C.byref(gs), C.byref(tp.s), _ptr(cache.phi), C.byref(cells), s))
     if sync:
-        torch.cuda.current_stream(dev).synchronize() if stream is None else torch.cuda.synchronize(dev)
+        torch.cuda.synchronize(dev) if current is None else current.synchronize()
     return cache
 
 

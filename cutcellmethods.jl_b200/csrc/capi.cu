@@ -33,6 +33,7 @@ cc_status fail(cc_status s, const std::string& msg) {
 // boundary and padded to a multiple of 4 elements (at most 16), plus, for a smooth-min, its k --
 // at most 3 + 16 + 1 = 20 slots per op.
 constexpr int PACK_MAX_PARAMS = 20 * CC_TAPE_MAX_OPS;
+constexpr size_t TAPE_HEAD = 16;  // the cut count, before the tape (kept 16-byte aligned)
 constexpr size_t TAPE_CAP = CC_TAPE_MAX_OPS * sizeof(cc_op) + PACK_MAX_PARAMS * sizeof(double) + 64;
 
 int prim_params(int opcode, int dim) {
@@ -279,22 +280,28 @@ size_t tape_pack_capacity() { return TAPE_CAP; }
 
 namespace {
 
-// Pack a validated tape and upload it into the handle's buffer, ordered on stream s.
+// Pack a validated tape and upload it into the handle's buffer, ordered on stream s. The buffer's first
+// TAPE_HEAD bytes are the marching-cubes cut count; with `zero_count` they go up with the tape, zeroed, in
+// the one copy (a memset less per update).
 template <class T>
-cc_status upload_tape(cc_handle* h, const cc_optape* t, int dim, cudaStream_t s, cci::DevTape* out) {
+cc_status upload_tape(cc_handle* h, const cc_optape* t, int dim, cudaStream_t s, cci::DevTape* out,
+                      bool zero_count = false) {
   if (h->tape_pending) {
     const cudaError_t e = cudaEventSynchronize(h->tape_copied);
     if (e != cudaSuccess) return cuda_fail(e, "tape staging");
     h->tape_pending = false;
   }
   int np = 0;
-  const size_t bytes = cci::pack_tape<T>(t, dim, h->tape_host, &np);
-  cudaError_t e = cudaMemcpyAsync(h->tape_dev, h->tape_host, bytes, cudaMemcpyHostToDevice, s);
+  const size_t bytes = cci::pack_tape<T>(t, dim, h->tape_host + TAPE_HEAD, &np);
+  const size_t from = zero_count ? 0 : TAPE_HEAD;
+  if (zero_count) std::memset(h->tape_host, 0, TAPE_HEAD);
+  cudaError_t e = cudaMemcpyAsync(h->tape_dev + from, h->tape_host + from, bytes + TAPE_HEAD - from,
+                                  cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) return cuda_fail(e, "tape upload");
   e = cudaEventRecord(h->tape_copied, s);
   if (e != cudaSuccess) return cuda_fail(e, "tape upload");
   h->tape_pending = true;
-  out->bytes = h->tape_dev;
+  out->bytes = h->tape_dev + TAPE_HEAD;
   out->n_ops = t->n_ops;
   out->n_params = np;
   out->bytes_len = int(bytes);
@@ -413,8 +420,8 @@ cc_status cc_handle_create(int32_t device, int32_t method, int32_t dim, int32_t 
   h->tree = tree;
   for (int a = 0; a < 3; ++a) h->n[a] = a < dim ? n[a] : 1;
   if (tree) { h->n[1] = 0; h->n[2] = 0; }
-  cudaError_t e = cudaMalloc(&h->tape_dev, TAPE_CAP);
-  if (e == cudaSuccess) e = cudaMallocHost(&h->tape_host, TAPE_CAP);
+  cudaError_t e = cudaMalloc(&h->tape_dev, TAPE_HEAD + TAPE_CAP);
+  if (e == cudaSuccess) e = cudaMallocHost(&h->tape_host, TAPE_HEAD + TAPE_CAP);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->tape_copied, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaMalloc(&h->vol_scratch, (2 * cci::calc_volume_blocks() + 2) * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&h->rep_scratch, 8 * sizeof(unsigned long long));
@@ -423,7 +430,7 @@ cc_status cc_handle_create(int32_t device, int32_t method, int32_t dim, int32_t 
   if (e == cudaSuccess && method == CC_MARCHING_CUBES) {
     const int64_t ncell = h->n[0] * h->n[1] * h->n[2];
     e = cudaMalloc(&h->cut_list, size_t(ncell) * sizeof(unsigned));
-    if (e == cudaSuccess) e = cudaMalloc(&h->cut_count, sizeof(unsigned));
+    h->cut_count = reinterpret_cast<unsigned*>(h->tape_dev);
   }
   if (e == cudaSuccess && method == CC_PLIC && dim == 3 && !tree)
     e = cudaMalloc(&h->plic_sides, size_t(h->n[0] * h->n[1]) * size_t(h->n[2] + 1) + 64);  // see plic_resolve_kernel
@@ -446,7 +453,6 @@ cc_status cc_handle_destroy(cc_handle* h) {
   if (h->rep_scratch) cudaFree(h->rep_scratch);
   if (h->rep_host) cudaFreeHost(h->rep_host);
   if (h->cut_list) cudaFree(h->cut_list);
-  if (h->cut_count) cudaFree(h->cut_count);
   if (h->plic_sides) cudaFree(h->plic_sides);
   if (h->mesh_vbase) cudaFree(h->mesh_vbase);
   if (h->mesh_scan) cudaFree(h->mesh_scan);
@@ -490,19 +496,19 @@ static cc_status mc_common(cc_handle* h, const cc_grid* g, const cc_optape* body
   cudaError_t e;
   ++h->generation;
   if (h->prec == CC_F64) {
-    if (body && (st = upload_tape<double>(h, body, 3, s, &tape)) != CC_OK) return st;
+    if (body && (st = upload_tape<double>(h, body, 3, s, &tape, true)) != CC_OK) return st;
     const size_t pb = tape.prunable ? cci::mc_prune_bytes(g->n[0], g->n[1], g->n[2], tape.n_ops, true) : 0;
     void* ps = pb ? cci::prune_scratch(h, pb) : nullptr;
     e = cci::launch_mc<double>(dev_grid<double>(g), tape, static_cast<const double*>(phi_in),
                                static_cast<double*>(phi_out), cols_of(cells), h->tb, h->cut_list, h->cut_count, s,
-                               true, false, ps, ps ? pb : 0);
+                               true, false, ps, ps ? pb : 0, body != nullptr);
   } else {
-    if (body && (st = upload_tape<float>(h, body, 3, s, &tape)) != CC_OK) return st;
+    if (body && (st = upload_tape<float>(h, body, 3, s, &tape, true)) != CC_OK) return st;
     const size_t pb = tape.prunable ? cci::mc_prune_bytes(g->n[0], g->n[1], g->n[2], tape.n_ops, false) : 0;
     void* ps = pb ? cci::prune_scratch(h, pb) : nullptr;
     e = cci::launch_mc<float>(dev_grid<float>(g), tape, static_cast<const float*>(phi_in),
                               static_cast<float*>(phi_out), cols_of(cells), h->tb, h->cut_list, h->cut_count, s, true,
-                              h->prec == CC_MIXED, ps, ps ? pb : 0);
+                              h->prec == CC_MIXED, ps, ps ? pb : 0, body != nullptr);
   }
   if (e != cudaSuccess) return cuda_fail(e, "marching cubes launch");
   return CC_OK;

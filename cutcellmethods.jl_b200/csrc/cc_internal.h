@@ -71,12 +71,12 @@ struct Cols {
 // every cell. Returns the CUDA launch status.
 // `cut_list` (one slot per cell) and `cut_count` are scratch: the fill pass lists the cut band
 // there and the cut pass reads it back.
-// With with_cut false only the fill pass runs (the cut band is listed, not built).
+// With count_zeroed, *cut_count is 0 already in stream order. With with_cut false only the fill pass runs (the cut band is listed, not built).
 template <class T>
 cudaError_t launch_mc(const DevGrid<T>& g, const DevTape& tape, const T* phi_in, T* phi_out,
                       const Cols& cols, const DevTable& tb, unsigned* cut_list, unsigned* cut_count,
                       cudaStream_t s, bool with_cut = true, bool mixed = false,
-                      void* prune_scratch = nullptr, size_t prune_bytes = 0);
+                      void* prune_scratch = nullptr, size_t prune_bytes = 0, bool count_zeroed = false);
 // The mbarrier poll limit of the learned kernels (cc_set_wait_limit): set returns the old value; a
 // negative argument restores the default.
 long long set_wait_limit(long long polls);
@@ -182,7 +182,7 @@ struct cc_handle {
   size_t table_bytes = 0;
   cci::DevTable tb{};
   unsigned* cut_list = nullptr;   // marching cubes: the cut band's cell indices (one slot per cell)
-  unsigned* cut_count = nullptr;
+  unsigned* cut_count = nullptr;  // its length: the head of tape_dev
   int8_t* plic_sides = nullptr;  // 3D PLIC: the fit's per-cell side bytes for the face pass
   double* vol_scratch = nullptr;  // calc_volume partials + result
   unsigned long long* rep_scratch = nullptr;  // report counters + the complement of the min's bits

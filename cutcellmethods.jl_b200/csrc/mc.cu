@@ -648,7 +648,8 @@ cudaError_t launch_fill(const McArgs<T>& a, const ColumnMaps& maps, unsigned blo
 template <class T>
 cudaError_t launch_mc(const DevGrid<T>& g, const DevTape& tape, const T* phi_in, T* phi_out,
                       const Cols& cols, const DevTable& tb, unsigned* cut_list, unsigned* cut_count,
-                      cudaStream_t s, bool with_cut, bool mixed, void* prune_scratch, size_t prune_bytes) {
+                      cudaStream_t s, bool with_cut, bool mixed, void* prune_scratch, size_t prune_bytes,
+                      bool count_zeroed) {
   using TL = Tile<T>;
   McArgs<T> a;
   a.g = g;
@@ -671,7 +672,7 @@ cudaError_t launch_mc(const DevGrid<T>& g, const DevTape& tape, const T* phi_in,
   const long long nk = (g.n[2] + a.kz - 1) / a.kz;
   const long long blocks = (long long)a.n_itiles * a.n_jtiles * nk;
   if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-  cudaError_t e = cudaMemsetAsync(cut_count, 0, sizeof(unsigned), s);
+  cudaError_t e = count_zeroed ? cudaSuccess : cudaMemsetAsync(cut_count, 0, sizeof(unsigned), s);
   if (e != cudaSuccess) return e;
   const bool sample = phi_in == nullptr;
   a.pruned_ops = nullptr;
@@ -713,9 +714,9 @@ cudaError_t launch_mc(const DevGrid<T>& g, const DevTape& tape, const T* phi_in,
 
 template cudaError_t launch_mc<float>(const DevGrid<float>&, const DevTape&, const float*, float*,
                                       const Cols&, const DevTable&, unsigned*, unsigned*, cudaStream_t, bool, bool,
-                                      void*, size_t);
+                                      void*, size_t, bool);
 template cudaError_t launch_mc<double>(const DevGrid<double>&, const DevTape&, const double*, double*,
                                        const Cols&, const DevTable&, unsigned*, unsigned*, cudaStream_t, bool, bool,
-                                       void*, size_t);
+                                       void*, size_t, bool);
 
 }  // namespace cci
