@@ -253,9 +253,9 @@ __device__ __forceinline__ S tape_combine(int mode, const S& top, const S& v, T 
     case CC_COMB_SMIN: {
       const S ad = dabs(top - v);
       const S hk = k - ad;
-      const S zero = Lift<S, T>::c(T(0));
-      const S h = (val(hk) > T(0) ? hk : zero) / k;
       const S m = val(v) < val(top) ? v : top;
+      if (!(val(hk) > T(0))) return m;  // h = 0 / k: the step subtracts an exact 0, so no division is needed
+      const S h = hk / k;
       return m - ((h * h) * k) * T(0.25);
     }
     default: return v;
@@ -431,11 +431,25 @@ __device__ __forceinline__ void tape_eval_multi(const STape<T>& t, const T (&x)[
 #pragma unroll
         for (int q = 0; q < NB; ++q) acc[q] = v[q] > acc[q] ? v[q] : acc[q];
         break;
-      default: {
-        const T k = op.combine == CC_COMB_SMIN ? t.p[op.kparam] : T(0);
+      case CC_COMB_SMIN: {
+        // most nodes are k or more from where two operands blend: no point's step divides then (the
+        // fill of a smooth blob at 256^3 Float32: 562 -> 425 us)
+        const T k = t.p[op.kparam];
+        bool blend = false;
 #pragma unroll
-        for (int q = 0; q < NB; ++q) acc[q] = tape_combine<T, T>(op.combine, acc[q], v[q], k);
+        for (int q = 0; q < NB; ++q) blend = blend || k - dabs(acc[q] - v[q]) > T(0);
+        if (blend) {
+#pragma unroll
+          for (int q = 0; q < NB; ++q) acc[q] = tape_combine<T, T>(CC_COMB_SMIN, acc[q], v[q], k);
+        } else {
+#pragma unroll
+          for (int q = 0; q < NB; ++q) acc[q] = v[q] < acc[q] ? v[q] : acc[q];
+        }
+        break;
       }
+      default:
+#pragma unroll
+        for (int q = 0; q < NB; ++q) acc[q] = tape_combine<T, T>(op.combine, acc[q], v[q], T(0));
     }
   }
 #pragma unroll
