@@ -618,20 +618,6 @@ __device__ int prune_union(const STape<T>& t, int mode, const double lo[D], cons
   return *count;
 }
 
-// Shared-memory places of prune_union's output and scratch, after a tape loaded at `base`.
-struct PruneSmem {
-  int ops, ls, us, end;
-  template <class DT>
-  __host__ __device__ static PruneSmem of(const DT& tape, int base) {
-    PruneSmem p;
-    p.ops = base + ((tape.bytes_len + 15) / 16) * 16;
-    p.ls = p.ops + ((tape.n_ops * int(sizeof(cc_op)) + 15) / 16) * 16;
-    p.us = p.ls + tape.n_ops * 8;
-    p.end = p.us + tape.n_ops * 8;
-    return p;
-  }
-};
-
 // ---------------------------------------------------------------------------------------------
 // The value and gradient of a body at a cell centroid, with the gradient formed only where it is
 // used. Evaluating the whole tape on duals pays every primitive's gradient (three divisions for a
@@ -765,14 +751,14 @@ __device__ __forceinline__ Dual<T, 3> tape_eval_select(const STape<T>& t, const 
 // input). Bounds are formed in Float32 whatever T is; the margin, 2^-18 of every magnitude involved
 // (`mag`: the grid's coordinates, plus the sphere's own), is at least eight times their rounding and
 // that of the coordinates and of T's evaluation. A NaN or infinite bound keeps its sphere. Writes the
-// kept spheres in op order, poff | kparam << 16, to `out` (n_ops entries) and returns their number;
+// kept spheres in op order, as indices (INDEX) or poff | kparam << 16, to `out` (n_ops entries) and returns their number;
 // low and up receive the smallest lower and upper bound over the spheres.
 __device__ __forceinline__ float sqrt_approx(float x) {
   float r;
   asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
-template <class T>
+template <class T, bool INDEX = false>
 __device__ __forceinline__ int prune_warp(const STape<T>& t, int mode, const float lo[3], const float hi[3], float mag,
                                           unsigned* out, float& low, float& up) {
   const int lane = threadIdx.x & 31, n = t.n_ops;
@@ -842,7 +828,7 @@ __device__ __forceinline__ int prune_warp(const STape<T>& t, int mode, const flo
     const unsigned b = __ballot_sync(0xffffffffu, keep);
     if (keep) {
       const cc_op op = t.ops[i];
-      out[kept + __popc(b & ((1u << lane) - 1u))] = unsigned(op.poff) | (unsigned(op.kparam) << 16);
+      out[kept + __popc(b & ((1u << lane) - 1u))] = INDEX ? unsigned(i) : unsigned(op.poff) | (unsigned(op.kparam) << 16);
     }
     kept += __popc(b);
   }

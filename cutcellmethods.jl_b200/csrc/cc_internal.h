@@ -40,7 +40,7 @@ struct DevTape {
   int n_ops;
   int n_params;
   int bytes_len;
-  int prunable = 0;  // 1: a union (MIN) of spheres, 2: a smooth union (SMIN) of spheres; see prune_union
+  int prunable = 0;  // 1: a union (MIN) of spheres, 2: a smooth union (SMIN) of spheres; see prune_union, prune_warp
   int select = 0;    // no smooth minimum: value and gradient are one primitive's (tape_eval_select)
   int slab = 8;      // the 3D PLIC passes' pruning slab in cell layers (prune_slab)
 };
@@ -75,16 +75,11 @@ struct Cols {
 template <class T>
 cudaError_t launch_mc(const DevGrid<T>& g, const DevTape& tape, const T* phi_in, T* phi_out,
                       const Cols& cols, const DevTable& tb, unsigned* cut_list, unsigned* cut_count,
-                      cudaStream_t s, bool with_cut = true, bool mixed = false,
-                      void* prune_scratch = nullptr, size_t prune_bytes = 0, bool count_zeroed = false);
+                      cudaStream_t s, bool with_cut = true, bool mixed = false, bool count_zeroed = false);
 // The mbarrier poll limit of the learned kernels (cc_set_wait_limit): set returns the old value; a
 // negative argument restores the default.
 long long set_wait_limit(long long polls);
 long long wait_limit();
-// Scratch launch_mc needs to prune a union-of-spheres tape per fill CTA (n_ops ops per CTA).
-size_t mc_prune_bytes(long long n0, long long n1, long long n2, int n_ops, bool f64);
-// The handle's pruning scratch, grown to at least `bytes` (null on failure).
-void* prune_scratch(cc_handle* h, size_t bytes);
 
 // The learned correction (learned.cu).
 int mlp_nparam();
@@ -193,8 +188,6 @@ struct cc_handle {
   size_t mesh_scan_n = 0;
   unsigned long long* mesh_list = nullptr;  // generate_mesh: cut nodes and cut cells in order
   unsigned long long mesh_node_cap = 0, mesh_cell_cap = 0;
-  void* prune = nullptr;  // marching cubes: per fill CTA pruned op lists of a union of spheres
-  size_t prune_bytes = 0;
   void* ms_mesh = nullptr;  // marching squares: the last contour built (ms_mesh.cu)
   void* plic_mesh = nullptr;  // PLIC: the last surface count's block offsets (plic_mesh.cu)
   cci::MeshKey mesh_key;      // marching cubes: what the kept mesh count was taken from

@@ -64,9 +64,6 @@ struct McArgs {
   int tma_mask;  // bit c: column c leaves through TMA tensor stores (its map below is valid)
   int byte_words;  // kind/ambiguous rows start on 4-byte boundaries
   int thread_cols;  // bit c: column c is copied element by element by the threads (no TMA, no words)
-  // a union of spheres: each CTA's kept ops (stride tape.n_ops) and their count, or null
-  const cc_op* pruned_ops;
-  const int* pruned_count;
 };
 
 // One TMA tensor map per output column: kind, ambiguous, volume_fraction (n0 x n1 x n2), centroid
@@ -143,37 +140,6 @@ __device__ __forceinline__ Stage<T> stage_at(unsigned char* base) {
   return st;
 }
 
-// For a union of spheres: each fill CTA's pencil (cells i0.., j0.., k0..k1) gets the tape pruned to
-// the box of its nodes (prune_union), written to out[cta * n_ops ..] with its count.
-template <class T>
-__global__ void __launch_bounds__(256) prune_pencils_kernel(const McArgs<T> A, cc_op* __restrict__ out,
-                                                            int* __restrict__ count) {
-  extern __shared__ __align__(128) unsigned char smem[];  // one alignment for every extern declaration
-  __shared__ int s_count;
-  using TL = Tile<T>;
-  const STape<T> t = load_tape<T>(A.tape.bytes, A.tape.n_ops, A.tape.n_params, smem);
-  __syncthreads();
-  const PruneSmem ps = PruneSmem::of(A.tape, 0);
-  int b = blockIdx.x;
-  const int it = b % A.n_itiles; b /= A.n_itiles;
-  const int jt = b % A.n_jtiles; b /= A.n_jtiles;
-  const long long n0 = A.g.n[0], n1 = A.g.n[1], n2 = A.g.n[2];
-  const long long i0 = (long long)it * TL::TX, j0 = (long long)jt * TL::TY, k0 = (long long)b * A.kz;
-  const long long i1 = i0 + TL::TX < n0 ? i0 + TL::TX : n0, j1 = j0 + TL::TY < n1 ? j0 + TL::TY : n1;
-  const long long k1 = k0 + A.kz < n2 ? k0 + A.kz : n2;
-  const double lo[3] = {double(A.g.x0[0]) + double(i0) * double(A.g.d[0]),
-                        double(A.g.x0[1]) + double(j0) * double(A.g.d[1]),
-                        double(A.g.x0[2]) + double(k0) * double(A.g.d[2])};
-  const double hi[3] = {double(A.g.x0[0]) + double(i1) * double(A.g.d[0]),
-                        double(A.g.x0[1]) + double(j1) * double(A.g.d[1]),
-                        double(A.g.x0[2]) + double(k1) * double(A.g.d[2])};
-  cc_op* kept = reinterpret_cast<cc_op*>(smem + ps.ops);
-  const int m = prune_union<T, 3>(t, A.tape.prunable, lo, hi, reinterpret_cast<double*>(smem + ps.ls),
-                                  reinterpret_cast<double*>(smem + ps.us), kept, &s_count);
-  for (int q = threadIdx.x; q < m; q += blockDim.x) out[(long long)blockIdx.x * A.tape.n_ops + q] = kept[q];
-  if (threadIdx.x == 0) count[blockIdx.x] = m;
-}
-
 // An uncut cell whose staging slot held an uncut cell of the same kind at the slot's previous use
 // (two slices earlier, in the same column): kind, flag, fraction, face fractions and the x, y
 // parts are the same values, so only what depends on the slice is written -- the centroid's and
@@ -219,12 +185,37 @@ __global__ void __launch_bounds__(Tile<T>::NT, Tile<T>::MINB) mc_fill_kernel(con
   STape<T> tape;
   if (SAMPLE) {
     tape = load_tape<T>(A.tape.bytes, A.tape.n_ops, A.tape.n_params, smem + L::tape);
-    if (PRUNED) {  // this pencil's kept ops over the loaded ones (same places, fewer)
-      const int m = A.pruned_count[blockIdx.x];
-      cc_op* ops = reinterpret_cast<cc_op*>(smem + L::tape);
+    if (PRUNED) {
+      // a union of spheres: one warp prunes it to the box of the pencil's nodes, the kept ops follow the
+      // tape. (A launch of its own used to write every pencil's ops to memory. At 256^3 Float32: 64 spheres
+      // 470 -> 454 us an update, a smooth blob 581 -> 571. Unions of any primitives, bounded by their value at
+      // the box's centre and a Lipschitz constant, were no faster: the CSG body at 512^3 2.57 -> 2.56 ms, at
+      // 256^3 Float64 642 -> 662 us.)
+      __shared__ int s_kept;
+      const int n = A.tape.n_ops;
+      cc_op* kept = reinterpret_cast<cc_op*>(smem + L::tape + ((A.tape.bytes_len + 15) / 16) * 16);
       __syncthreads();
-      for (int q = tid; q < m; q += NT) ops[q] = A.pruned_ops[(long long)blockIdx.x * A.tape.n_ops + q];
-      tape.n_ops = m;
+      if (tid < 32) {
+        const long long first[3] = {i0, j0, k0}, last[3] = {i0 + TX < n0 ? i0 + TX : n0, j0 + TY < n1 ? j0 + TY : n1, k1};
+        float lo[3], hi[3], mag = 0.0f, low, up;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          lo[a] = float(node_coord(A.g.x0[a], A.g.d[a], first[a]));
+          hi[a] = float(node_coord(A.g.x0[a], A.g.d[a], last[a]));
+          mag += fabsf(float(A.g.x0[a])) + float(A.g.n[a]) * float(A.g.d[a]);
+        }
+        unsigned* list = reinterpret_cast<unsigned*>(kept + n);
+        const int m = prune_warp<T, true>(tape, A.tape.prunable, lo, hi, mag, list, low, up);
+        for (int q = tid; q < m; q += 32) {
+          cc_op op = tape.ops[list[q]];
+          if (q == 0) op.combine = CC_COMB_PUSH;
+          kept[q] = op;
+        }
+        if (tid == 0) s_kept = m;
+      }
+      __syncthreads();
+      tape.ops = kept;
+      tape.n_ops = s_kept;
     }
   }
   T* const ring = reinterpret_cast<T*>(smem + L::slab0);
@@ -621,13 +612,6 @@ int pencil_slices(long long n0, long long n1, long long n2, bool f64) {
   return best;
 }
 
-size_t mc_prune_bytes(long long n0, long long n1, long long n2, int n_ops, bool f64) {
-  const long long tx = f64 ? Tile<double>::TX : Tile<float>::TX, ty = Tile<float>::TY;
-  const long long kz = pencil_slices(n0, n1, n2, f64);
-  const long long blocks = ((n0 + tx - 1) / tx) * ((n1 + ty - 1) / ty) * ((n2 + kz - 1) / kz);
-  return size_t(((blocks * 4 + 15) / 16) * 16 + blocks * (long long)n_ops * (long long)sizeof(cc_op));
-}
-
 namespace {
 // One fill launch. (4 CTAs per SM at Float32 was measured too: faster only while grids whose x
 // extent is not a multiple of 16 still walked a per-row copy loop; without it 3 is faster at
@@ -648,8 +632,7 @@ cudaError_t launch_fill(const McArgs<T>& a, const ColumnMaps& maps, unsigned blo
 template <class T>
 cudaError_t launch_mc(const DevGrid<T>& g, const DevTape& tape, const T* phi_in, T* phi_out,
                       const Cols& cols, const DevTable& tb, unsigned* cut_list, unsigned* cut_count,
-                      cudaStream_t s, bool with_cut, bool mixed, void* prune_scratch, size_t prune_bytes,
-                      bool count_zeroed) {
+                      cudaStream_t s, bool with_cut, bool mixed, bool count_zeroed) {
   using TL = Tile<T>;
   McArgs<T> a;
   a.g = g;
@@ -675,25 +658,13 @@ cudaError_t launch_mc(const DevGrid<T>& g, const DevTape& tape, const T* phi_in,
   cudaError_t e = count_zeroed ? cudaSuccess : cudaMemsetAsync(cut_count, 0, sizeof(unsigned), s);
   if (e != cudaSuccess) return e;
   const bool sample = phi_in == nullptr;
-  a.pruned_ops = nullptr;
-  a.pruned_count = nullptr;
-  if (sample && tape.prunable && prune_scratch && prune_bytes >= mc_prune_bytes(g.n[0], g.n[1], g.n[2], tape.n_ops, sizeof(T) == 8)) {
-    int* cnt = static_cast<int*>(prune_scratch);
-    cc_op* ops = reinterpret_cast<cc_op*>(static_cast<unsigned char*>(prune_scratch) + ((blocks * 4 + 15) / 16) * 16);
-    const int psm = PruneSmem::of(tape, 0).end;
-    if (psm > 48 * 1024) {
-      e = cudaFuncSetAttribute(prune_pencils_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, psm);
-      if (e != cudaSuccess) return e;
-    }
-    prune_pencils_kernel<T><<<unsigned(blocks), 256, psm, s>>>(a, ops, cnt);
-    a.pruned_ops = ops;
-    a.pruned_count = cnt;
-  }
-  const int sm = smem_bytes<T>(sample ? tape.bytes_len : 0);
+  const bool pruned = sample && tape.prunable;
+  int sm = smem_bytes<T>(sample ? tape.bytes_len : 0);
+  if (pruned) sm += tape.n_ops * int(sizeof(cc_op) + sizeof(unsigned));
   const int cut_blocks = 148 * 16;
   // the FP64 islands of mixed precision exist for Float32 caches only
   const bool mx = mixed && sizeof(T) == 4;
-  if (sample && a.pruned_ops) {
+  if (pruned) {
     e = launch_fill<T, true, true>(a, maps, unsigned(blocks), sm, s);
     if (e != cudaSuccess) return e;
     if (with_cut && mx) mc_cut_kernel<T, true, true><<<cut_blocks, CUT_NT, 0, s>>>(a);
@@ -714,9 +685,9 @@ cudaError_t launch_mc(const DevGrid<T>& g, const DevTape& tape, const T* phi_in,
 
 template cudaError_t launch_mc<float>(const DevGrid<float>&, const DevTape&, const float*, float*,
                                       const Cols&, const DevTable&, unsigned*, unsigned*, cudaStream_t, bool, bool,
-                                      void*, size_t, bool);
+                                      bool);
 template cudaError_t launch_mc<double>(const DevGrid<double>&, const DevTape&, const double*, double*,
                                        const Cols&, const DevTable&, unsigned*, unsigned*, cudaStream_t, bool, bool,
-                                       void*, size_t, bool);
+                                       bool);
 
 }  // namespace cci

@@ -26,12 +26,31 @@ def _spheres(k, smooth=None):
     return cc.SmoothUnion(*s, k=smooth) if smooth else cc.Union(*s)
 
 
+def _mixed(k):
+    """Primitives of every kind that evaluates alike on host and device, some far from the grid."""
+    rng = np.random.default_rng(k)
+    out = []
+    for i in range(k):
+        c = tuple(rng.uniform(-0.5, 1.5, 3))
+        if i % 4 == 0:
+            out.append(cc.Box(c, tuple(rng.uniform(0.02, 0.2, 3))))
+        elif i % 4 == 1:
+            out.append(cc.Torus(c, 0.2, 0.05, cc.quat_to_matrix(rng.normal(size=4)) * rng.uniform(0.5, 2.0)))
+        elif i % 4 == 2:
+            out.append(cc.Plane((c[0], c[1], -0.3), (0.1 * c[0], 0.2, 1.5)))
+        else:
+            out.append(cc.Sphere(c, float(rng.uniform(0.02, 0.15))))
+    return out + [cc.Const(0.4)]
+
+
 def _bodies():
     sphere, box = cc.Sphere((0.3, 0.25, 0.4), 0.22), cc.Box((0.45, 0.35, 0.5), (0.2, 0.12, 0.3))
     torus = cc.Torus((0.5, 0.4, 0.3), 0.25, 0.08, cc.quat_to_matrix((0.8, 0.1, -0.5, 0.3)))
     return {
         "spheres_2": _spheres(2), "spheres_33": _spheres(33), "spheres_200": _spheres(200),
         "smooth_5": _spheres(5, 0.08), "smooth_70": _spheres(70, 0.05),
+        "union": cc.Union(sphere, box, torus),
+        "union_long": cc.Union(*_mixed(45)),
         "one_sphere": sphere, "plane": cc.Plane((0.4, 0.3, 0.5), (0.6, -0.64, 0.48)),
         "select": cc.Subtraction(cc.Union(sphere, box, torus), cc.Intersection(cc.Sphere((0.5, 0.4, 0.5), 0.15), box)),
         "negated": cc.Negate(cc.Union(cc.Negate(cc.Intersection(sphere, torus)), box)),
@@ -85,3 +104,19 @@ def test_calc_volume_is_the_sum_of_the_cell_fractions(name, pname, prec):
         pd = float(T(h) * T(h) * T(h))
         v = cc.calc_volume(tape, g, dtype=dtype, precision="mixed" if prec == 2 else "plain")
         assert abs(v / pd - math.fsum(frac.tolist())) <= tol, (name, n)
+
+
+@pytest.mark.parametrize("name", ["union", "union_long", "spheres_33", "spheres_200", "smooth_70"])
+@pytest.mark.parametrize("pname,prec", PREC)
+def test_marching_cubes_of_pruned_unions_bitwise(name, pname, prec):
+    """The fill evaluates a pencil's nodes with the ops it keeps: phi and every column as the oracle's whole
+    tape gives them, at sizes around the pencil and far from the origin."""
+    dtype = torch.float64 if prec == 1 else torch.float32
+    tape = cc.flatten(_bodies()[name], 3)
+    for n, x0 in [((1, 1, 1), 0.0), ((33, 9, 5), -0.07), ((31, 17, 66), 0.0), ((64, 24, 35), -0.02), ((20, 20, 20), 300.0)]:
+        g = cc.CartesianGrid((x0, 0.03, -0.02), n, (1.0 / max(n),) * 3)
+        c = cc.allocate_cache(g, cc.MarchingCubesCutCell(), dtype=dtype, precision="mixed" if prec == 2 else "plain")
+        cc.update_cache(c, tape, g)
+        phi, ref = po.mc_update(g, tape, cc.mc_tables.project_table(), prec)
+        assert np.array_equal(bits(c.phi.cpu().numpy()), bits(phi)), n
+        assert_cells_bitwise(c.to_host(), ref, label=f"{name} {n}")
