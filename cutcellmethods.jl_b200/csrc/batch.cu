@@ -11,7 +11,8 @@
 // the one tile that owns it), then builds every cell from those values. Per leaf chunk each
 // thread samples its leaf's four corners and builds the leaf. Every cell's arithmetic is the
 // single-update kernels' (ms.cu), so a batched update is bit-identical to the same update run
-// alone, whatever the launch shape.
+// alone, whatever the launch shape. Where the shape allows, a warp takes a tile by itself
+// (ms_batch_warp_kernel); the rest of this describes the CTA kernel.
 //
 // cc_batch_run replays a CUDA graph: the upload of the bodies' op-tapes (from pinned staging, so a
 // body moved with cc_batch_set_body is picked up by the next replay), the counter reset and the
@@ -27,14 +28,13 @@
 #include "cc_device.cuh"
 #include "cc_internal.h"
 #include "ms_cell.cuh"
+#include "ms_tile.cuh"
 
 namespace {
 
 using namespace ccd;
 using namespace ccms;
 
-// get_node's coordinate x0 + T(i) d from a 32-bit index: T(i) is the same value as from 64 bits.
-template <class T> __device__ __forceinline__ T node_coord_i(T x0, T d, int i) { return x0 + T(i) * d; }
 using cci::Cols;
 
 // One update as the kernel sees it.
@@ -60,6 +60,7 @@ struct BatchArgs {
   unsigned long long* counter;
   long long total_tiles;
   int tape_smem;  // bytes reserved for one op-tape in shared memory
+  int warp_smem;  // ms_batch_warp_kernel: bytes per warp, its op-tape and then its nodes
   int band;       // band compaction: percent of a tile's cells (0 never, 100 always)
 };
 
@@ -69,6 +70,20 @@ __device__ __forceinline__ int find_item(const BatchItem* items, int n, long lon
     const int mid = (lo + hi + 1) >> 1;
     if (items[mid].tile_begin <= tile) lo = mid;
     else hi = mid - 1;
+  }
+  return lo;
+}
+
+// The same by a whole warp, 32 probes at a time: two dependent loads for up to 1024 items.
+__device__ __forceinline__ int find_item_warp(const BatchItem* items, int n, long long tile) {
+  const int lane = threadIdx.x & 31;
+  int lo = 0;
+  while (n > 1) {
+    const int stride = (n + 31) / 32, at = lane * stride;
+    const unsigned b = __ballot_sync(0xffffffffu, at < n && items[lo + at].tile_begin <= tile);
+    const int hit = 31 - __clz(b);  // lane 0's probe always holds
+    lo += hit * stride;
+    n = n - hit * stride < stride ? n - hit * stride : stride;
   }
   return lo;
 }
@@ -201,26 +216,82 @@ __global__ void __launch_bounds__(256) ms_batch_kernel(const BatchArgs A) {
       } else {
         // one chunk of tree leaves, a leaf per thread (as ms_tree_kernel)
         const long long l = lt * nt + threadIdx.x;
-        if (l < I.n0) {
-          const T x00 = T(I.x0[0]), x01 = T(I.x0[1]);
-          const int lv = I.level[l];
-          const T scale = T(ldexp(1.0, -lv));
-          const T h[2] = {T(I.d[0]) * scale, T(I.d[1]) * scale};
-          const long long cx = I.coord[2 * l], cy = I.coord[2 * l + 1];
-          const T xa = x00 + T(cx) * h[0], xb = x00 + T(cx + 1) * h[0];
-          const T ya = x01 + T(cy) * h[1], yb = x01 + T(cy + 1) * h[1];
-          const T nd[4][2] = {{xa, ya}, {xb, ya}, {xb, yb}, {xa, yb}};
-          T* phi4 = static_cast<T*>(I.phi);
-          T ph[4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            ph[q] = tape_eval<T, 2, T>(tp, nd[q]);
-            phi4[4 * l + q] = ph[q];
-          }
-          ms_cell<T, MX>(nd, ph, h, I.cols, l);
-        }
+        if (l < I.n0)
+          ms_leaf<T, MX>(tp, T(I.x0[0]), T(I.x0[1]), T(I.d[0]), T(I.d[1]), I.level[l], I.coord[2 * l], I.coord[2 * l + 1],
+                         static_cast<T*>(I.phi), I.cols, l);
       }
       __syncthreads();  // the next tile overwrites the node values this one's cells read
+    }
+  }
+}
+
+// The same work list with a warp, not a CTA, per tile: for tiles of whole 32-cell strips, without band
+// compaction, while a warp's tape and strip fit its share of shared memory (warp_tiles). The work list then
+// holds strips of 32 x tile_y cells, whatever tile_x, and chunks of 32 leaves. 35% of the CTA kernel's instructions. What
+// bounds it is where the stores go: with each warp popping for itself the tiles in flight were spread so
+// far that their half-written sectors left L2 (DRAM reads of 165-300 MB, 700-900 us); side by side in a CTA
+// there are none. More warps do not help: 3 CTAs of 256 per SM at Float32 (4: 578 us; 2: 452), 2 at
+// Float64. 96 moving circles on 64^2..1024^2 grids, 32 x 8 tiles and tuned, against the CTA kernel: Float32
+// 825 -> 443 us and 516 -> 408, Float64 1628 -> 884 and 985 -> 814.
+template <class T, bool MX>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) ms_batch_warp_kernel(const BatchArgs A) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int lane = threadIdx.x & 31;
+  unsigned char* own = smem + (threadIdx.x >> 5) * A.warp_smem;
+  unsigned char* strip = own + A.tape_smem;
+  // the warp's current item: read once per change of item, a word a lane (every global load waits behind
+  // the stores, some thousand cycles)
+  __shared__ __align__(16) BatchItem s_item[8];
+  BatchItem& I = s_item[threadIdx.x >> 5];
+  // The CTA pops chunk tiles per warp at a time, and its warps take them side by side: consecutive tiles are
+  // neighbours along x, so the CTA writes long row segments and few sectors are left half written for a
+  // later CTA. The next pop is asked for before the current tiles are worked on.
+  __shared__ long long s_first[2];
+  const int warps = blockDim.x >> 5, step = A.chunk * warps;
+  auto ask = [&]() { return threadIdx.x == 0 ? atomicAdd(A.counter, (unsigned long long)step) : 0ull; };
+  int turn = 0;
+  long long begin = 0, end = 0;  // its tiles
+  STape<T> tp{nullptr, nullptr, 0};
+  unsigned long long asked = ask();
+  for (;;) {
+    if (threadIdx.x == 0) s_first[turn] = (long long)asked;
+    __syncthreads();
+    const long long first = s_first[turn];
+    turn ^= 1;
+    if (first >= A.total_tiles) break;
+    const long long last = first + step < A.total_tiles ? first + step : A.total_tiles;
+    asked = ask();
+    for (long long tile = first + (threadIdx.x >> 5); tile < last; tile += warps) {
+      if (tile < begin || tile >= end) {
+        const int cur = find_item_warp(A.items, A.n_items, tile);
+        __syncwarp();
+        static_assert(sizeof(BatchItem) % 8 == 0 && sizeof(BatchItem) / 8 <= 32, "one 8-byte word per lane");
+        if (lane < int(sizeof(BatchItem) / 8))
+          reinterpret_cast<unsigned long long*>(&I)[lane] = reinterpret_cast<const unsigned long long*>(A.items + cur)[lane];
+        const long long after = cur + 1 < A.n_items ? A.items[cur + 1].tile_begin : A.total_tiles;
+        __syncwarp();
+        begin = I.tile_begin;
+        end = after;
+        const int ops_bytes = tape_ops_bytes(I.n_ops), words = (ops_bytes + I.n_params * int(sizeof(T)) + 7) / 8;
+        const unsigned long long* src = reinterpret_cast<const unsigned long long*>(A.tapes + I.tape_off);
+        for (int v = lane; v < words; v += 32) reinterpret_cast<unsigned long long*>(own)[v] = __ldg(src + v);
+        tp.ops = reinterpret_cast<const cc_op*>(own);
+        tp.p = reinterpret_cast<const T*>(own + ops_bytes);
+        tp.n_ops = I.n_ops;
+        __syncwarp();
+      }
+      const long long lt = tile - begin;
+      if (I.kind == 0) {
+        const unsigned ltu = unsigned(lt), row = ltu / unsigned(I.tiles_x);  // 32-bit: tiles of one grid
+        const int n0 = int(I.n0), n1 = int(I.n1), i0 = int(ltu - row * unsigned(I.tiles_x)) * STRIP, j0 = int(row) * A.ty;
+        ms_strip<T, MX, true, int>(tp, T(I.x0[0]), T(I.x0[1]), T(I.d[0]), T(I.d[1]), n0, n1, i0, j0, A.ty, strip,
+                                   static_cast<T*>(I.phi), I.cols);
+      } else {
+        const long long l = lt * 32 + lane;
+        if (l < I.n0)
+          ms_leaf<T, MX>(tp, T(I.x0[0]), T(I.x0[1]), T(I.d[0]), T(I.d[1]), I.level[l], I.coord[2 * l], I.coord[2 * l + 1],
+                         static_cast<T*>(I.phi), I.cols, l);
+      }
     }
   }
 }
@@ -324,6 +395,15 @@ int smem_of(const cc_batch* b) {
   return tape_smem_of(b) + (nodes + 15) / 16 * 16 + list;
 }
 
+// Whether the current config runs a warp per tile: whole strips, no band compaction, and at most 64 KB of
+// tapes and strips per CTA (then at least three CTAs of eight warps fit an SM).
+int warp_smem_of(const cc_batch* b) {
+  return tape_smem_of(b) + (b->prec == CC_F64 ? strip_bytes<double>(b->cfg.tile_y) : strip_bytes<float>(b->cfg.tile_y));
+}
+bool warp_tiles(const cc_batch* b) {
+  return b->cfg.tile_x % STRIP == 0 && b->cfg.band_percent == 0 && (b->cfg.threads / 32) * warp_smem_of(b) <= 64 * 1024;
+}
+
 // Pack every body into the staging buffer and lay the work list out for the current config.
 cc_status build_layout(cc_batch* b) {
   if (b->layout_ok) return CC_OK;
@@ -337,7 +417,7 @@ cc_status build_layout(cc_batch* b) {
   size_t off = 0;
   int max_tape = 0;
   long long tiles = 0;
-  const int tx = b->cfg.tile_x, ty = b->cfg.tile_y, nt = b->cfg.threads;
+  const int ty = b->cfg.tile_y;
   // sizes first, so the staging buffer is grown once
   std::vector<size_t> sz(b->items.size());
   std::vector<int> nps(b->items.size());
@@ -349,6 +429,8 @@ cc_status build_layout(cc_batch* b) {
     if (int(sz[k]) > max_tape) max_tape = int(sz[k]);
   }
   if (off > 0x7fffffffULL) return fail(CC_TOO_LARGE, "the batch's op-tapes exceed 2 GiB");
+  b->max_tape = max_tape;
+  const int tx = warp_tiles(b) ? STRIP : b->cfg.tile_x, nt = warp_tiles(b) ? 32 : b->cfg.threads;  // nt: leaves per chunk
   if (off > b->tapes_host_cap) {
     if (b->tapes_host) cudaFreeHost(b->tapes_host);
     b->tapes_host = nullptr;
@@ -399,7 +481,6 @@ cc_status build_layout(cc_batch* b) {
     }
   }
   b->tapes_bytes = off;
-  b->max_tape = max_tape;
   b->total_tiles = tiles;
   if (smem_of(b) > 200 * 1024) return fail(CC_TOO_LARGE, "batch tile and op-tape exceed shared memory");
   const size_t ib = dev.size() * sizeof(BatchItem);
@@ -434,12 +515,18 @@ cudaError_t issue(cc_batch* b, cudaStream_t s) {
   a.counter = b->counter;
   a.total_tiles = b->total_tiles;
   a.tape_smem = tape_smem_of(b);
+  a.warp_smem = warp_smem_of(b);
   a.band = b->cfg.band_percent;
-  const int sm = smem_of(b);
+  const bool warps = warp_tiles(b);
+  const int sm = warps ? (b->cfg.threads / 32) * a.warp_smem : smem_of(b);
   const int grid = 148 * b->cfg.ctas_per_sm;
   const int nt = b->cfg.threads;
   const bool bd = a.band > 0;
-  if (b->prec == CC_F64) {
+  if (warps) {
+    if (b->prec == CC_F64) ms_batch_warp_kernel<double, false><<<grid, nt, sm, s>>>(a);
+    else if (b->prec == CC_MIXED) ms_batch_warp_kernel<float, true><<<grid, nt, sm, s>>>(a);
+    else ms_batch_warp_kernel<float, false><<<grid, nt, sm, s>>>(a);
+  } else if (b->prec == CC_F64) {
     if (bd) ms_batch_kernel<double, false, true><<<grid, nt, sm, s>>>(a);
     else ms_batch_kernel<double, false, false><<<grid, nt, sm, s>>>(a);
   } else if (b->prec == CC_MIXED) {
@@ -454,8 +541,14 @@ cudaError_t issue(cc_batch* b, cudaStream_t s) {
 
 // The kernel's dynamic shared-memory limit for the current layout (set outside any capture).
 cudaError_t prepare_kernel(const cc_batch* b) {
-  const int sm = smem_of(b);
   const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  if (warp_tiles(b)) {
+    const int wsm = (b->cfg.threads / 32) * warp_smem_of(b);
+    if (b->prec == CC_F64) return cudaFuncSetAttribute(ms_batch_warp_kernel<double, false>, at, wsm);
+    if (b->prec == CC_MIXED) return cudaFuncSetAttribute(ms_batch_warp_kernel<float, true>, at, wsm);
+    return cudaFuncSetAttribute(ms_batch_warp_kernel<float, false>, at, wsm);
+  }
+  const int sm = smem_of(b);
   const bool bd = b->cfg.band_percent > 0;
   if (b->prec == CC_F64)
     return bd ? cudaFuncSetAttribute(ms_batch_kernel<double, false, true>, at, sm)
@@ -602,7 +695,8 @@ cc_status cc_batch_set_config(cc_batch* b, const cc_batch_config* cfg) {
   cc_status st = check_config(cfg);
   if (st != CC_OK) return st;
   if ((st = wait_pending(b)) != CC_OK) return st;
-  const bool layout = cfg->tile_x != b->cfg.tile_x || cfg->tile_y != b->cfg.tile_y || cfg->threads != b->cfg.threads;
+  const bool layout = cfg->tile_x != b->cfg.tile_x || cfg->tile_y != b->cfg.tile_y || cfg->threads != b->cfg.threads ||
+                      (cfg->band_percent > 0) != (b->cfg.band_percent > 0);  // strips or tiles (warp_tiles)
   b->cfg = *cfg;
   if (layout) b->layout_ok = false;
   b->graph_ok = false;

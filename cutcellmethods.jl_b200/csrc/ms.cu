@@ -1,14 +1,16 @@
 // ms.cu -- MarchingSquaresCutCell update_cache! on sm_100a: a grid (nodal phi block) and the
 // leaves of an AdaptiveMesh{2} quadtree.
 //
-// Grid: one pass samples every node from the op-tape (the reference's _sample_nodes_kernel!,
-// src/marching_squares/cache.jl:67-70), a second builds every cell from its four corners
-// (_nodal_cells_kernel!, :75-78). Tree: one thread per leaf samples its four lattice corners and
-// builds its moments from exactly those (_leaf_cells_kernel!, :129-137).
+// Grid: a warp per strip of 32 cells by a few rows samples its nodes from the op-tape and builds its cells
+// from them (the reference's _sample_nodes_kernel!, src/marching_squares/cache.jl:67-70, and
+// _nodal_cells_kernel!, :75-78, in one pass). Tree: one thread per leaf samples its four lattice corners
+// and builds its moments from exactly those (_leaf_cells_kernel!, :129-137).
 #include <cstdint>
+#include <type_traits>
 #include "cc_device.cuh"
 #include "cc_internal.h"
 #include "ms_cell.cuh"
+#include "ms_tile.cuh"
 
 namespace {
 
@@ -20,49 +22,29 @@ using cci::DevTape;
 
 constexpr int NT = 256;
 
-// (i, j) of item v of an n0-wide box: a 32-bit quotient where the box has fewer than 2^32 items
-// (every grid that fits a device), else 64-bit.
-__device__ __forceinline__ void split2(long long v, long long n0, bool small, long long& i, long long& j) {
-  if (small) {
-    const unsigned q = unsigned(v) / unsigned(n0);
-    j = q;
-    i = (long long)(unsigned(v) - q * unsigned(n0));
-  } else {
-    j = v / n0;
-    i = v - j * n0;
-  }
-}
+constexpr int GRID_NT = 128;  // four warps, each with its own strips
 
-
-template <class T>
-__global__ void __launch_bounds__(NT) ms_sample_kernel(const DevGrid<T> g, const DevTape tape, T* phi) {
+// SAMPLE: phi is written from the tape; else it holds the nodal values. I: the grid's index type. A strip per
+// warp, strips numbered x fastest. Sampling and cells used to be two kernels with phi in between: 2000 x 1500
+// Float32 43 -> 32 us; 200 x 200 Float64, bound by one cut cell's latency, 6.3 -> 6.5 us with one launch less.
+template <class T, bool MX, bool SAMPLE, class I>
+__global__ void __launch_bounds__(GRID_NT, sizeof(T) == 4 ? 8 : 4) ms_grid_kernel(const DevGrid<T> g, const DevTape tape, T* phi, const Cols cols,
+                                                          int ty) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const STape<T> t = load_tape<T>(tape.bytes, tape.n_ops, tape.n_params, smem);
-  __syncthreads();
-  const long long nx = g.n[0] + 1, ny = g.n[1] + 1, total = nx * ny;
-  const bool small = total + (long long)gridDim.x * NT < (1LL << 32);
-  for (long long v = blockIdx.x * (long long)NT + threadIdx.x; v < total; v += (long long)gridDim.x * NT) {
-    long long i, j;
-    split2(v, nx, small, i, j);
-    const T x[2] = {node_coord(g.x0[0], g.d[0], i), node_coord(g.x0[1], g.d[1], j)};
-    phi[v] = tape_eval<T, 2, T>(t, x);
+  STape<T> t{nullptr, nullptr, 0};
+  if (SAMPLE) {
+    t = load_tape<T>(tape.bytes, tape.n_ops, tape.n_params, smem);
+    __syncthreads();
   }
-}
-
-template <class T, bool MX>
-__global__ void __launch_bounds__(NT) ms_cells_kernel(const DevGrid<T> g, const T* __restrict__ phi, const Cols cols) {
-  const long long n0 = g.n[0], n1 = g.n[1], nx = n0 + 1, total = n0 * n1;
-  const T cs[2] = {g.d[0], g.d[1]};
-  const bool small = total + (long long)gridDim.x * NT < (1LL << 32);
-  for (long long ci = blockIdx.x * (long long)NT + threadIdx.x; ci < total; ci += (long long)gridDim.x * NT) {
-    long long i, j;
-    split2(ci, n0, small, i, j);
-    const T xa = node_coord(g.x0[0], g.d[0], i), xb = node_coord(g.x0[0], g.d[0], i + 1);
-    const T ya = node_coord(g.x0[1], g.d[1], j), yb = node_coord(g.x0[1], g.d[1], j + 1);
-    const T nd[4][2] = {{xa, ya}, {xb, ya}, {xb, yb}, {xa, yb}};
-    const long long b = i + nx * j;
-    const T ph[4] = {phi[b], phi[b + 1], phi[b + nx + 1], phi[b + nx]};
-    ms_cell<T, MX>(nd, ph, cs, cols, ci);
+  const int w = threadIdx.x >> 5;
+  unsigned char* own = smem + (SAMPLE ? ((tape.bytes_len + 15) / 16) * 16 : 0) + w * strip_bytes<T>(ty);
+  const I n0 = I(g.n[0]), n1 = I(g.n[1]);
+  const unsigned long long nsx = ((unsigned long long)n0 + STRIP - 1) / STRIP, nsy = ((unsigned long long)n1 + ty - 1) / ty;
+  for (unsigned long long s = blockIdx.x * (unsigned long long)(GRID_NT / 32) + w; s < nsx * nsy;
+       s += gridDim.x * (unsigned long long)(GRID_NT / 32)) {
+    const unsigned long long sy = nsx * nsy < (1ull << 32) ? unsigned(s) / unsigned(nsx) : s / nsx;
+    ms_strip<T, MX, SAMPLE, I>(t, g.x0[0], g.x0[1], g.d[0], g.d[1], n0, n1, I((s - sy * nsx) * STRIP), I(sy * ty), ty,
+                               own, phi, cols);
   }
 }
 
@@ -75,20 +57,7 @@ __global__ void __launch_bounds__(NT) ms_tree_kernel(const T x00, const T x01, c
   const STape<T> t = load_tape<T>(tape.bytes, tape.n_ops, tape.n_params, smem);
   __syncthreads();
   for (long long i = blockIdx.x * (long long)NT + threadIdx.x; i < nl; i += (long long)gridDim.x * NT) {
-    const int lv = level[i];
-    const T scale = T(ldexp(1.0, -lv));
-    const T h[2] = {T(bd0) * scale, T(bd1) * scale};
-    const long long cx = coord[2 * i], cy = coord[2 * i + 1];
-    const T xa = x00 + T(cx) * h[0], xb = x00 + T(cx + 1) * h[0];
-    const T ya = x01 + T(cy) * h[1], yb = x01 + T(cy + 1) * h[1];
-    const T nd[4][2] = {{xa, ya}, {xb, ya}, {xb, yb}, {xa, yb}};
-    T ph[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      ph[q] = tape_eval<T, 2, T>(t, nd[q]);
-      phi4[4 * i + q] = ph[q];
-    }
-    ms_cell<T, MX>(nd, ph, h, cols, i);
+    ms_leaf<T, MX>(t, x00, x01, T(bd0), T(bd1), level[i], coord[2 * i], coord[2 * i + 1], phi4, cols, i);
   }
 }
 
@@ -105,15 +74,33 @@ namespace cci {
 template <class T>
 cudaError_t launch_ms(const DevGrid<T>& g, const DevTape& tape, const T* phi_in, T* phi_out,
                       const Cols& cols, cudaStream_t s, bool mixed) {
-  const T* phi = phi_in;
-  if (!phi_in) {
-    const int sm = ((tape.bytes_len + 15) / 16) * 16;
-    ms_sample_kernel<T><<<grid_blocks((g.n[0] + 1) * (g.n[1] + 1)), NT, sm, s>>>(g, tape, phi_out);
-    phi = phi_out;
+  // eight rows per strip, fewer while that leaves SMs without warps (the strip's one extra node row
+  // then costs more, latency less)
+  int ty = 8;
+  const long long nsx = (g.n[0] + STRIP - 1) / STRIP;
+  while (ty > 1 && nsx * ((g.n[1] + ty - 1) / ty) < 148 * 8) ty /= 2;
+  const long long strips = nsx * ((g.n[1] + ty - 1) / ty), ctas = (strips + GRID_NT / 32 - 1) / (GRID_NT / 32);
+  const unsigned blocks = unsigned(ctas < 148LL * 64 ? ctas : 148LL * 64);
+  const int sm = (phi_in ? 0 : ((tape.bytes_len + 15) / 16) * 16) + (GRID_NT / 32) * strip_bytes<T>(ty);
+  T* phi = phi_in ? const_cast<T*>(phi_in) : phi_out;  // read only without SAMPLE
+  const bool wide = g.n[0] >= 0x7fffff00LL || g.n[1] >= 0x7fffff00LL;
+  auto run = [&](auto kernel) {
+    if (sm > 40 * 1024) {
+      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+      if (e != cudaSuccess) return e;
+    }
+    kernel<<<blocks, GRID_NT, sm, s>>>(g, tape, phi, cols, ty);
+    return cudaGetLastError();
+  };
+  auto pick = [&](auto mx) {
+    constexpr bool MX = decltype(mx)::value;
+    if (phi_in) return wide ? run(ms_grid_kernel<T, MX, false, long long>) : run(ms_grid_kernel<T, MX, false, int>);
+    return wide ? run(ms_grid_kernel<T, MX, true, long long>) : run(ms_grid_kernel<T, MX, true, int>);
+  };
+  if constexpr (sizeof(T) == 4) {
+    if (mixed) return pick(std::true_type());
   }
-  if (mixed && sizeof(T) == 4) ms_cells_kernel<T, true><<<grid_blocks(g.n[0] * g.n[1]), NT, 0, s>>>(g, phi, cols);
-  else ms_cells_kernel<T, false><<<grid_blocks(g.n[0] * g.n[1]), NT, 0, s>>>(g, phi, cols);
-  return cudaGetLastError();
+  return pick(std::false_type());
 }
 
 template <class T>
