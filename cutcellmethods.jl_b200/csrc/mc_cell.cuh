@@ -221,8 +221,16 @@ __device__ __forceinline__ void put_cell(const Stage<T>& st, long long lc, int k
   st.amb[lc] = uint8_t(amb);
   st.vf[lc] = vf;
   st.c[3 * lc] = c[0]; st.c[3 * lc + 1] = c[1]; st.c[3 * lc + 2] = c[2];
-  put_vec<T>(st.ff + 6 * lc, ff, 6);
-  put_vec<T>(st.fcl + 12 * lc, fcl, 12);
+  // wide stores where the columns allow them; a caller's need only their element's alignment
+  if (((reinterpret_cast<uintptr_t>(st.ff) & (2 * sizeof(T) - 1)) | (reinterpret_cast<uintptr_t>(st.fcl) & 15u)) == 0) {
+    put_vec<T>(st.ff + 6 * lc, ff, 6);
+    put_vec<T>(st.fcl + 12 * lc, fcl, 12);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 6; ++i) st.ff[6 * lc + i] = ff[i];
+#pragma unroll
+    for (int i = 0; i < 12; ++i) st.fcl[12 * lc + i] = fcl[i];
+  }
   st.ic[3 * lc] = ic[0]; st.ic[3 * lc + 1] = ic[1]; st.ic[3 * lc + 2] = ic[2];
 }
 
