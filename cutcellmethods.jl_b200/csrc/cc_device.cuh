@@ -641,6 +641,26 @@ __device__ __forceinline__ T sphere_at(const T* __restrict__ p, const T x[3], Sp
   h.s = dsqrt(u);
   return h.s - c[3];
 }
+// Whether the sphere's value v is below `top`, without its square root where its squared distance already
+// tells that it is not: sqrt(u) > top + r by more than 2^-18 (2^-47) of the magnitudes, the rounding of u,
+// of the root and of v being a few 2^-24 (2^-53) of them. (512^3, 64 spheres, Float32 PLIC update, where
+// two spheres of a row's box are left: 1.29 -> 1.23 ms.)
+template <class T>
+__device__ __forceinline__ bool sphere_below(const T* __restrict__ p, const T x[3], T top, SphereAt<T>& h, T& v) {
+  T c[4];
+  ldq(p, c);
+  h.d[0] = x[0] - c[0];
+  h.d[1] = x[1] - c[1];
+  h.d[2] = x[2] - c[2];
+  T u = h.d[0] * h.d[0];
+  u = u + h.d[1] * h.d[1];
+  u = u + h.d[2] * h.d[2];
+  const T reach = (top + c[3]) + (sizeof(T) == 4 ? T(0x1p-18) : T(0x1p-47)) * (dabs(top) + dabs(c[3]));
+  if (reach > T(0) && u > reach * reach) return false;
+  h.s = dsqrt(u);
+  v = h.s - c[3];
+  return v < top;
+}
 // The dual arithmetic of tape_prim's sphere on unit seeds: u's gradient is d + d per axis (the
 // other axes add signed zeros, which change no bit of a sum with a value of +0 or larger magnitude;
 // x - c is never -0 for the centroid of a cell), over 2 s.

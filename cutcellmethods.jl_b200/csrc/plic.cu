@@ -8,6 +8,7 @@
 // (src/plic/apertures.jl:112-125), so both cells of a face compute identical bits.
 #include <cmath>
 #include <cstdint>
+#include <type_traits>
 #include "cc_device.cuh"
 #include "cc_internal.h"
 
@@ -376,8 +377,8 @@ struct RowBody {
       r.v = sphere_at<T>(t.p + (list[0] & 0xffffu), x, h);
       for (int i = 1; i < m; ++i) {
         SphereAt<T> w;
-        const T v = sphere_at<T>(t.p + (list[i] & 0xffffu), x, w);
-        if (v < r.v) { r.v = v; h = w; }
+        T v;
+        if (sphere_below<T>(t.p + (list[i] & 0xffffu), x, r.v, w, v)) { r.v = v; h = w; }
       }
       sphere_grad<T>(h, r.g);
     } else if constexpr (MODE == SMOOTH) {
@@ -511,7 +512,7 @@ __device__ __forceinline__ void clip_crossed(const CrossedCell<T>* cells, int n,
 // 1.6 instead of 2.0 at 512^3) but their stores cost more: 1.44 and 1.41 against 1.33 ms. CTAs per SM: 4
 // at Float32 (3: 1.36 ms), at Float64 2 with spheres (3: 2.46 against 2.38 ms), else 3 (CSG body at
 // 150 x 97 x 131: 101 against 111 us).
-// Update at 512^3, 64 spheres, kernels: Float32 2.50 -> 1.43 ms, Float64 3.92 -> 2.50, mixed 2.75 -> 1.55;
+// Update at 512^3, 64 spheres, kernels, by that change: Float32 2.50 -> 1.43 ms, Float64 3.92 -> 2.50, mixed 2.75 -> 1.55;
 // a smooth blob at 256^3 714 -> 455 us; a CSG body at 150 x 97 x 131, Float64, 281 -> 112 us.
 template <class T, bool MX, int MODE>
 __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : (MODE == SPHERES || MODE == SMOOTH ? 2 : 3))
@@ -558,9 +559,12 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : (MODE == SPHERES || M
   uint8_t* okp = valid + row + lane;
   T* const ff0 = fp;
   const bool pairs = (reinterpret_cast<uintptr_t>(cols.ff) & (2 * sizeof(T) - 1)) == 0;
-  auto march = [&](auto&& body) {
+  // FULL: a whole row, whose stores need no bounds, in a column that takes pairs (the seven bounds tests a
+  // layer were a tenth of the issue slots: update at 512^3 Float32 1.43 -> 1.29 ms)
+  auto march = [&](auto&& body, auto full) {
+    constexpr bool FULL = decltype(full)::value;
     for (int kk = 0; kk < nk; ++kk) {
-      const T z = exact_z ? z0 + ((kf + T(kk)) + T(0.5)) * dz : centroid_coord(z0, dz, k0 + kk);
+      const T z = FULL || exact_z ? z0 + ((kf + T(kk)) + T(0.5)) * dz : centroid_coord(z0, dz, k0 + kk);
       int side;
       const PlaneFit<T, 3> pl = plane_of<T, MX>(body.at(z), g.d[0], side);
       const T frac = T(1) - pl.fraction;
@@ -570,9 +574,9 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : (MODE == SPHERES || M
       __syncwarp();
 #pragma unroll
       for (int e = 0; e < 3; ++e)
-        if (lane + 32 * e < 3 * ni) np[32 * e] = nrm[lane + 32 * e];
+        if (FULL || lane + 32 * e < 3 * ni) np[32 * e] = nrm[lane + 32 * e];
       __syncwarp();  // read before the next layer's normals are staged
-      if (in) {
+      if (FULL || in) {
         *ap = pl.a;
         *vp = frac;
         *okp = pl.valid ? 1 : 0;
@@ -581,19 +585,19 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : (MODE == SPHERES || M
       }
       // every face of a cell that its plane misses is open (1) or closed (0), all of it
       const unsigned open = __ballot_sync(0xffffffffu, side > 0);
-      if (pairs) {
+      if (FULL || pairs) {
 #pragma unroll
         for (int e = 0; e < 3; ++e) {
           const T v = (open >> cell_of[e]) & 1u ? T(1) : T(0);
-          if (cell_of[e] < ni) put_pair(fp + 2 * (lane + 32 * e), v, v);
+          if (FULL || cell_of[e] < ni) put_pair(fp + 2 * (lane + 32 * e), v, v);
         }
       } else {
         for (int e = lane; e < 6 * ni; e += 32) fp[e] = (open >> (e / 6)) & 1u ? T(1) : T(0);
       }
       // crossed cells wait until there are enough to clip their faces on full warps
-      const unsigned cross = __ballot_sync(0xffffffffu, in && side == 0);
+      const unsigned cross = __ballot_sync(0xffffffffu, (FULL || in) && side == 0);
       if (cross) {
-        if (in && side == 0) {
+        if ((FULL || in) && side == 0) {
           CrossedCell<T>& c = crossed[ncrossed + __popc(cross & ((1u << lane) - 1u))];
           c.n[0] = pl.n[0];
           c.n[1] = pl.n[1];
@@ -618,8 +622,12 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : (MODE == SPHERES || M
     }
     clip_crossed<T, MX>(crossed, ncrossed, g, ff0);
   };
-  if (MODE == SPHERES && m == 1) march(OneSphere<T>(t.p + (list[0] & 0xffffu), x, y));
-  else march(RowBody<T, MODE>{t, list, m, {x, y, T(0)}});
+  auto run = [&](auto full) {
+    if (MODE == SPHERES && m == 1) march(OneSphere<T>(t.p + (list[0] & 0xffffu), x, y), full);
+    else march(RowBody<T, MODE>{t, list, m, {x, y, T(0)}}, full);
+  };
+  if (ni == FZ_X && pairs && exact_z) run(std::true_type());
+  else run(std::false_type());
 }
 
 // 0x80 in each byte of x that is zero, nothing elsewhere (no carry crosses a byte: (b & 0x7f) +
@@ -1075,12 +1083,15 @@ cudaError_t launch_monte_carlo(const DevTape& tape, const double lo[3], const do
 namespace {
 
 // Layers per warp of the 3D fit: the pruning slab of a union of spheres, else 16; halved while the
-// launch would leave SMs without their eight CTAs, so that a small grid is not a few long columns.
+// launch would leave SMs without their eight CTAs, so that a small grid is not a few long columns. Without
+// pruning a box costs less to start and 16 CTAs are better (CSG body at 150 x 97 x 131, Float64: fit 134, 105
+// and 94 us at 4, 8 and 16; with, 64 spheres at 128^3: 43, 43 and 49).
 template <class T>
 int fit_depth(const DevGrid<T>& g, const DevTape& tape) {
   int depth = tape.prunable && tape.slab > 0 && tape.slab <= FZ_KZ ? tape.slab : 16;
   const long long tiles = ((g.n[0] + FZ_X - 1) / FZ_X) * ((g.n[1] + FZ_Y - 1) / FZ_Y);
-  while (depth > 2 && tiles * ((g.n[2] + depth - 1) / depth) < 148 * 8) depth /= 2;
+  const long long enough = 148 * (tape.prunable ? 8 : 16);
+  while (depth > 2 && tiles * ((g.n[2] + depth - 1) / depth) < enough) depth /= 2;
   return depth;
 }
 
