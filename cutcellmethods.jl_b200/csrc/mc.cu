@@ -156,6 +156,11 @@ __device__ __forceinline__ void put_uncut_z(const Stage<float>& st, int lc, floa
 // A warp copies n <= MOST contiguous elements.
 template <class E, int MOST>
 __device__ __forceinline__ void copy_row(E* __restrict__ dst, const E* __restrict__ src, int n, int lane) {
+  if (n == MOST && MOST % 32 == 0) {  // a whole row, without bounds
+#pragma unroll
+    for (int v = 0; v < MOST; v += 32) dst[v + lane] = src[v + lane];
+    return;
+  }
 #pragma unroll
   for (int v = 0; v < MOST; v += 32)
     if (v + lane < n) dst[v + lane] = src[v + lane];
@@ -226,13 +231,19 @@ __global__ void __launch_bounds__(Tile<T>::NT, Tile<T>::MINB) mc_fill_kernel(con
   const T dx = A.g.d[0], dy = A.g.d[1], dz = A.g.d[2];
   const long long nxy = nx * ny;
 
+  // Slabs are counted from the pencil's first, in 32 bits: nk + 1 of them, of which this CTA writes nown.
+  // (64-bit slab numbers and node indices, a modulo per access and all eight corners compared on every slice
+  // cost: the CSG body at 512^3 Float32 2.49 -> 2.41 ms a fill, 301 x 187 x 130 mixed 226 -> 195 us, 64 spheres
+  // at 256^3 402 -> 382; 512^3 then writes 5.9 TB/s, the output pipeline alone 6.1-6.2.)
+  const int nk = int(k1 - k0), kfirst = int(k0), nown = k1 == n2 ? nk + 1 : nk;
+
   // This thread's node slots for one sampling round of NS slabs, fixed for the whole march:
-  // which of the round's slabs, the slab index, coordinates, the node index in the z = 0 plane,
+  // which of the round's slabs, the slab index, coordinates, its place in phi (moved up NS slabs a round),
   // and whether this CTA owns (writes) the node.
   constexpr int NSL = (NS * NSLAB + NT - 1) / NT;
   int sl_s[NSL], sl_v[NSL];
   T sl_x[NSL], sl_y[NSL];
-  long long sl_g[NSL];
+  T* sl_p[NSL];
   bool sl_ok[NSL], sl_own[NSL];
 #pragma unroll
   for (int q = 0; q < NSL; ++q) {
@@ -246,44 +257,45 @@ __global__ void __launch_bounds__(Tile<T>::NT, Tile<T>::MINB) mc_fill_kernel(con
     sl_own[q] = (tx < TX || i == n0) && (ty < TY || j == n1);
     sl_x[q] = node_coord(x0, dx, i);
     sl_y[q] = node_coord(y0, dy, j);
-    sl_g[q] = i + nx * j;
+    sl_p[q] = (SAMPLE ? A.phi_out : const_cast<T*>(A.phi_in)) + (i + nx * j + nxy * (k0 + s));
   }
 
-  // One round: slabs zbase, zbase+1, ... (slot s samples slab zbase + s, for slabs <= zlast),
-  // into ring slot z % (NS + 1); phi written for owned nodes of owned slabs. `first` samples
-  // only slab zbase (the first slab of the march).
-  auto sample_round = [&](long long zbase, long long zlast, bool first) {
+  // The next round: slabs zr, zr + 1, .. (slot s samples slab zr + s, for slabs <= nk), into ring slot
+  // slab % (NS + 1); phi written for owned nodes of owned slabs.
+  int zr = 0, ring_zr = 0;  // the round's first slab, and that modulo NS + 1
+  auto sample_round = [&]() {
     T pts[NSL][3];
     T val[NSL];
     bool use[NSL];
 #pragma unroll
     for (int q = 0; q < NSL; ++q) {
-      const long long z = zbase + sl_s[q];
-      use[q] = sl_ok[q] && z <= zlast && (!first || sl_s[q] == 0);
+      const int z = zr + sl_s[q];
+      use[q] = sl_ok[q] && z <= nk;
       pts[q][0] = sl_x[q];
       pts[q][1] = sl_y[q];
-      pts[q][2] = node_coord(z0, dz, (long long)(int)z);
+      pts[q][2] = z0 + T(kfirst + z) * dz;  // node_coord
     }
     if (SAMPLE) {
       tape_eval_multi<T, 3, NSL>(tape, pts, val);
     }
 #pragma unroll
     for (int q = 0; q < NSL; ++q) {
-      if (!use[q]) continue;
-      const long long z = zbase + sl_s[q];
-      const long long gi = sl_g[q] + nxy * z;
-      T v;
-      if (SAMPLE) {
-        v = val[q];
-        const bool own_slab = z < k1 || z == n2;
-        if (own_slab && sl_own[q]) A.phi_out[gi] = v;
-      } else {
-        v = A.phi_in[gi];
+      if (use[q]) {
+        T v;
+        if (SAMPLE) {
+          v = val[q];
+          if (zr + sl_s[q] < nown && sl_own[q]) *sl_p[q] = v;
+        } else {
+          v = *sl_p[q];
+        }
+        const int r = ring_zr + sl_s[q];
+        ring[(r > NS ? r - (NS + 1) : r) * RS + sl_v[q]] = v;
       }
-      ring[(int)(z - k0) % (NS + 1) * RS + sl_v[q]] = v;
+      sl_p[q] += NS * nxy;
     }
+    zr += NS;
+    ring_zr = ring_zr == 0 ? NS : ring_zr - 1;  // + NS modulo NS + 1
   };
-
 
   const int tx = tid % TX, ty = tid / TX;
   const long long ci = i0 + tx, cj = j0 + ty;
@@ -302,40 +314,39 @@ __global__ void __launch_bounds__(Tile<T>::NT, Tile<T>::MINB) mc_fill_kernel(con
                             reinterpret_cast<unsigned char*>(A.cols.ff), reinterpret_cast<unsigned char*>(A.cols.fcl),
                             reinterpret_cast<unsigned char*>(A.cols.ic)};
 
+  // nudge_zeros(v) >= 0  <=>  v > -eps  (and false for NaN, as there)
+  const T neps = -Eps<T>::v();
+  auto outside4 = [&](const T* slab) {  // of the cell's four corners on one slab
+    return (slab[s00] > neps) + (slab[s00 + 1] > neps) + (slab[s00 + NSX + 1] > neps) + (slab[s00 + NSX] > neps);
+  };
   // What this thread's slot of each staging buffer holds: 0 not known (first use, or a cut cell,
   // whose slot the fill leaves alone), 1 an uncut cell outside, 2 inside (2 bits per buffer).
   int slots = 0;
-  for (long long k = k0; k < k1; ++k) {
-    const int sb = (int)((k - k0) & 1);
+  int below = 0, rk = 0;  // corners outside on the lower slab, and its ring slot
+  T za = z0 + T(kfirst) * dz;
+  long long k = k0;
+  for (int kk = 0; kk < nk; ++kk, ++k) {
+    const int sb = kk & 1;
     unsigned char* sbase = smem + sb * L::stage_bytes;
-    {
-      // round r samples slabs k0 + NS r .. k0 + NS r + NS - 1 before the slice that first needs its
-      // first slab; the slabs it overwrites were last read before the previous slice's barriers
-      const int kk = (int)(k - k0);
-      if (kk == 0) sample_round(k0, k1, false);
-      else if (kk % NS == NS - 1) sample_round(k + 1, k1, false);
-    }
+    // round r samples slabs NS r .. NS r + NS - 1 before the slice that first needs its first slab; the slabs
+    // it overwrites were last read before the previous slice's barriers
+    if (kk == 0 || kk % NS == NS - 1) sample_round();
     if (fast && tid == 0) bulk_wait_read<1>();  // staging buffer sb: its copy two slices ago has been read
-    __syncthreads();  // slabs k and k+1 ready; staging sb free
+    __syncthreads();  // slabs kk and kk + 1 ready; staging sb free
 
-    const T za = node_coord(z0, dz, (long long)(int)k), zb = node_coord(z0, dz, (long long)(int)(k + 1));
+    if (kk == 0) below = outside4(ring);
+    rk = rk == NS ? 0 : rk + 1;
+    const int above = outside4(ring + rk * RS), nout = below + above;
+    below = above;
+    const T zb = z0 + T(kfirst + kk + 1) * dz, zl = za;
+    za = zb;
     bool is_cut = false;
     if (valid) {
-      const int rk = (int)(k - k0) % (NS + 1);
-      const T* sa = ring + rk * RS;
-      const T* sbb = ring + (rk == NS ? 0 : rk + 1) * RS;
-      const T ph[8] = {sa[s00], sa[s00 + 1], sa[s00 + NSX + 1], sa[s00 + NSX],
-                       sbb[s00], sbb[s00 + 1], sbb[s00 + NSX + 1], sbb[s00 + NSX]};
-      // nudge_zeros(v) >= 0  <=>  v > -eps  (and false for NaN, as there)
-      const T neps = -Eps<T>::v();
-      int nout = 0;
-#pragma unroll
-      for (int q = 0; q < 8; ++q) nout += ph[q] > neps ? 1 : 0;
       const int state = nout == 8 ? 2 : (nout == 0 ? 1 : 0);
       if (state != 0) {
-        const T hz = T(0.5) * (zb - za);
+        const T hz = T(0.5) * (zb - zl);
         const T one = nout == 8 ? T(1) : T(0);
-        const T cen[3] = {cx, cy, za + T(0.5) * dz};
+        const T cen[3] = {cx, cy, zl + T(0.5) * dz};
         // (Float32 only: at Float64 the split cost more than the stores it saved, 4.91 vs 4.76 ms)
         if (sizeof(T) == 4 && ((slots >> (2 * sb)) & 3) == state) {
           if constexpr (sizeof(T) == 4) put_uncut_z(stage_at<T>(sbase), lc, cen[2], hx, hy, hz);
@@ -399,7 +410,7 @@ __global__ void __launch_bounds__(Tile<T>::NT, Tile<T>::MINB) mc_fill_kernel(con
       // the rest row by row, a warp taking the rows it staged itself: a column's part of a row is
       // contiguous, so lane-strided elements are full-width stores whatever the row's alignment. (A CTA
       // stepping through every row and column with all its threads ran mostly idle: 301 x 187 x 130
-      // mixed: fill 581 -> 228 us; 203^3 Float64: 1126 -> 434 us.) Most grids have none.
+      // mixed: fill 581 -> 226 us; 203^3 Float64: 1126 -> 434 us.) Most grids have none.
       if (A.thread_cols) {
         const int lane = tid & 31;
         for (int r = tid >> 5; r < rows; r += NT / 32) {
