@@ -52,20 +52,6 @@ constexpr int BW = MB * IPT;     // bitmap words per block (32768 nodes)
 template <class T>
 __device__ __forceinline__ bool outside(T v) { return nudge(v) >= T(0); }
 
-// Bit a set: node (i,j,k)'s edge to the next node along axis a crosses the surface.
-template <class T>
-__device__ __forceinline__ unsigned node_edges(const T* __restrict__ phi, long long i, long long j, long long k,
-                                               const long long n[3]) {
-  const long long nx = n[0] + 1, ny = n[1] + 1;
-  const long long v = i + nx * (j + ny * k);
-  const bool o = outside(phi[v]);
-  unsigned m = 0;
-  if (i < n[0] && outside(phi[v + 1]) != o) m |= 1u;
-  if (j < n[1] && outside(phi[v + nx]) != o) m |= 2u;
-  if (k < n[2] && outside(phi[v + nx * ny]) != o) m |= 4u;
-  return m;
-}
-
 // The crossing on node v's edge along axis a (world coordinates), as the cells place it.
 template <class T>
 __device__ __forceinline__ void edge_vertex(const T* __restrict__ phi, const DevGrid<T>& g, long long i, long long j,
@@ -91,10 +77,9 @@ __device__ __forceinline__ void edge_vertex(const T* __restrict__ phi, const Dev
 template <class T>
 __device__ __forceinline__ bool out_fast(T v) { return v > -Eps<T>::v(); }
 
-// The sign bitmap. Node row r = j + ny k keeps its nx nodes in W 32-bit words, bit b of word w set
-// when node i = 32 w + b is outside (bits past nx stay clear); word u = r W + w. Rows are padded to
-// whole words so that every word lies in one row: its +y and +z neighbours are the words W and
-// W ny further on, and a 32-node test is a few word operations.
+// The sign bitmap: bit v is set when node v (linear, x fastest) is outside. A row's nodes are tested 32 at
+// a time: word u = r W + w stands for nodes 32 w.. of row r = j + ny k, wherever their bits start in the
+// bitmap (row_bits).
 // Quotient and remainder of a 32-bit value by a fixed divisor d >= 1 through one multiply-high
 // (division by invariant integers, Granlund and Montgomery 1994): with m = floor((2^32 - 1) / d),
 // umulhi(u, m) is floor(u / d) or one less, and a single correction step makes it exact.
@@ -114,27 +99,38 @@ struct FastDiv {
 
 struct Signs {
   unsigned* s;
-  unsigned W, ny, words;
+  unsigned W, nx, ny, words;
   int n0, n1, n2;
   FastDiv byW, byny;
 };
 
-// One warp per node row: lane b tests node 32 w + b of each of the row's W words in turn and a
-// ballot forms the word. One load per lane in flight per warp, many warps per SM: on a 513^3
-// Float32 field this read 5.2 TB/s where batches of 4, 8 and 16 loads per lane read 4.8, 4.1 and
-// 3.5. No index needs a division.
+// A warp takes 256 consecutive nodes: eight full, aligned loads in flight, a ballot each. (Rows padded to
+// words made every load straddle two lines; a persistent grid that loads ahead is no faster. 384^3 Float32:
+// 53 -> 50 us, 4.5 TB/s.)
+constexpr int SIGN_W = 8;  // words per warp
 template <class T>
-__global__ void __launch_bounds__(256) sign_kernel(const T* __restrict__ phi, const Signs sg, unsigned nx,
-                                                   unsigned rows) {
-  const unsigned lane = threadIdx.x & 31u, r = blockIdx.x * 8u + (threadIdx.x >> 5);
-  if (r >= rows) return;  // warp-uniform
-  const T* __restrict__ row = phi + (size_t)nx * r;
-  unsigned* __restrict__ out = sg.s + (size_t)sg.W * r;
-  for (unsigned w = 0; w < sg.W; ++w) {
-    const unsigned i = 32u * w + lane;
-    const unsigned m = __ballot_sync(0xffffffffu, i < nx && out_fast(row[i < nx ? i : 0u]));
-    if (lane == 0) out[w] = m;
+__global__ void __launch_bounds__(256) sign_kernel(const T* __restrict__ phi, unsigned* __restrict__ out, unsigned nn) {
+  const unsigned lane = threadIdx.x & 31u, w0 = (blockIdx.x * 8u + (threadIdx.x >> 5)) * SIGN_W;
+  if ((unsigned long long)w0 * 32u >= nn) return;  // warp-uniform
+  T v[SIGN_W];
+#pragma unroll
+  for (int q = 0; q < SIGN_W; ++q) {
+    const unsigned long long i = 32ull * (w0 + q) + lane;
+    v[q] = i < nn ? phi[i] : -T(1);
   }
+  unsigned mine = 0;
+#pragma unroll
+  for (int q = 0; q < SIGN_W; ++q) {
+    const unsigned m = __ballot_sync(0xffffffffu, out_fast(v[q]));
+    if (lane == q) mine = m;
+  }
+  if (lane < SIGN_W) out[w0 + lane] = mine;  // the bitmap is padded to whole warps
+}
+
+// The 33 bits of nodes v, v + 1, ...
+__device__ __forceinline__ unsigned long long row_bits(const unsigned* __restrict__ s, unsigned v) {
+  const unsigned* p = s + (v >> 5);
+  return ((unsigned long long)p[0] | (unsigned long long)p[1] << 32) >> (v & 31u);
 }
 
 // The cuts of bitmap word u, one bit per node: its x, y and z edges to the next node that cross
@@ -146,25 +142,21 @@ struct Cuts {
   unsigned ax, ay, az, cell;
 };
 __device__ __forceinline__ Cuts word_cuts(const Signs& sg, unsigned u) {
-  const bool in = u < sg.words;
-  const unsigned uc = in ? u : 0u;
-  unsigned w, j;
-  const unsigned r = sg.byW.div(uc, w), k = sg.byny.div(r, j);
-  const bool hx = w + 1u < sg.W, hy = int(j) < sg.n1, hz = int(k) < sg.n2;
-  const unsigned ox = hx ? 1u : 0u, oy = hy ? sg.W : 0u, oz = hz ? sg.W * sg.ny : 0u;
-  const unsigned* p = sg.s + uc;  // every address below stays inside the bitmap
-  const unsigned A = p[0], B = p[oy], C = p[oz], D = p[oy + oz];
-  unsigned An = p[ox], Bn = p[oy + ox], Cn = p[oz + ox], Dn = p[oy + oz + ox];
-  if (!hx) An = Bn = Cn = Dn = 0u;  // the row's last word: bit 31 is past n0 and masked below
-  const int lo = sg.n0 - int(32u * w);
-  const unsigned xm = lo >= 32 ? 0xffffffffu : lo <= 0 ? 0u : (1u << lo) - 1u;  // nodes with i < n0
   Cuts c{0u, 0u, 0u, 0u};
-  if (!in) return c;
-  c.ax = (A ^ ((A >> 1) | (An << 31))) & xm;
-  c.ay = A ^ B;  // B is A itself on the last row along y, C on the last layer along z
-  c.az = A ^ C;
-  const unsigned d = (A ^ B) | (A ^ C) | (A ^ D), dn = (An ^ Bn) | (An ^ Cn) | (An ^ Dn);
-  c.cell = hy && hz ? (d | (d >> 1) | (dn << 31) | c.ax) & xm : 0u;
+  if (u >= sg.words) return c;
+  unsigned w, j;
+  const unsigned r = sg.byW.div(u, w), k = sg.byny.div(r, j);
+  const bool hy = int(j) < sg.n1, hz = int(k) < sg.n2;
+  const unsigned v = 32u * w + sg.nx * r, vy = v + (hy ? sg.nx : 0u), dz = hz ? sg.nx * sg.ny : 0u;
+  const unsigned long long A = row_bits(sg.s, v), B = row_bits(sg.s, vy), C = row_bits(sg.s, v + dz), D = row_bits(sg.s, vy + dz);
+  const int lo = sg.n0 - int(32u * w);
+  const unsigned xm = lo >= 32 ? 0xffffffffu : lo <= 0 ? 0u : (1u << lo) - 1u;    // nodes with i < n0
+  const unsigned nm = lo >= 31 ? 0xffffffffu : (1u << (lo + 1)) - 1u;             // nodes of this row
+  c.ax = unsigned(A ^ (A >> 1)) & xm;
+  c.ay = unsigned(A ^ B) & nm;  // B is A itself on the last row along y, C on the last layer along z
+  c.az = unsigned(A ^ C) & nm;
+  const unsigned long long d = (A ^ B) | (A ^ C) | (A ^ D);
+  c.cell = hy && hz ? (unsigned(d | (d >> 1)) | c.ax) & xm : 0u;
   return c;
 }
 
@@ -368,19 +360,32 @@ __global__ void __launch_bounds__(MB) cell_emit_kernel(const T* __restrict__ phi
     return;
   }
   const long long c = i + g.n[0] * (j + g.n[1] * k);
-  // the vertex of each of the cell's cut edges (code e + 1), from its lower node's numbering
+  // The vertex of each of the cell's cut edges (code e + 1), from its lower node's numbering: a node's cut
+  // edges along x, y, z in turn. An edge's rank among them takes the signs of the cell's corners and, for
+  // lower nodes on its far sides, of five nodes beyond it.
+  const long long nx = g.n[0] + 1, nxy = nx * (g.n[1] + 1), v0 = i + nx * j + nxy * k;
+  const bool hx = i + 1 < g.n[0], hy = j + 1 < g.n[1];
+  const bool ex[3] = {hx && outside(phi[v0 + 2]), hx && outside(phi[v0 + 2 + nxy]), hx && outside(phi[v0 + 2 + nx])};
+  const bool ey[2] = {hy && outside(phi[v0 + 2 * nx]), hy && outside(phi[v0 + 2 * nx + 1])};
+  constexpr int at[2][2][2] = {{{0, 4}, {3, 7}}, {{1, 5}, {2, 6}}};  // the corner of bits (x, y, z)
   unsigned vid[12];
 #pragma unroll
   for (int e = 0; e < 12; ++e) {
-    const int ca = edge_node(e, 0), cb = edge_node(e, 1);
+    const int lo = edge_node(e, 0), hi = edge_node(e, 1), a = edge_axis(e);
+    const int bx = cbit(lo, 0), by = cbit(lo, 1), bz = cbit(lo, 2);
     vid[e] = 0;
-    if ((ph[ca] >= T(0)) == (ph[cb] >= T(0))) continue;
-    const int a = cbit(ca, 0) != cbit(cb, 0) ? 0 : (cbit(ca, 1) != cbit(cb, 1) ? 1 : 2);
-    const int lo = cbit(ca, a) < cbit(cb, a) ? ca : cb;
-    const long long li = i + cbit(lo, 0), lj = j + cbit(lo, 1), lk = k + cbit(lo, 2);
-    const unsigned m = node_edges(phi, li, lj, lk, g.n);
-    const long long v = li + (g.n[0] + 1) * (lj + (g.n[1] + 1) * lk);
-    vid[e] = vbase[v] + __popc(m & ((1u << a) - 1u));
+    const bool o = ph[lo] >= T(0);
+    if (o == (ph[hi] >= T(0))) continue;
+    unsigned rank = 0;
+    if (a >= 1) {
+      if (bx == 0) rank += (ph[at[1][by][bz]] >= T(0)) != o;
+      else rank += hx && (ex[by ? 2 : bz]) != o;
+    }
+    if (a == 2) {
+      if (by == 0) rank += (ph[at[bx][1][bz]] >= T(0)) != o;
+      else rank += hy && ey[bx] != o;
+    }
+    vid[e] = vbase[v0 + bx + nx * by + nxy * bz] + rank;
   }
   unsigned centre = 0;
   if (it) {
@@ -439,6 +444,7 @@ cc_status run_mesh(cc_handle* h, const cc_grid* gg, const T* phi, T* verts, int6
   const DevGrid<T> g = grid_of<T>(gg);
   const long long nx = g.n[0] + 1, ny = g.n[1] + 1, nn = nx * ny * (g.n[2] + 1);
   const long long W = (nx + 31) / 32, words = W * ny * (g.n[2] + 1);
+  const long long bits = ((nn + 255) / 256) * SIGN_W + 2;  // bitmap words: whole warps, and row_bits' second word
   const long long nb = (words + BW - 1) / BW;
   // 32-bit node and word indices, with room for the last block's words past the end
   if (nn > 0xffffffffLL || words > 0xffffffffLL - BW)
@@ -458,7 +464,7 @@ cc_status run_mesh(cc_handle* h, const cc_grid* gg, const T* phi, T* verts, int6
   // totals, the 2 tile totals (triangles, interior vertices), the overflow flag; then the sign
   // bitmap, 32-bit words
   const size_t head = size_t(3 * nb + 6);
-  const size_t scan_n = head + size_t(words + 1) / 2;
+  const size_t scan_n = head + size_t(bits + 1) / 2;
   if (scan_n > h->mesh_scan_n) {
     if (h->mesh_scan) cudaFree(h->mesh_scan);
     h->mesh_scan = nullptr;
@@ -475,6 +481,7 @@ cc_status run_mesh(cc_handle* h, const cc_grid* gg, const T* phi, T* verts, int6
   Signs sg;
   sg.s = reinterpret_cast<unsigned*>(h->mesh_scan + head);
   sg.W = unsigned(W);
+  sg.nx = unsigned(nx);
   sg.ny = unsigned(ny);
   sg.words = unsigned(words);
   sg.n0 = int(g.n[0]);
@@ -498,8 +505,7 @@ cc_status run_mesh(cc_handle* h, const cc_grid* gg, const T* phi, T* verts, int6
   };
   if (!reuse) {
     key.valid = false;
-    const long long rows = ny * (g.n[2] + 1);
-    sign_kernel<T><<<unsigned((rows + 7) / 8), 256, 0, s>>>(phi, sg, unsigned(nx), unsigned(rows));
+    sign_kernel<T><<<unsigned((nn + 2047) / 2048), 256, 0, s>>>(phi, sg.s, unsigned(nn));
     band_count_kernel<<<unsigned(nb), MB, 0, s>>>(sg, bsum);
     cccompact::scan_series_kernel<512, 3><<<3, 512, 0, s>>>(bsum, nb, tot);
     // the list pass and the tile counts, into the lists as they are; run again below when the
@@ -516,9 +522,9 @@ cc_status run_mesh(cc_handle* h, const cc_grid* gg, const T* phi, T* verts, int6
         cudaMemsetAsync(tot2, 0, 2 * sizeof(unsigned long long), s);
       }
     };
-    unsigned long long c5[5];  // cut nodes, edge vertices, cut cells, triangles, interior vertices
+    unsigned long long* c5 = h->rep_host;  // pinned: cut nodes, edge vertices, cut cells, triangles, interior vertices
     if (h->mesh_list) list_pass();
-    if ((e = cudaGetLastError()) == cudaSuccess) e = cudaMemcpyAsync(c5, tot, sizeof c5, cudaMemcpyDeviceToHost, s);
+    if ((e = cudaGetLastError()) == cudaSuccess) e = cudaMemcpyAsync(c5, tot, 5 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(e, "generate_mesh count");
     n_nodes = c5[0];
@@ -562,7 +568,7 @@ cc_status run_mesh(cc_handle* h, const cc_grid* gg, const T* phi, T* verts, int6
   auto [nodes, tsum, cells, ntb_cap] = lists();
   (void)ntb_cap;
   const unsigned long long ntb = (n_cells + MB - 1) / MB;
-  unsigned long long flag = 0;
+  unsigned long long* flag = h->rep_host + 5;
   e = cudaMemsetAsync(overflow, 0, sizeof(unsigned long long), s);
   if (e == cudaSuccess && n_nodes > 0)
     node_emit_kernel<T><<<unsigned((n_nodes + MB - 1) / MB), MB, 0, s>>>(phi, g, nd, nodes, n_nodes, h->mesh_vbase, verts,
@@ -572,11 +578,11 @@ cc_status run_mesh(cc_handle* h, const cc_grid* gg, const T* phi, T* verts, int6
                                                         verts, (unsigned long long)vcap, tris, (unsigned long long)tcap,
                                                         tri_cells, overflow);
   if (e == cudaSuccess) e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&flag, overflow, sizeof flag, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(flag, overflow, sizeof *flag, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   key.valid = false;  // one emit per count
   if (e != cudaSuccess) return cuda_fail(e, "generate_mesh emit");
-  if (flag) return fail(CC_BAD_ARG, "generate_mesh: phi changed between the count and the emit call");
+  if (*flag) return fail(CC_BAD_ARG, "generate_mesh: phi changed between the count and the emit call");
   return CC_OK;
 }
 
