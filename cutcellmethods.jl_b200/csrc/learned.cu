@@ -658,15 +658,13 @@ __global__ void __launch_bounds__(TILE)
 }
 
 // ---------------------------------------------------------------------------------------------
-// Fused cut-band kernel with the learned correction: each CTA takes tiles of 128 listed cut cells,
-// one per thread, builds their plain moments (writing every field), then runs the network on the
-// tile and replaces the volume fraction where the correction is accepted.
+// The learned correction of the listed cut cells, whose plain moments mc_cut_kernel has written: the network on
+// tiles of 128 cells, one per thread, and the volume fraction replaced where the correction is accepted.
 template <class T>
 struct LearnedArgs {
   DevGrid<T> g;
   const T* phi;
   cci::Cols cols;
-  DevTable tb;
   const unsigned* cut_list;
   const unsigned* cut_count;
   const float* P;
@@ -676,11 +674,11 @@ struct LearnedArgs {
   long long wait_limit;
 };
 
-// BUILD: the kernel builds each listed cell's plain moments itself; without it the plain cut-band
-// kernel has already written them (mc_cut_kernel, the same construction at three times this
-// kernel's occupancy) and this kernel only reads the plain fraction back and corrects it.
-template <class T, bool BUILD>
-__global__ void __launch_bounds__(TILE) mc_cut_learned_kernel(const LearnedArgs<T> A) {
+// Bound by instruction issue: 128 GELUs a cell, each erff taking both its branches in most warps; the tensor
+// pipe is nearly idle. (Twice the warps an SM, six groups of 128 threads sharing one copy of the weights: 63
+// against 70 us for a smooth blob at 256^3, 1% of the update.)
+template <class T>
+__global__ void __launch_bounds__(TILE) mc_correct_kernel(const LearnedArgs<T> A) {
   extern __shared__ __align__(128) unsigned char smem[];
   const MlpShared s = mlp_shared(smem, false, A.wait_limit);
   const int t = threadIdx.x;
@@ -695,15 +693,7 @@ __global__ void __launch_bounds__(TILE) mc_cut_learned_kernel(const LearnedArgs<
   uint32_t phase = 0;
   const long long n0 = A.g.n[0], n1 = A.g.n[1];
   const long long nx = n0 + 1, ny = n1 + 1;
-  Stage<T> st;
-  st.kind = A.cols.kind;
-  st.amb = A.cols.amb;
-  st.vf = static_cast<T*>(A.cols.vf);
-  st.c = static_cast<T*>(A.cols.c);
-  st.ff = static_cast<T*>(A.cols.ff);
-  st.fcl = static_cast<T*>(A.cols.fcl);
-  st.ic = static_cast<T*>(A.cols.ic);
-  const T cs[3] = {A.g.d[0], A.g.d[1], A.g.d[2]};
+  T* const vf = static_cast<T*>(A.cols.vf);
   const float inv_h = 1.0f / float(A.g.d[0]);
   const long long total = *A.cut_count;
   unsigned long long fb = 0;
@@ -711,24 +701,17 @@ __global__ void __launch_bounds__(TILE) mc_cut_learned_kernel(const LearnedArgs<
   for (long long base = (long long)blockIdx.x * TILE; base < total; base += (long long)gridDim.x * TILE) {
     const long long q = base + t;
     float x[8] = {0, 0, 0, 0, 0, 0, 0, 0}, sc = 0.0f;
-    long long ci = -1;
+    unsigned ci = 0;
     T plain = T(0);
     if (q < total) {
-      ci = A.cut_list[q];
-      const long long i = ci % n0, j = (ci / n0) % n1, k = ci / (n0 * n1);
+      ci = A.cut_list[q];  // a cache has fewer than 2^32 cells: 32-bit quotients
+      const unsigned row = ci / unsigned(n0), k = row / unsigned(n1);
+      const unsigned i = ci - row * unsigned(n0), j = row - k * unsigned(n1);
       const long long b0 = i + nx * (j + ny * k);
       const long long bz = nx * ny;
       const T ph[8] = {A.phi[b0], A.phi[b0 + 1], A.phi[b0 + nx + 1], A.phi[b0 + nx],
                        A.phi[b0 + bz], A.phi[b0 + bz + 1], A.phi[b0 + bz + nx + 1], A.phi[b0 + bz + nx]};
-      if constexpr (BUILD) {
-        const T org[3] = {node_coord(A.g.x0[0], A.g.d[0], i), node_coord(A.g.x0[1], A.g.d[1], j),
-                          node_coord(A.g.x0[2], A.g.d[2], k)};
-        const T l[3] = {node_coord(A.g.x0[0], A.g.d[0], i + 1) - org[0],
-                        node_coord(A.g.x0[1], A.g.d[1], j + 1) - org[1],
-                        node_coord(A.g.x0[2], A.g.d[2], k + 1) - org[2]};
-        mc_cut_cell<T>(ph, l, org, cs, A.tb, st, ci);
-      }
-      plain = st.vf[ci];
+      plain = vf[ci];
       float xr[8];
 #pragma unroll
       for (int c = 0; c < 8; ++c) xr[c] = float(ph[c]) * inv_h;
@@ -741,7 +724,7 @@ __global__ void __launch_bounds__(TILE) mc_cut_learned_kernel(const LearnedArgs<
       const float corr = sc * CORR * (2.0f * p - 1.0f);
       const T v = plain + T(corr);
       const bool accept = isfinite(corr) && fabsf(corr) <= A.bound && v >= T(0) && v <= T(1);
-      if (accept) st.vf[ci] = v;
+      if (accept) vf[ci] = v;
       else ++fb;
     }
     tc_fence_before();
@@ -847,29 +830,20 @@ namespace cci {
 int mlp_nparam() { return NPARAM; }
 
 template <class T>
-cudaError_t launch_mc_cut_learned(const DevGrid<T>& g, const T* phi, const Cols& cols, const DevTable& tb,
-                                  const unsigned* cut_list, const unsigned* cut_count, const float* P, float bound,
-                                  unsigned long long* fallback, int* err, cudaStream_t s, bool build) {
-  LearnedArgs<T> a{g, phi, cols, tb, cut_list, cut_count, P, bound, fallback, err, wait_limit()};
-  const int sm = MlpLayout::INFER_SMEM;
-  cudaError_t e;
-  if (build) {
-    e = cudaFuncSetAttribute(mc_cut_learned_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    if (e != cudaSuccess) return e;
-    mc_cut_learned_kernel<T, true><<<148 * 3, TILE, sm, s>>>(a);
-  } else {
-    e = cudaFuncSetAttribute(mc_cut_learned_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    if (e != cudaSuccess) return e;
-    mc_cut_learned_kernel<T, false><<<148 * 3, TILE, sm, s>>>(a);
-  }
+cudaError_t launch_mc_correct(const DevGrid<T>& g, const T* phi, const Cols& cols, const unsigned* cut_list,
+                              const unsigned* cut_count, const float* P, float bound, unsigned long long* fallback,
+                              int* err, cudaStream_t s) {
+  LearnedArgs<T> a{g, phi, cols, cut_list, cut_count, P, bound, fallback, err, wait_limit()};
+  constexpr int sm = MlpLayout::INFER_SMEM;
+  cudaError_t e = cudaFuncSetAttribute(mc_correct_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  if (e != cudaSuccess) return e;
+  mc_correct_kernel<T><<<148 * 3, TILE, sm, s>>>(a);
   return cudaGetLastError();
 }
-template cudaError_t launch_mc_cut_learned<float>(const DevGrid<float>&, const float*, const Cols&, const DevTable&,
-                                                  const unsigned*, const unsigned*, const float*, float,
-                                                  unsigned long long*, int*, cudaStream_t, bool);
-template cudaError_t launch_mc_cut_learned<double>(const DevGrid<double>&, const double*, const Cols&, const DevTable&,
-                                                   const unsigned*, const unsigned*, const float*, float,
-                                                   unsigned long long*, int*, cudaStream_t, bool);
+template cudaError_t launch_mc_correct<float>(const DevGrid<float>&, const float*, const Cols&, const unsigned*, const unsigned*,
+                                              const float*, float, unsigned long long*, int*, cudaStream_t);
+template cudaError_t launch_mc_correct<double>(const DevGrid<double>&, const double*, const Cols&, const unsigned*, const unsigned*,
+                                               const float*, float, unsigned long long*, int*, cudaStream_t);
 
 // One training step's gradients: per-CTA partials in grad[tiles][NPARAM], per-CTA squared-error
 // sums in loss[tiles].
