@@ -42,7 +42,7 @@ struct DevTape {
   int bytes_len;
   int prunable = 0;  // 1: a union (MIN) of spheres, 2: a smooth union (SMIN) of spheres; see prune_union, prune_warp
   int select = 0;    // no smooth minimum: value and gradient are one primitive's (tape_eval_select)
-  int slab = 8;      // the 3D PLIC passes' pruning slab in cell layers (prune_slab)
+  int slab = 8;      // the 3D PLIC fit's pruning slab in cell layers (prune_slab)
 };
 
 // Bounds of a 3D body over all space: how fast its value can change (the Lipschitz constant), the
@@ -53,7 +53,7 @@ struct TapeBounds {
 };
 TapeBounds tape_bounds(const cc_optape* t);
 
-// The slab depth, in cell layers, over which the 3D PLIC fit and calc_volume prune a union of
+// The slab depth, in cell layers, over which the 3D PLIC fit prunes a union of
 // spheres of cell size h: about 0.6 of the median radius, rounded to 4, 8, 16 or 32 layers.
 int prune_slab(const cc_optape* t, double h);
 
@@ -108,9 +108,10 @@ cudaError_t launch_ms_tree(const T x0[2], const double base_d[2], long long nlea
                            const int32_t* level, const int32_t* coord, const DevTape& tape,
                            T* phi4, const Cols& cols, cudaStream_t s, bool mixed = false);
 
-// PLIC update: the fit pass, then the face pass. In 3D the fit records each cell's side (whether
-// its plane crosses the cell, or every face is empty or full) in `sides`, one byte per cell, for
-// the face pass; 2D takes null.
+// PLIC update. In 3D the fit pass writes every cell's one-sided face fractions and records its side
+// (whether its plane crosses the cell, or every face is empty or full) in `sides`, one byte per cell
+// and a layer to spare, from which the second pass picks the faces to resolve; in 2D the face pass
+// works from the stored planes and `sides` is null.
 template <class T, int D>
 cudaError_t launch_plic(const DevGrid<T>& g, const DevTape& tape, const Cols& cols, T* normals,
                         T* intercepts, uint8_t* valid, int8_t* sides, cudaStream_t s, bool mixed = false);
@@ -178,7 +179,7 @@ struct cc_handle {
   cci::DevTable tb{};
   unsigned* cut_list = nullptr;   // marching cubes: the cut band's cell indices (one slot per cell)
   unsigned* cut_count = nullptr;  // its length: the head of tape_dev
-  int8_t* plic_sides = nullptr;  // 3D PLIC: the fit's per-cell side bytes for the face pass
+  int8_t* plic_sides = nullptr;  // 3D PLIC: the fit's per-cell side bytes for the resolve pass
   double* vol_scratch = nullptr;  // calc_volume partials + result
   unsigned long long* rep_scratch = nullptr;  // report counters + the complement of the min's bits
   unsigned long long* rep_host = nullptr;     // pinned: the report's results read back

@@ -1,11 +1,12 @@
 // plic.cu -- PLICCutCell update_cache!, calc_volume and cut_cell_report on sm_100a.
 //
-// Fit pass (_plic_fit_kernel!, src/plic/cache.jl:96-113): per cell one forward-mode evaluation of
-// the op-tape at the centroid gives (dist, normal) -- get_sdf -- and cell_plane
-// (src/plic/plic.jl:72-88) turns it into the stored plane. Face pass
-// (_plic_face_fraction_kernel!, src/plic/cache.jl:118-162): per cell, per face, the mean of the
-// two one-sided candidates evaluated from the two cells' stored planes by the same _face_area
-// (src/plic/apertures.jl:112-125), so both cells of a face compute identical bits.
+// Fit pass (_plic_fit_kernel!, src/plic/cache.jl:96-113): per cell one evaluation of the op-tape's
+// value and gradient at the centroid gives (dist, normal) -- get_sdf -- and cell_plane
+// (src/plic/plic.jl:72-88) turns it into the stored plane. Faces (_plic_face_fraction_kernel!,
+// src/plic/cache.jl:118-162): per cell, per face, the mean of the two one-sided candidates of the two
+// cells' planes by the same _face_area (src/plic/apertures.jl:112-125), so both cells of a face hold
+// identical bits. In 3D the fit writes the one-sided fractions and a second pass resolves the faces
+// whose two cells differ; in 2D a face pass computes both sides from the stored planes.
 #include <cmath>
 #include <cstdint>
 #include <type_traits>
@@ -31,56 +32,39 @@ struct PlaneFit {
   bool valid;
 };
 
-// cell_plane, src/plic/plic.jl:72-88 (with MX the plane-cube clip runs in FP64)
-template <class T, int D, bool MX>
-__device__ __forceinline__ PlaneFit<T, D> cell_plane(const STape<T>& t, const DevGrid<T>& g, const long long idx[3]) {
-  Dual<T, D> x[D];
+// cell_plane, src/plic/plic.jl:72-88, in 2D (with MX the line-square clip runs in FP64)
+template <class T, bool MX>
+__device__ __forceinline__ PlaneFit<T, 2> cell_plane(const STape<T>& t, const DevGrid<T>& g, const long long idx[2]) {
+  Dual<T, 2> x[2];
 #pragma unroll
-  for (int a = 0; a < D; ++a) {
+  for (int a = 0; a < 2; ++a) {
     x[a].v = centroid_coord(g.x0[a], g.d[a], idx[a]);
 #pragma unroll
-    for (int b = 0; b < D; ++b) x[a].g[b] = a == b ? T(1) : T(0);
+    for (int b = 0; b < 2; ++b) x[a].g[b] = a == b ? T(1) : T(0);
   }
-  const Dual<T, D> r = tape_eval<T, D, Dual<T, D>>(t, x);
-  T s = r.g[0];
+  const Dual<T, 2> r = tape_eval<T, 2, Dual<T, 2>>(t, x);
+  const T a = T(0.5) * (r.g[0] + r.g[1]) - r.v / g.d[0];
+  PlaneFit<T, 2> pl;
+  pl.valid = !(isnan(a) || (r.g[0] == T(0) && r.g[1] == T(0)));
 #pragma unroll
-  for (int a = 1; a < D; ++a) s = s + r.g[a];
-  const T a = T(0.5) * s - r.v / g.d[0];
-  bool allzero = true;
-#pragma unroll
-  for (int q = 0; q < D; ++q) allzero = allzero && (r.g[q] == T(0));
-  PlaneFit<T, D> pl;
-  if (isnan(a) || allzero) {
-#pragma unroll
-    for (int q = 0; q < D; ++q) pl.n[q] = T(0);
-    pl.a = T(0);
-    pl.fraction = r.v <= T(0) ? T(1) : T(0);
-    pl.valid = false;
-    return pl;
-  }
-#pragma unroll
-  for (int q = 0; q < D; ++q) pl.n[q] = r.g[q];
-  pl.a = a;
-  if constexpr (D == 2) pl.fraction = gvf2m<T, MX>(r.g[0], r.g[1], a);
-  else pl.fraction = gvf3m<T, MX>(r.g[0], r.g[1], r.g[D - 1], a);
-  pl.valid = true;
+  for (int q = 0; q < 2; ++q) pl.n[q] = pl.valid ? r.g[q] : T(0);
+  pl.a = pl.valid ? a : T(0);
+  if (pl.valid) pl.fraction = gvf2m<T, MX>(r.g[0], r.g[1], a);
+  else pl.fraction = r.v <= T(0) ? T(1) : T(0);
   return pl;
 }
 
-// The cell tiles the centroid kernels work in: NT cells, 32 along x (coalesced stores), and the
-// tape pruned to the box of each tile's centroids when the body is a union of spheres.
-template <int D> struct PTile;
-template <> struct PTile<3> { static constexpr int X = 32, Y = 4, Z = 2; };
-template <> struct PTile<2> { static constexpr int X = 32, Y = 8, Z = 1; };
+// The 2D kernels' tile: NT cells, 32 along x (coalesced stores); the tape is pruned to the box of a
+// tile's centroids when the body is a union of spheres.
+constexpr int PX = 32, PY = 8;
+static_assert(PX * PY == NT, "one cell per thread");
 
 // Tile t's first cell, tiles numbered x fastest, from 32-bit quotients (a grid has far fewer
 // than 2^32 tiles: that would be 2^40 cells).
-template <int D>
-__device__ __forceinline__ void tile_origin(unsigned t, unsigned tx, unsigned ty, long long i0[3]) {
-  const unsigned a = t / tx, b = a / ty;
-  i0[0] = (long long)(t - a * tx) * PTile<D>::X;
-  i0[1] = (long long)(a - b * ty) * PTile<D>::Y;
-  i0[2] = (long long)b * PTile<D>::Z;
+__device__ __forceinline__ void tile_origin(unsigned t, unsigned tx, long long i0[2]) {
+  const unsigned a = t / tx;
+  i0[0] = (long long)(t - a * tx) * PX;
+  i0[1] = (long long)a * PY;
 }
 
 // Shared-memory layout of a centroid kernel: the tape, then the pruned ops and the bounds.
@@ -96,23 +80,23 @@ struct CentroidSmem {
   }
 };
 
-// The tape a box of cells (first cell i0, ext cells per axis, clipped to the grid) is evaluated
-// with: pruned to the box of their centroids if it can be.
-template <class T, int D>
-__device__ __forceinline__ STape<T> box_tape(const STape<T>& t, const DevTape& tape, const DevGrid<T>& g,
-                                             const long long i0[3], const int ext[3], unsigned char* smem,
-                                             int* count) {
+// The tape a tile's cells (first cell i0, clipped to the grid) are evaluated with: pruned to the box of
+// their centroids if it can be.
+template <class T>
+__device__ __forceinline__ STape<T> tile_tape(const STape<T>& t, const DevTape& tape, const DevGrid<T>& g,
+                                              const long long i0[2], unsigned char* smem, int* count) {
   if (!tape.prunable) return t;
   const CentroidSmem L = CentroidSmem::of(tape);
-  double lo[D], hi[D];
+  const int ext[2] = {PX, PY};
+  double lo[2], hi[2];
 #pragma unroll
-  for (int a = 0; a < D; ++a) {
+  for (int a = 0; a < 2; ++a) {
     const long long last = i0[a] + ext[a] - 1 < g.n[a] - 1 ? i0[a] + ext[a] - 1 : g.n[a] - 1;
     lo[a] = double(g.x0[a]) + (double(i0[a]) + 0.5) * double(g.d[a]);
     hi[a] = double(g.x0[a]) + (double(last) + 0.5) * double(g.d[a]);
   }
   cc_op* ops = reinterpret_cast<cc_op*>(smem + L.ops_off);
-  const int m = prune_union<T, D>(t, tape.prunable, lo, hi, reinterpret_cast<double*>(smem + L.ls_off),
+  const int m = prune_union<T, 2>(t, tape.prunable, lo, hi, reinterpret_cast<double*>(smem + L.ls_off),
                                   reinterpret_cast<double*>(smem + L.us_off), ops, count);
   STape<T> u = t;
   u.ops = ops;
@@ -120,38 +104,28 @@ __device__ __forceinline__ STape<T> box_tape(const STape<T>& t, const DevTape& t
   return u;
 }
 
-// The tape a tile's cells are evaluated with (a PTile box).
-template <class T, int D>
-__device__ __forceinline__ STape<T> tile_tape(const STape<T>& t, const DevTape& tape, const DevGrid<T>& g,
-                                              const long long i0[3], unsigned char* smem, int* count) {
-  const int ext[3] = {PTile<D>::X, PTile<D>::Y, PTile<D>::Z};
-  return box_tape<T, D>(t, tape, g, i0, ext, smem, count);
-}
-
-template <class T, int D, bool MX>
+template <class T, bool MX>
 __global__ void __launch_bounds__(NT) plic_fit_kernel(const DevGrid<T> g, const DevTape tape, const Cols cols,
                                                       T* normals, T* intercepts, uint8_t* valid) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_count;
   const STape<T> t = load_tape<T>(tape.bytes, tape.n_ops, tape.n_params, smem);
   __syncthreads();
-  using P = PTile<D>;
-  const long long n0 = g.n[0], n1 = g.n[1], n2 = D == 3 ? g.n[2] : 1;
-  const long long tx = (n0 + P::X - 1) / P::X, ty = (n1 + P::Y - 1) / P::Y, tz = (n2 + P::Z - 1) / P::Z;
+  const long long n0 = g.n[0], n1 = g.n[1];
+  const long long tx = (n0 + PX - 1) / PX, ty = (n1 + PY - 1) / PY;
   T* vf = static_cast<T*>(cols.vf);
-  const unsigned ntiles = unsigned(tx * ty * tz);
+  const unsigned ntiles = unsigned(tx * ty);
   for (unsigned tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    long long i0[3];
-    tile_origin<D>(tile, unsigned(tx), unsigned(ty), i0);
-    const STape<T> u = tile_tape<T, D>(t, tape, g, i0, smem, &s_count);
-    const int q = threadIdx.x;
-    const long long idx[3] = {i0[0] + q % P::X, i0[1] + (q / P::X) % P::Y, i0[2] + q / (P::X * P::Y)};
-    if (idx[0] < n0 && idx[1] < n1 && idx[2] < n2) {
-      const long long ci = idx[0] + n0 * (idx[1] + n1 * idx[2]);
-      const PlaneFit<T, D> pl = cell_plane<T, D, MX>(u, g, idx);
+    long long i0[2];
+    tile_origin(tile, unsigned(tx), i0);
+    const STape<T> u = tile_tape<T>(t, tape, g, i0, smem, &s_count);
+    const long long idx[2] = {i0[0] + threadIdx.x % PX, i0[1] + threadIdx.x / PX};
+    if (idx[0] < n0 && idx[1] < n1) {
+      const long long ci = idx[0] + n0 * idx[1];
+      const PlaneFit<T, 2> pl = cell_plane<T, MX>(u, g, idx);
       const T frac = T(1) - pl.fraction;
-#pragma unroll
-      for (int a = 0; a < D; ++a) normals[D * ci + a] = pl.n[a];
+      normals[2 * ci] = pl.n[0];
+      normals[2 * ci + 1] = pl.n[1];
       intercepts[ci] = pl.a;
       valid[ci] = pl.valid ? 1 : 0;
       vf[ci] = frac;
@@ -161,31 +135,19 @@ __global__ void __launch_bounds__(NT) plic_fit_kernel(const DevGrid<T> g, const 
   }
 }
 
-// _cell_wet + _face_area, src/plic/apertures.jl:73-125 (k is the 0-based direction)
-template <class T, int D, bool MX>
+// _cell_wet + _face_area, src/plic/apertures.jl:73-125, in 2D (k is the 0-based direction)
+template <class T, bool MX>
 __device__ __forceinline__ T face_area(const T* n, T a, T frac, bool valid, const T* cs, int k) {
   const T s = (k & 1) ? T(1) : T(0);
-  if constexpr (D == 2) {
-    const int c = k < 2 ? 0 : 1, p = k < 2 ? 1 : 0;
-    const T len = cs[p];
-    if (!valid) return frac < T(0.5) ? T(0) : len;
-    const T base = n[c] * s - a;
-    return open_fraction<T, MX>(base, base + n[p]) * len;
-  } else {
-    const int c = k >> 1;
-    const int p = c == 0 ? 1 : 0;
-    const int q = c == 2 ? 1 : 2;
-    const T U = cs[p], V = cs[q];
-    if (!valid) return frac < T(0.5) ? T(0) : U * V;
-    const T base = n[c] * s - a;
-    if (n[p] == T(0) && n[q] == T(0)) return base >= T(0) ? U * V : T(0);
-    const T solid = gvf2m<T, MX>(n[p], n[q], -base);
-    return (U * V) * (T(1) - solid);
-  }
+  const int c = k >> 1, p = 1 - c;
+  const T len = cs[p];
+  if (!valid) return frac < T(0.5) ? T(0) : len;
+  const T base = n[c] * s - a;
+  return open_fraction<T, MX>(base, base + n[p]) * len;
 }
 
 // Whether a valid 3D plane misses its cell by more than rounding, and on which side: -1 when
-// every face's face_area is 0, +1 when it is the face's full area U V, 0 when it must be computed.
+// every face's _face_area is 0, +1 when it is the face's full area U V, 0 when it must be computed.
 // Over the unit cube n . xi spans [lo, hi] = [sum min(n_i, 0), sum max(n_i, 0)]. If a - hi exceeds
 // 64 u (|n|_1 + |a|) (u the unit roundoff of T), every face has n_p x + n_q y < a - n_c s with that
 // margin, so gvf2 (whose rounding error is a few u of the same scale, in T or, mixed, in FP64
@@ -200,8 +162,6 @@ __device__ __forceinline__ int plane_side(const T n[3], T a) {
   return a - hi > tol ? -1 : (lo - a > tol ? 1 : 0);
 }
 
-__host__ __device__ constexpr int ilog2(int v) { return v <= 1 ? 0 : 1 + ilog2(v >> 1); }
-
 // m / full for a face area m of a face of area full > 0, bit for bit: an area of exactly 0 or
 // exactly full (every face the plane misses) gives m itself (0 / full keeps m's sign) or 1
 // without the division. The resolved value's halving, (a + b) / 2, is taken as (a + b) * 0.5:
@@ -209,111 +169,86 @@ __host__ __device__ constexpr int ilog2(int v) { return v <= 1 ? 0 : 1 + ilog2(v
 template <class T>
 __device__ __forceinline__ T frac_of(T m, T full) { return m == T(0) ? m : (m == full ? T(1) : m / full); }
 
-// The resolved faces (src/plic/cache.jl:118-162) in 2D (3D marches z, plic_face_z_kernel) of one tile: every cell's one-sided areas
+// The resolved faces (src/plic/cache.jl:118-162) in 2D, tile by tile: every cell's one-sided lengths
 // (_face_area, apertures.jl:73-125) computed once into shared memory, with the faces the
 // neighbouring cells outside the tile show it; each shared face is then resolved from its two
-// one-sided areas, (left / full + right / full) / 2, the same expression in the same order from
+// one-sided lengths, (left / full + right / full) / 2, the same expression in the same order from
 // either side, so the face is single-valued bit for bit. Boundary faces are one-sided.
-template <class T, int D, bool MX>
+template <class T, bool MX>
 __global__ void __launch_bounds__(NT, 6) plic_face_kernel(const DevGrid<T> g, const Cols cols, const T* __restrict__ normals,
                                                        const T* __restrict__ intercepts, const uint8_t* __restrict__ valid) {
-  using P = PTile<D>;
-  constexpr int NF = 2 * D;
-  constexpr int EXT[3] = {P::X, P::Y, P::Z};
-  constexpr int E0 = P::Y * P::Z, E1 = P::X * P::Z, E2 = P::X * P::Y;  // halo face sizes per axis
-  constexpr int HB[3] = {0, 2 * E0, 2 * E0 + 2 * E1};                  // halo base per axis
-  constexpr int NH = D == 3 ? 2 * (E0 + E1 + E2) : 2 * (E0 + E1);
-  static_assert(P::X * P::Y * P::Z == NT, "one cell per thread");
-  static_assert((P::X & (P::X - 1)) == 0 && (P::Y & (P::Y - 1)) == 0 && (P::Z & (P::Z - 1)) == 0, "powers of two");
-  constexpr int LX = ilog2(P::X), LY = ilog2(P::Y), LZ = ilog2(P::Z);
-  constexpr int LE0 = LY + LZ, LE1 = LX + LZ, LE2 = LX + LY;  // log2 of the halo face sizes
-  __shared__ T own[NF][NT];                  // one-sided areas, face-major (no bank conflicts)
+  constexpr int NF = 4;
+  constexpr int NH = 2 * (PX + PY);         // the halo: 2 PY faces along x, then 2 PX along y
+  __shared__ T own[NF][NT];                 // one-sided lengths, face-major (no bank conflicts)
   __shared__ T halo[NH];
-  __shared__ __align__(16) T res[NT * NF];   // resolved fractions, cell-major as in the column
-  const long long n[3] = {g.n[0], g.n[1], D == 3 ? g.n[2] : 1};
+  __shared__ __align__(16) T res[NT * NF];  // resolved fractions, cell-major as in the column
+  const long long n[2] = {g.n[0], g.n[1]};
   const T* vf = static_cast<const T*>(cols.vf);
   T* ff = static_cast<T*>(cols.ff);
-  const T cs[3] = {g.d[0], g.d[1], D == 3 ? g.d[2] : T(1)};
-  const long long tx = (n[0] + P::X - 1) / P::X, ty = (n[1] + P::Y - 1) / P::Y, tz = (n[2] + P::Z - 1) / P::Z;
-  const unsigned ntiles = unsigned(tx * ty * tz);
+  const T cs[2] = {g.d[0], g.d[1]};
+  const long long tx = (n[0] + PX - 1) / PX, ty = (n[1] + PY - 1) / PY;
+  const unsigned ntiles = unsigned(tx * ty);
+  const int q = threadIdx.x, lq[2] = {q % PX, q / PX};
   for (unsigned tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    long long i0[3];
-    tile_origin<D>(tile, unsigned(tx), unsigned(ty), i0);
-    const int q = threadIdx.x;
-    const int lq[3] = {q % P::X, (q / P::X) % P::Y, q / (P::X * P::Y)};
-    const long long idx[3] = {i0[0] + lq[0], i0[1] + lq[1], i0[2] + lq[2]};
-    const bool in = idx[0] < n[0] && idx[1] < n[1] && idx[2] < n[2];
-    const long long ci = idx[0] + n[0] * (idx[1] + n[1] * idx[2]);
+    long long i0[2];
+    tile_origin(tile, unsigned(tx), i0);
+    const long long idx[2] = {i0[0] + lq[0], i0[1] + lq[1]};
+    const bool in = idx[0] < n[0] && idx[1] < n[1];
     if (in) {  // this cell's plane, read once, on all its faces
-      T nrm[D];
-#pragma unroll
-      for (int a = 0; a < D; ++a) nrm[a] = normals[D * ci + a];
+      const long long ci = idx[0] + n[0] * idx[1];
+      const T nrm[2] = {normals[2 * ci], normals[2 * ci + 1]};
       const T a = intercepts[ci], frac = vf[ci];
       const bool ok = valid[ci] != 0;
 #pragma unroll
-      for (int k = 0; k < NF; ++k) own[k][q] = face_area<T, D, MX>(nrm, a, frac, ok, cs, k);
+      for (int k = 0; k < NF; ++k) own[k][q] = face_area<T, MX>(nrm, a, frac, ok, cs, k);
     }
     // the halo: for each axis and side, the cell beyond the tile shows its face toward the tile
-    for (int h = threadIdx.x; h < NH; h += NT) {
-      int ax = 0;
-      if (D == 3 && h >= HB[2]) ax = 2;
-      else if (h >= HB[1]) ax = 1;
-      // the extents are powers of two: shifts and masks, not divisions
-      const int lE = ax == 0 ? LE0 : (ax == 1 ? LE1 : LE2);
-      const int side = (h - HB[ax]) >> lE, pos = (h - HB[ax]) & ((1 << lE) - 1);
-      const int o1 = ax == 0 ? 1 : 0, o2 = ax == 2 ? 1 : 2;  // the other two axes, increasing
-      const int lX = o1 == 0 ? LX : LY;
-      long long nb[3];
-      nb[ax] = side == 0 ? i0[ax] - 1 : i0[ax] + EXT[ax];
-      nb[o1] = i0[o1] + (pos & ((1 << lX) - 1));
-      nb[o2] = i0[o2] + (pos >> lX);
-      if (nb[ax] >= 0 && nb[ax] < n[ax] && nb[o1] < n[o1] && nb[o2] < n[o2]) {
-        const long long cj = nb[0] + n[0] * (nb[1] + n[1] * nb[2]);
-        halo[h] = face_area<T, D, MX>(normals + D * cj, intercepts[cj], vf[cj], valid[cj] != 0, cs,
-                                      side == 0 ? 2 * ax + 1 : 2 * ax);
+    if (q < NH) {
+      const int ax = q >= 2 * PY, h = ax ? q - 2 * PY : q, len = ax ? PX : PY;
+      const int side = h / len, pos = h % len;
+      long long nb[2];
+      nb[ax] = side == 0 ? i0[ax] - 1 : i0[ax] + (ax ? PY : PX);
+      nb[1 - ax] = i0[1 - ax] + pos;
+      if (nb[ax] >= 0 && nb[ax] < n[ax] && nb[1 - ax] < n[1 - ax]) {
+        const long long cj = nb[0] + n[0] * nb[1];
+        halo[q] = face_area<T, MX>(normals + 2 * cj, intercepts[cj], vf[cj], valid[cj] != 0, cs,
+                                   side == 0 ? 2 * ax + 1 : 2 * ax);
       }
     }
     __syncthreads();
     if (in) {
 #pragma unroll
       for (int k = 0; k < NF; ++k) {
-        const int c = k >> 1;
-        const int o1 = c == 0 ? 1 : 0, o2 = c == 2 ? 1 : 2;
-        T full;
-        if constexpr (D == 2) full = cs[1 - c];
-        else full = (T(1) * cs[o1]) * cs[o2];
-        const int lstride = c == 0 ? 1 : (c == 1 ? P::X : P::X * P::Y);
-        const int hpos = lq[o1] + EXT[o1] * (D == 3 ? lq[o2] : 0);
+        const int c = k >> 1, stride = c == 0 ? 1 : PX, ext = c == 0 ? PX : PY;
+        const T full = cs[1 - c];
+        const T* shown = halo + (c == 0 ? 0 : 2 * PY) + lq[1 - c];  // by the cells beyond the lower side
         const T mine = own[k][q];
         T r;
         if ((k & 1) == 0) {
-          const bool has = idx[c] >= 1;
-          const T below = lq[c] > 0 ? own[k + 1][q - lstride] : halo[HB[c] + hpos];
-          r = has ? (frac_of(below, full) + frac_of(mine, full)) * T(0.5) : frac_of(mine, full);
+          const T below = lq[c] > 0 ? own[k + 1][q - stride] : shown[0];
+          r = idx[c] >= 1 ? (frac_of(below, full) + frac_of(mine, full)) * T(0.5) : frac_of(mine, full);
         } else {
-          const bool has = idx[c] <= n[c] - 2;
-          const int Ec = c == 0 ? E0 : (c == 1 ? E1 : E2);
-          const T above = lq[c] < EXT[c] - 1 ? own[k - 1][q + lstride] : halo[HB[c] + Ec + hpos];
-          r = has ? (frac_of(mine, full) + frac_of(above, full)) * T(0.5) : frac_of(mine, full);
+          const T above = lq[c] < ext - 1 ? own[k - 1][q + stride] : shown[c == 0 ? PY : PX];
+          r = idx[c] <= n[c] - 2 ? (frac_of(mine, full) + frac_of(above, full)) * T(0.5) : frac_of(mine, full);
         }
         res[q * NF + k] = r;
       }
     }
     __syncthreads();
-    // the tile's rows leave whole: a row is P::X cells x NF values, contiguous in the column
-    const int rowcells = (int)(n[0] - i0[0] < P::X ? n[0] - i0[0] : P::X);
-    constexpr int RV = P::X * NF * int(sizeof(T)) / 16;  // 16-byte vectors per full row
-    for (int w = threadIdx.x; w < P::Y * P::Z * RV; w += NT) {
+    // the tile's rows leave whole: a row is PX cells x NF values, contiguous in the column
+    const int rowcells = (int)(n[0] - i0[0] < PX ? n[0] - i0[0] : PX);
+    constexpr int RV = PX * NF * int(sizeof(T)) / 16;  // 16-byte vectors per full row
+    for (int w = q; w < PY * RV; w += NT) {
       const int row = w / RV, v = w - row * RV;
-      const long long j = i0[1] + row % P::Y, k = i0[2] + row / P::Y;
-      if (j >= n[1] || k >= n[2]) continue;
-      const long long c0 = i0[0] + n[0] * (j + n[1] * k);
-      if (rowcells == P::X && (reinterpret_cast<uintptr_t>(ff + NF * c0) & 15u) == 0) {
-        reinterpret_cast<uint4*>(ff + NF * c0)[v] = reinterpret_cast<const uint4*>(res + row * P::X * NF)[v];
+      const long long j = i0[1] + row;
+      if (j >= n[1]) continue;
+      const long long c0 = i0[0] + n[0] * j;
+      if (rowcells == PX && (reinterpret_cast<uintptr_t>(ff + NF * c0) & 15u) == 0) {
+        reinterpret_cast<uint4*>(ff + NF * c0)[v] = reinterpret_cast<const uint4*>(res + row * PX * NF)[v];
       } else {
         constexpr int PER = 16 / int(sizeof(T));
         for (int e = v * PER; e < (v + 1) * PER; ++e)
-          if (e < rowcells * NF) ff[NF * c0 + e] = res[row * P::X * NF + e];
+          if (e < rowcells * NF) ff[NF * c0 + e] = res[row * PX * NF + e];
       }
     }
     __syncthreads();  // the next tile reuses own, halo and res
@@ -484,7 +419,7 @@ struct CrossedCell {
 };
 constexpr int CROSSED_MAX = 64;
 
-// The one-sided fractions (face_area over the full face, frac_of) of n crossed cells, one face per lane.
+// The one-sided fractions (_face_area over the full face, frac_of) of n crossed cells, one face per lane.
 template <class T, bool MX>
 __device__ __forceinline__ void clip_crossed(const CrossedCell<T>* cells, int n, const DevGrid<T>& g, T* ff) {
   const T full = (T(1) * g.d[0]) * g.d[0];  // PLIC grids are isotropic
@@ -779,24 +714,22 @@ __device__ __forceinline__ void block_ksum(KSum a, double* out) {
 }
 
 // calc_volume, src/volume.jl:29-40: every cell's cell_plane solid fraction, summed (2D).
-template <class T, int D, bool MX>
+template <class T, bool MX>
 __global__ void __launch_bounds__(NT) calc_volume_kernel(const DevGrid<T> g, const DevTape tape, double* partial) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_count;
   const STape<T> t = load_tape<T>(tape.bytes, tape.n_ops, tape.n_params, smem);
   __syncthreads();
-  using P = PTile<D>;
-  const long long n0 = g.n[0], n1 = g.n[1], n2 = D == 3 ? g.n[2] : 1;
-  const long long tx = (n0 + P::X - 1) / P::X, ty = (n1 + P::Y - 1) / P::Y, tz = (n2 + P::Z - 1) / P::Z;
+  const long long n0 = g.n[0], n1 = g.n[1];
+  const long long tx = (n0 + PX - 1) / PX, ty = (n1 + PY - 1) / PY;
   KSum acc{0.0, 0.0};
-  const unsigned ntiles = unsigned(tx * ty * tz);
+  const unsigned ntiles = unsigned(tx * ty);
   for (unsigned tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    long long i0[3];
-    tile_origin<D>(tile, unsigned(tx), unsigned(ty), i0);
-    const STape<T> u = tile_tape<T, D>(t, tape, g, i0, smem, &s_count);
-    const int q = threadIdx.x;
-    const long long idx[3] = {i0[0] + q % P::X, i0[1] + (q / P::X) % P::Y, i0[2] + q / (P::X * P::Y)};
-    if (idx[0] < n0 && idx[1] < n1 && idx[2] < n2) acc.add(double(cell_plane<T, D, MX>(u, g, idx).fraction));
+    long long i0[2];
+    tile_origin(tile, unsigned(tx), i0);
+    const STape<T> u = tile_tape<T>(t, tape, g, i0, smem, &s_count);
+    const long long idx[2] = {i0[0] + threadIdx.x % PX, i0[1] + threadIdx.x / PX};
+    if (idx[0] < n0 && idx[1] < n1) acc.add(double(cell_plane<T, MX>(u, g, idx).fraction));
     __syncthreads();
   }
   block_ksum(acc, partial + 2 * blockIdx.x);
@@ -1139,17 +1072,17 @@ cudaError_t launch_plic(const DevGrid<T>& g, const DevTape& tape, const Cols& co
   } else {  // 2D works in tiles
     const int sm = CentroidSmem::of(tape).bytes;
     if (sm > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(plic_fit_kernel<T, D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+      cudaError_t e = cudaFuncSetAttribute(plic_fit_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
       if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(plic_fit_kernel<T, D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+        e = cudaFuncSetAttribute(plic_fit_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
       if (e != cudaSuccess) return e;
     }
     if (mixed && sizeof(T) == 4) {
-      plic_fit_kernel<T, D, true><<<blocks_for(total, 16), NT, sm, s>>>(g, tape, cols, normals, intercepts, valid);
-      plic_face_kernel<T, D, true><<<blocks_for(total, 16), NT, 0, s>>>(g, cols, normals, intercepts, valid);
+      plic_fit_kernel<T, true><<<blocks_for(total, 16), NT, sm, s>>>(g, tape, cols, normals, intercepts, valid);
+      plic_face_kernel<T, true><<<blocks_for(total, 16), NT, 0, s>>>(g, cols, normals, intercepts, valid);
     } else {
-      plic_fit_kernel<T, D, false><<<blocks_for(total, 16), NT, sm, s>>>(g, tape, cols, normals, intercepts, valid);
-      plic_face_kernel<T, D, false><<<blocks_for(total, 16), NT, 0, s>>>(g, cols, normals, intercepts, valid);
+      plic_fit_kernel<T, false><<<blocks_for(total, 16), NT, sm, s>>>(g, tape, cols, normals, intercepts, valid);
+      plic_face_kernel<T, false><<<blocks_for(total, 16), NT, 0, s>>>(g, cols, normals, intercepts, valid);
     }
   }
   return cudaGetLastError();
@@ -1208,13 +1141,13 @@ cudaError_t launch_calc_volume(const DevGrid<T>& g, const DevTape& tape, const T
   } else {
     const int sm = CentroidSmem::of(tape).bytes;
     if (sm > 48 * 1024) {
-      e = cudaFuncSetAttribute(calc_volume_kernel<T, D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+      e = cudaFuncSetAttribute(calc_volume_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
       if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(calc_volume_kernel<T, D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+        e = cudaFuncSetAttribute(calc_volume_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
       if (e != cudaSuccess) return e;
     }
-    if (mixed && sizeof(T) == 4) calc_volume_kernel<T, D, true><<<nb, NT, sm, s>>>(g, tape, partial);
-    else calc_volume_kernel<T, D, false><<<nb, NT, sm, s>>>(g, tape, partial);
+    if (mixed && sizeof(T) == 4) calc_volume_kernel<T, true><<<nb, NT, sm, s>>>(g, tape, partial);
+    else calc_volume_kernel<T, false><<<nb, NT, sm, s>>>(g, tape, partial);
   }
   calc_volume_final<<<1, NT, 0, s>>>(partial, nb, out);
   return cudaGetLastError();
