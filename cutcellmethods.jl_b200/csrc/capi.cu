@@ -413,7 +413,7 @@ cc_status cc_handle_create(int32_t device, int32_t method, int32_t dim, int32_t 
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->tape_copied, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaMalloc(&h->vol_scratch, (2 * cci::calc_volume_blocks() + 2) * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&h->rep_scratch, 8 * sizeof(unsigned long long));
-  if (e == cudaSuccess) e = cudaMallocHost(&h->rep_host, 8 * sizeof(unsigned long long));
+  if (e == cudaSuccess) e = cudaMallocHost(&h->rep_host, 24 * sizeof(unsigned long long));
 
   if (e == cudaSuccess && method == CC_MARCHING_CUBES) {
     const int64_t ncell = h->n[0] * h->n[1] * h->n[2];
@@ -644,10 +644,10 @@ cc_status cc_calc_volume(cc_handle* h, const cc_grid* g, const cc_optape* body, 
   }
   if (e != cudaSuccess) return cuda_fail(e, "calc_volume launch");
   double sum = 0.0;
-  e = cudaMemcpyAsync(h->rep_host, res, sizeof(double), cudaMemcpyDeviceToHost, s);  // pinned
+  e = cudaMemcpyAsync(h->vol_host(), res, sizeof(double), cudaMemcpyDeviceToHost, s);  // pinned
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_fail(e, "calc_volume");
-  std::memcpy(&sum, h->rep_host, sizeof(double));
+  std::memcpy(&sum, h->vol_host(), sizeof(double));
   *out = sum * pd;
   return CC_OK;
 }

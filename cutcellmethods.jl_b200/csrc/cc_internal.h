@@ -182,7 +182,11 @@ struct cc_handle {
   int8_t* plic_sides = nullptr;  // 3D PLIC: the fit's per-cell side bytes for the resolve pass
   double* vol_scratch = nullptr;  // calc_volume partials + result
   unsigned long long* rep_scratch = nullptr;  // report counters + the complement of the min's bits
-  unsigned long long* rep_host = nullptr;     // pinned: the report's results read back
+  // pinned, for results read back: the report's, then calc_volume's and generate_mesh's own words (threads may
+  // be in different ones of them at once)
+  unsigned long long* rep_host = nullptr;
+  unsigned long long* vol_host() const { return rep_host + 8; }
+  unsigned long long* mesh_host() const { return rep_host + 16; }
   unsigned* mesh_vbase = nullptr;  // generate_mesh: first vertex of each node's cut edges
   size_t mesh_vbase_n = 0;
   unsigned long long* mesh_scan = nullptr;  // generate_mesh: per-block counts and offsets

@@ -522,7 +522,7 @@ cc_status run_mesh(cc_handle* h, const cc_grid* gg, const T* phi, T* verts, int6
         cudaMemsetAsync(tot2, 0, 2 * sizeof(unsigned long long), s);
       }
     };
-    unsigned long long* c5 = h->rep_host;  // pinned: cut nodes, edge vertices, cut cells, triangles, interior vertices
+    unsigned long long* c5 = h->mesh_host();  // pinned: cut nodes, edge vertices, cut cells, triangles, interior vertices
     if (h->mesh_list) list_pass();
     if ((e = cudaGetLastError()) == cudaSuccess) e = cudaMemcpyAsync(c5, tot, 5 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -568,7 +568,7 @@ cc_status run_mesh(cc_handle* h, const cc_grid* gg, const T* phi, T* verts, int6
   auto [nodes, tsum, cells, ntb_cap] = lists();
   (void)ntb_cap;
   const unsigned long long ntb = (n_cells + MB - 1) / MB;
-  unsigned long long* flag = h->rep_host + 5;
+  unsigned long long* flag = h->mesh_host() + 5;
   e = cudaMemsetAsync(overflow, 0, sizeof(unsigned long long), s);
   if (e == cudaSuccess && n_nodes > 0)
     node_emit_kernel<T><<<unsigned((n_nodes + MB - 1) / MB), MB, 0, s>>>(phi, g, nd, nodes, n_nodes, h->mesh_vbase, verts,
