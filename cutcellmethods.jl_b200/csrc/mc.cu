@@ -32,7 +32,7 @@ using cci::DevTable;
 using cci::DevTape;
 
 // Fill-kernel tile: TX cells along x (32 at Float32, 16 at Float64, so a staging buffer is about
-// 26 KB either way) by TY = 8 rows, one thread per cell, marching KZ slices along z. A slab of
+// 26 KB either way) by TY = 8 rows, one thread per cell, marching up to KZ slices along z. A slab of
 // (TX+1) x (TY+1) nodes serves TX x TY cells: 1.16 node evaluations per cell at Float32.
 template <class T> struct Tile {
   static constexpr int TX = sizeof(T) == 4 ? 32 : 16;
@@ -43,7 +43,7 @@ template <class T> struct Tile {
   static constexpr int MINB = sizeof(T) == 4 ? 3 : 3;  // Float64 at 4 spills
 };
 constexpr int NS = 4;   // node slabs sampled per round (one op-major tape pass per thread)
-constexpr int KZ = 31;  // most z slices marched per CTA: KZ + 1 = 32 node slabs, 8 sampling rounds
+constexpr int KZ = 31;  // most z slices marched per CTA: KZ + 1 = 32 node slabs, 8 sampling rounds (deepest_pencil)
 // The cut kernel: 128 threads, bounded to 5 CTAs per SM at Float32 and 3 at Float64 (its registers: 111
 // and 239 unbounded). Kernel time in us of 128 (5, 3), 256 (3, 2) and 64 (8, 4): 512^3 Float32 80, 87, 81;
 // 256^3 Float64 40, 49, 46; a wave field at 192 x 160 x 129, Float64, 136, 138, 164.
@@ -234,7 +234,8 @@ __global__ void __launch_bounds__(Tile<T>::NT, Tile<T>::MINB) mc_fill_kernel(con
   // Slabs are counted from the pencil's first, in 32 bits: nk + 1 of them, of which this CTA writes nown.
   // (64-bit slab numbers and node indices, a modulo per access and all eight corners compared on every slice
   // cost: the CSG body at 512^3 Float32 2.49 -> 2.41 ms a fill, 301 x 187 x 130 mixed 226 -> 195 us, 64 spheres
-  // at 256^3 402 -> 382; 512^3 then writes 5.9 TB/s, the output pipeline alone 6.1-6.2.)
+  // at 256^3 402 -> 382; 512^3 then writes 5.9 TB/s, the output pipeline alone 6.1-6.2. With pencils of 31
+  // slices the quicker march was slower on the largest other grids, 512^3 Float64 4.64 -> 4.74 ms; see deepest_pencil.)
   const int nk = int(k1 - k0), kfirst = int(k0), nown = k1 == n2 ? nk + 1 : nk;
 
   // This thread's node slots for one sampling round of NS slabs, fixed for the whole march:
@@ -567,14 +568,25 @@ long long device_sms() {
 // order), a pencil taking its slices plus PENCIL_OVERHEAD slice-times (its tape load, first
 // sampling round and last drain). Few waves of deep pencils leave SMs idle in the last wave: at
 // 256^3, 31-slice pencils make 5.2 waves of the 444 resident CTAs; 27-slice pencils fill 5.8.
-int pencil_slices(long long n0, long long n1, long long n2, bool f64) {
+//
+// The deepest candidate: CTAs drift apart in z by up to a pencil, and the further they do the more places each
+// column is written in at once, which memory takes more slowly; a shallow pencil pays its first sampling
+// round more often. Fill in us at most 31, 19, 15, 11 and 7 slices (CSG body; the field is given values):
+//   Float32, all columns by TMA      512^3 2414 2423 2428 2451 2490    256^3 335 324 328 326 334    -> 19
+//   Float32, some by the threads     500^3 2867 2593 2537 2548 2632    301 x 187 x 130 197 195 192 198 204    -> 15
+//   Float64, all by TMA              512^3 4744 4397 4238 4090 4225    256^3 579 555 540 531 558
+//                                    192 x 160 x 129 field 164 152 154 150 148    -> 11
+//   Float64, some by the threads     404^3 2347 2379 2408 2463 2585    -> 31
+int deepest_pencil(bool f64, bool all_tma) { return f64 ? (all_tma ? 11 : KZ) : (all_tma ? 19 : 15); }
+
+int pencil_slices(long long n0, long long n1, long long n2, bool f64, int deepest) {
   const long long tx = f64 ? Tile<double>::TX : Tile<float>::TX, ty = Tile<float>::TY;
   const long long tiles = ((n0 + tx - 1) / tx) * ((n1 + ty - 1) / ty);
   const long long slots = device_sms() * (f64 ? Tile<double>::MINB : Tile<float>::MINB);
   constexpr double PENCIL_OVERHEAD = 2.0;
-  int best = KZ;
+  int best = deepest;
   double best_t = 0;
-  for (int kz = KZ; kz >= NS - 1; kz -= NS) {
+  for (int kz = deepest; kz >= NS - 1; kz -= NS) {
     const long long layers = (n2 + kz - 1) / kz;
     const long long rem = n2 - (layers - 1) * kz;
     // groups of resident CTAs that become free at the same time: (time, count), times increasing
@@ -615,7 +627,7 @@ int pencil_slices(long long n0, long long n1, long long n2, bool f64) {
         }
       }
     }
-    if (kz == KZ || end < best_t * 0.995) {  // a shallower pencil only for a clear gain
+    if (kz == deepest || end < best_t * 0.995) {  // a shallower pencil only for a clear gain
       best = kz;
       best_t = end;
     }
@@ -662,7 +674,7 @@ cudaError_t launch_mc(const DevGrid<T>& g, const DevTape& tape, const T* phi_in,
   a.thread_cols = ~a.tma_mask & 0x7f & ~(a.byte_words ? 3 : 0);
   a.n_itiles = int((g.n[0] + TL::TX - 1) / TL::TX);
   a.n_jtiles = int((g.n[1] + TL::TY - 1) / TL::TY);
-  a.kz = pencil_slices(g.n[0], g.n[1], g.n[2], sizeof(T) == 8);
+  a.kz = pencil_slices(g.n[0], g.n[1], g.n[2], sizeof(T) == 8, deepest_pencil(sizeof(T) == 8, a.tma_mask == 0x7f));
   const long long nk = (g.n[2] + a.kz - 1) / a.kz;
   const long long blocks = (long long)a.n_itiles * a.n_jtiles * nk;
   if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
