@@ -543,14 +543,13 @@ def traffic_per_update(n):
     return (1.7377e9 + 3.9e6) * s ** 3 + 21.3e6 * s ** 2
 
 
-# Per-cell counts of the PLIC Float32 update (fit + face pass) on the 64-sphere union. Warp
-# instructions from one ncu capture at 512^3 (sm__inst_executed.sum, one pass: 1812.4 M + 1372.8 M
+# Per-cell counts of the PLIC Float32 update (fit + resolve pass) on the 64-sphere union. Warp
+# instructions from one ncu capture at 512^3 (sm__inst_executed.sum, one pass: 1076.6 M + 59.3 M
 # over 134,217,728 cells). FP32 flops (FADD + FMUL + 2 FFMA thread instructions) from a capture at
-# 256^3 (3756 M + 266 M over 16,777,216 cells), scaled to 512^3 by the two sizes' ratio of
-# instructions per cell (23.73 / 30.37).
-PLIC_F32_WARP_INSTS_PER_CELL = (1812.37e6 + 1372.79e6) / 134217728
-PLIC_F32_FLOPS_PER_CELL = (((1307.33 + 475.00 + 2 * 986.78) + (109.12 + 105.61 + 2 * 25.52)) * 1e6 / 16777216
-                           * PLIC_F32_WARP_INSTS_PER_CELL / ((316.58e6 + 192.88e6) / 16777216))
+# 256^3 (2014 M + 2 M over 16,777,216 cells), scaled to 512^3 by the two sizes' ratio of
+# instructions per cell.
+PLIC_F32_WARP_INSTS_PER_CELL = (1076.6e6 + 59.3e6) / 134217728
+PLIC_F32_FLOPS_PER_CELL = (2015.7e6 / 16777216 * PLIC_F32_WARP_INSTS_PER_CELL / (185.7e6 / 16777216))
 B200_SMS, B200_MHZ = 148, 1965.0
 
 
@@ -567,7 +566,7 @@ def plic_rooflines(cells, ms, peak_gbs, bytes_per_cell=46):
     return {"hbm_frac": hbm, "fp32_pipe_frac": fp32, "issue_frac": issue,
             "bound": max((("hbm", hbm), ("fp32 pipe", fp32), ("instruction issue", issue)), key=lambda x: x[1])[0],
             "fp32_flops_per_cell": PLIC_F32_FLOPS_PER_CELL, "warp_instructions_per_cell": PLIC_F32_WARP_INSTS_PER_CELL,
-            "counts_source": "ncu: instructions at 512^3, flops at 256^3 scaled (profiles/plic_fit_face_f32_256_fp.md)"}
+            "counts_source": "ncu: instructions at 512^3, flops at 256^3 scaled (profiles/plic_fit_resolve_f32.md)"}
 
 
 def plic_block(args, dev, cc):
