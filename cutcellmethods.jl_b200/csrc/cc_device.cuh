@@ -770,7 +770,8 @@ __device__ __forceinline__ Dual<T, 3> tape_eval_select(const STape<T>& t, const 
 // value the running minimum can take there (mode 2: by k, so that the smooth step returns its
 // input). Bounds are formed in Float32 whatever T is; the margin, 2^-18 of every magnitude involved
 // (`mag`: the grid's coordinates, plus the sphere's own), is at least eight times their rounding and
-// that of the coordinates and of T's evaluation. A NaN or infinite bound keeps its sphere. Writes the
+// that of the coordinates and of T's evaluation, in the range that the host checks (in_bounds_range); `lo`, `hi` and `mag`
+// are as bound_f32 gives them, and so are low and up. A NaN or infinite bound keeps its sphere. Writes the
 // kept spheres in op order, as indices (INDEX) or poff | kparam << 16, to `out` (n_ops entries) and returns their number;
 // low and up receive the smallest lower and upper bound over the spheres.
 __device__ __forceinline__ float sqrt_approx(float x) {
@@ -778,18 +779,25 @@ __device__ __forceinline__ float sqrt_approx(float x) {
   asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
+// A length as the bounds take it: Float64 ones times the tape's power of two.
+template <class T>
+__device__ __forceinline__ float bound_f32(T v, double scale) {
+  if constexpr (sizeof(T) == 8) return float(v * scale);
+  else return v;
+}
 template <class T, bool INDEX = false>
-__device__ __forceinline__ int prune_warp(const STape<T>& t, int mode, const float lo[3], const float hi[3], float mag,
-                                          unsigned* out, float& low, float& up) {
+__device__ __forceinline__ int prune_warp(const STape<T>& t, int mode, double scale, const float lo[3], const float hi[3],
+                                          float mag, unsigned* out, float& low, float& up) {
   const int lane = threadIdx.x & 31, n = t.n_ops;
   const float big = __int_as_float(0x7f800000);
   auto bounds = [&](int i, float& l, float& u) {
     T c[4];
     ldq(t.p + t.ops[i].poff, c);
-    float dmin2 = 0.0f, dmax2 = 0.0f, m = mag + fabsf(float(c[3]));
+    const float r = bound_f32(c[3], scale);
+    float dmin2 = 0.0f, dmax2 = 0.0f, m = mag + fabsf(r);
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      const float ca = float(c[a]);
+      const float ca = bound_f32(c[a], scale);
       const float below = lo[a] - ca, above = ca - hi[a];
       const float dn = fmaxf(fmaxf(below, above), 0.0f), dx = fmaxf(fabsf(below), fabsf(above));
       dmin2 += dn * dn;
@@ -797,8 +805,8 @@ __device__ __forceinline__ int prune_warp(const STape<T>& t, int mode, const flo
       m += fabsf(ca);
     }
     const float far = sqrt_approx(dmax2), margin = 0x1p-18f * (m + far);
-    l = sqrt_approx(dmin2) - float(c[3]) - margin;
-    u = far - float(c[3]) + margin;
+    l = sqrt_approx(dmin2) - r - margin;
+    u = far - r + margin;
   };
   auto warp_min = [](float v) {
 #pragma unroll
@@ -839,7 +847,7 @@ __device__ __forceinline__ int prune_warp(const STape<T>& t, int mode, const flo
       before = __shfl_up_sync(0xffffffffu, before, 1);
       before = fminf(lane == 0 ? big : before, running);
       if (i < n) {
-        const float k = float(t.p[t.ops[i].kparam]);
+        const float k = bound_f32(t.p[t.ops[i].kparam], scale);
         const float km = 0x1p-18f * (fabsf(k) + fabsf(before) + fabsf(l) + mag);
         keep = i == 0 || !(l >= before + k + km);
       }

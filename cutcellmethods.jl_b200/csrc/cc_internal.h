@@ -1,5 +1,6 @@
 // cc_internal.h -- launch interfaces between the C ABI (capi.cu) and the kernel files.
 #pragma once
+#include <cmath>
 #include <cstdint>
 #include <string>
 #include <cuda_runtime.h>
@@ -43,7 +44,23 @@ struct DevTape {
   int prunable = 0;  // 1: a union (MIN) of spheres, 2: a smooth union (SMIN) of spheres; see prune_union, prune_warp
   int select = 0;    // no smooth minimum: value and gradient are one primitive's (tape_eval_select)
   int slab = 8;      // the 3D PLIC fit's pruning slab in cell layers (prune_slab)
+  double scale = 1;  // a power of two that brings the grid's lengths near 1 (in_bounds_range)
 };
+
+// The tape as prune_warp may bound it over a grid, in every 3D pass that prunes. Its bounds are Float32 and
+// square distances, so Float64 lengths are first taken times `scale` (exact). A union of spheres stays prunable
+// while T's own squares are normal over the grid: `mag`, the size of its coordinates, within 2^-48..2^60 at
+// Float32 (below, the roots of T's squares err by up to 2^-73, near the bounds' margin of 2^-18 mag; above, squares
+// overflow) and within 2^-480..2^480 at Float64. Outside, it is evaluated whole like any other body.
+template <class T>
+DevTape in_bounds_range(DevTape tape, const DevGrid<T>& g) {
+  double mag = 0;
+  for (int a = 0; a < 3; ++a) mag += std::fabs(double(g.x0[a])) + double(g.n[a]) * double(g.d[a]);
+  const bool f64 = sizeof(T) == 8;
+  if (!(mag >= (f64 ? 0x1p-480 : 0x1p-48) && mag <= (f64 ? 0x1p480 : 0x1p60))) tape.prunable = 0;
+  else if (f64) tape.scale = std::ldexp(1.0, -std::ilogb(mag));
+  return tape;
+}
 
 // Bounds of a 3D body over all space: how fast its value can change (the Lipschitz constant), the
 // largest sum of |gradient components|, and the size of its parameters (for rounding margins).

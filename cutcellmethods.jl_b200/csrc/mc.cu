@@ -205,12 +205,12 @@ __global__ void __launch_bounds__(Tile<T>::NT, Tile<T>::MINB) mc_fill_kernel(con
         float lo[3], hi[3], mag = 0.0f, low, up;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-          lo[a] = float(node_coord(A.g.x0[a], A.g.d[a], first[a]));
-          hi[a] = float(node_coord(A.g.x0[a], A.g.d[a], last[a]));
-          mag += fabsf(float(A.g.x0[a])) + float(A.g.n[a]) * float(A.g.d[a]);
+          lo[a] = bound_f32(node_coord(A.g.x0[a], A.g.d[a], first[a]), A.tape.scale);
+          hi[a] = bound_f32(node_coord(A.g.x0[a], A.g.d[a], last[a]), A.tape.scale);
+          mag += fabsf(bound_f32(A.g.x0[a], A.tape.scale)) + float(A.g.n[a]) * bound_f32(A.g.d[a], A.tape.scale);
         }
         unsigned* list = reinterpret_cast<unsigned*>(kept + n);
-        const int m = prune_warp<T, true>(tape, A.tape.prunable, lo, hi, mag, list, low, up);
+        const int m = prune_warp<T, true>(tape, A.tape.prunable, A.tape.scale, lo, hi, mag, list, low, up);
         for (int q = tid; q < m; q += 32) {
           cc_op op = tape.ops[list[q]];
           if (q == 0) op.combine = CC_COMB_PUSH;
@@ -659,7 +659,7 @@ cudaError_t launch_mc(const DevGrid<T>& g, const DevTape& tape, const T* phi_in,
   using TL = Tile<T>;
   McArgs<T> a;
   a.g = g;
-  a.tape = tape;
+  a.tape = in_bounds_range(tape, g);
   a.phi_in = phi_in;
   a.phi_out = phi_out;
   a.cols = cols;
@@ -681,7 +681,7 @@ cudaError_t launch_mc(const DevGrid<T>& g, const DevTape& tape, const T* phi_in,
   cudaError_t e = count_zeroed ? cudaSuccess : cudaMemsetAsync(cut_count, 0, sizeof(unsigned), s);
   if (e != cudaSuccess) return e;
   const bool sample = phi_in == nullptr;
-  const bool pruned = sample && tape.prunable;
+  const bool pruned = sample && a.tape.prunable;
   int sm = smem_bytes<T>(sample ? tape.bytes_len : 0);
   if (pruned) sm += tape.n_ops * int(sizeof(cc_op) + sizeof(unsigned));
   const int cut_blocks = 148 * 16;

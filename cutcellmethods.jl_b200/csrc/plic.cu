@@ -9,6 +9,7 @@
 // whose two cells differ; in 2D a face pass computes both sides from the stored planes.
 #include <cmath>
 #include <cstdint>
+#include <limits>
 #include <type_traits>
 #include "cc_device.cuh"
 #include "cc_internal.h"
@@ -267,14 +268,14 @@ enum PlaneMode { DUAL = 0, SPHERES = 1, SMOOTH = 2, SELECT = 3 };
 template <class T>
 struct RowBox {
   float lo[3], hi[3], mag;
-  __device__ __forceinline__ RowBox(const DevGrid<T>& g, long long i0, int ni, long long j, long long k0, int nk) {
+  __device__ __forceinline__ RowBox(const DevGrid<T>& g, double scale, long long i0, int ni, long long j, long long k0, int nk) {
     const long long first[3] = {i0, j, k0}, last[3] = {i0 + ni - 1, j, k0 + nk - 1};
     mag = 0.0f;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      lo[a] = float(g.x0[a] + (T(first[a]) + T(0.5)) * g.d[a]);
-      hi[a] = float(g.x0[a] + (T(last[a]) + T(0.5)) * g.d[a]);
-      mag += fabsf(float(g.x0[a])) + float(g.n[a]) * float(g.d[a]);
+      lo[a] = bound_f32(g.x0[a] + (T(first[a]) + T(0.5)) * g.d[a], scale);
+      hi[a] = bound_f32(g.x0[a] + (T(last[a]) + T(0.5)) * g.d[a], scale);
+      mag += fabsf(bound_f32(g.x0[a], scale)) + float(g.n[a]) * bound_f32(g.d[a], scale);
     }
   }
 };
@@ -470,9 +471,9 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : (MODE == SPHERES || M
   unsigned* list = reinterpret_cast<unsigned*>(smem + ((tape.bytes_len + 15) / 16) * 16) + w * tape.n_ops;
   int m = 0;
   if constexpr (MODE == SPHERES || MODE == SMOOTH) {
-    const RowBox<T> box(g, i0, ni, j, k0, nk);
+    const RowBox<T> box(g, tape.scale, i0, ni, j, k0, nk);
     float low, up;
-    m = prune_warp<T>(t, MODE, box.lo, box.hi, box.mag, list, low, up);
+    m = prune_warp<T>(t, MODE, tape.scale, box.lo, box.hi, box.mag, list, low, up);
   }
   const bool in = lane < ni;
   const T x = centroid_coord(g.x0[0], g.d[0], i0 + lane), y = centroid_coord(g.x0[1], g.d[1], j);
@@ -791,16 +792,17 @@ __global__ void __launch_bounds__(NT) calc_volume_z_kernel(const DevGrid<T> g, c
       }
       if constexpr (MODE == SPHERES) {
         float least = __int_as_float(0x7f800000);
-        bool nan = false;
+        bool known = true;
+        const float b[3] = {bound_f32(x[0], tape.scale), bound_f32(x[1], tape.scale), bound_f32(x[2], tape.scale)};
         for (int i = lane % share; i < t.n_ops; i += share) {
           T c[4];
           ldq(t.p + t.ops[i].poff, c);
-          const float d0 = float(x[0]) - float(c[0]), d1 = float(x[1]) - float(c[1]), d2 = float(x[2]) - float(c[2]);
-          const float u = sqrt_approx(d0 * d0 + d1 * d1 + d2 * d2) - float(c[3]);
-          nan = nan || !(u == u);
+          const float d0 = b[0] - bound_f32(c[0], tape.scale), d1 = b[1] - bound_f32(c[1], tape.scale), d2 = b[2] - bound_f32(c[2], tape.scale);
+          const float u = sqrt_approx(d0 * d0 + d1 * d1 + d2 * d2) - bound_f32(c[3], tape.scale);
+          known = known && u - u == 0.0f;
           least = fminf(least, u);
         }
-        v = nan ? qnan<T>() : T(least);
+        v = known ? T(least) : qnan<T>();  // times the scale, as `beyond` is
       } else {
         v = tape_eval<T, 3, T>(t, x);
       }
@@ -812,8 +814,9 @@ __global__ void __launch_bounds__(NT) calc_volume_z_kernel(const DevGrid<T> g, c
       }
     }
     if (any && lane % share == 0) {
-      if (v < -beyond) whole += ext[0] * ext[1] * ext[2];
-      open = !(v > beyond) && !(v < -beyond);
+      const bool inside = v < -beyond && v - v == T(0);  // an infinite value says nothing of the box: it overflowed
+      if (inside) whole += ext[0] * ext[1] * ext[2];
+      open = !inside && !(v > beyond && v - v == T(0));
     }
     for (unsigned left = __ballot_sync(0xffffffffu, open); left; left &= left - 1) {
       const int src = __ffs(left) - 1;
@@ -829,11 +832,11 @@ __global__ void __launch_bounds__(NT) calc_volume_z_kernel(const DevGrid<T> g, c
         float lo[3], hi[3], mag = 0.0f, low, up;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-          lo[a] = float(g.x0[a] + (T(c0[a]) + T(0.5)) * g.d[a]);
-          hi[a] = float(g.x0[a] + (T(c0[a] + ce[a] - 1) + T(0.5)) * g.d[a]);
-          mag += fabsf(float(g.x0[a])) + float(g.n[a]) * float(g.d[a]);
+          lo[a] = bound_f32(g.x0[a] + (T(c0[a]) + T(0.5)) * g.d[a], tape.scale);
+          hi[a] = bound_f32(g.x0[a] + (T(c0[a] + ce[a] - 1) + T(0.5)) * g.d[a], tape.scale);
+          mag += fabsf(bound_f32(g.x0[a], tape.scale)) + float(g.n[a]) * bound_f32(g.d[a], tape.scale);
         }
-        m = prune_warp<T>(t, MODE, lo, hi, mag, list, low, up);
+        m = prune_warp<T>(t, MODE, tape.scale, lo, hi, mag, list, low, up);
       }
       // cells near enough to need their plane are listed, then taken on full warps
       const bool in = lane % VX < ce[0] && lane / VX < ce[1];
@@ -1054,9 +1057,10 @@ cudaError_t launch_fit_z(const DevGrid<T>& g, const DevTape& tape, const Cols& c
 }  // namespace
 
 template <class T, int D>
-cudaError_t launch_plic(const DevGrid<T>& g, const DevTape& tape, const Cols& cols, T* normals, T* intercepts,
+cudaError_t launch_plic(const DevGrid<T>& g, const DevTape& body, const Cols& cols, T* normals, T* intercepts,
                         uint8_t* valid, int8_t* sides, cudaStream_t s, bool mixed) {
   const long long total = g.n[0] * g.n[1] * (D == 3 ? g.n[2] : 1);
+  const DevTape tape = D == 3 ? in_bounds_range(body, g) : body;
   if constexpr (D == 3) {
     if (!sides) return cudaErrorInvalidValue;
     const bool mx = mixed && sizeof(T) == 4;
@@ -1098,10 +1102,14 @@ cudaError_t launch_volume_z(const DevGrid<T>& g, const DevTape& tape, const Tape
   const double h = double(g.d[0]);
   double mag = tb.mag;
   for (int a = 0; a < 3; ++a) mag += std::fabs(double(g.x0[a])) + double(g.n[a]) * double(g.d[a]);
-  const double thr = 0.5 * tb.grad1 * h * 1.001;
+  double thr = 0.5 * tb.grad1 * h * 1.001;
   const double half = 0.5 * h * std::sqrt(double(VX * VX + VY * VY + VZ * VZ));
   const double margin = (sizeof(T) == 4 || MODE == SPHERES ? 0x1p-16 : 0x1p-40) * (1.0 + tb.lipschitz) * mag;
-  const double beyond = (thr + tb.lipschitz * half) * 1.001 + margin;
+  double beyond = (thr + tb.lipschitz * half) * 1.001 + margin;
+  // where T's squares are not normal (as in in_bounds_range) values err by more than the margin: nothing is settled
+  const double inf = std::numeric_limits<double>::infinity();
+  if (!(mag >= (sizeof(T) == 8 ? 0x1p-480 : 0x1p-48) && mag <= (sizeof(T) == 8 ? 0x1p480 : 0x1p60))) thr = beyond = inf;
+  if (MODE == SPHERES) beyond *= tape.scale;
   const long long boxes = ((g.n[0] + VX - 1) / VX) * ((g.n[1] + VY - 1) / VY) * ((g.n[2] + VZ - 1) / VZ);
   // boxes per warp at a time: few enough that every resident warp has some
   int group = 32;
@@ -1127,9 +1135,10 @@ cudaError_t launch_volume_z(const DevGrid<T>& g, const DevTape& tape, const Tape
 }  // namespace
 
 template <class T, int D>
-cudaError_t launch_calc_volume(const DevGrid<T>& g, const DevTape& tape, const TapeBounds& tb, double* partial,
+cudaError_t launch_calc_volume(const DevGrid<T>& g, const DevTape& body, const TapeBounds& tb, double* partial,
                                double* out, cudaStream_t s, bool mixed) {
   int nb = VOL_BLOCKS;
+  const DevTape tape = D == 3 ? in_bounds_range(body, g) : body;
   cudaError_t e;
   if constexpr (D == 3) {
     const bool mx = mixed && sizeof(T) == 4;
