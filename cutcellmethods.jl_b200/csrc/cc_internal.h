@@ -74,6 +74,14 @@ TapeBounds tape_bounds(const cc_optape* t);
 // spheres of cell size h: about 0.6 of the median radius, rounded to 4, 8, 16 or 32 layers.
 int prune_slab(const cc_optape* t, double h);
 
+// Dynamic shared memory of a launch. A kernel may take 48 KB in all, its static arrays (at most 27 KB: the 3D
+// PLIC fit at Float64) among them, without asking for more; above 20 KB of its own a launch asks.
+template <class K>
+cudaError_t allow_dynamic_smem(K* kernel, int bytes) {
+  if (bytes <= 20 * 1024) return cudaSuccess;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+
 struct Cols {
   int8_t* kind;
   uint8_t* amb;

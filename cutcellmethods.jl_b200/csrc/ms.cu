@@ -85,10 +85,8 @@ cudaError_t launch_ms(const DevGrid<T>& g, const DevTape& tape, const T* phi_in,
   T* phi = phi_in ? const_cast<T*>(phi_in) : phi_out;  // read only without SAMPLE
   const bool wide = g.n[0] >= 0x7fffff00LL || g.n[1] >= 0x7fffff00LL;
   auto run = [&](auto kernel) {
-    if (sm > 40 * 1024) {
-      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-      if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_dynamic_smem(kernel, sm);
+    if (e != cudaSuccess) return e;
     kernel<<<blocks, GRID_NT, sm, s>>>(g, tape, phi, cols, ty);
     return cudaGetLastError();
   };

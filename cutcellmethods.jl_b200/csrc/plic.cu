@@ -457,6 +457,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : (MODE == SPHERES || M
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ T s_nrm[NT / 32][3 * FZ_X];
   __shared__ CrossedCell<T> s_crossed[NT / 32][CROSSED_MAX];
+  static_assert(sizeof(s_nrm) + sizeof(s_crossed) <= 27 * 1024, "see allow_dynamic_smem");
   const STape<T> t = load_tape<T>(tape.bytes, tape.n_ops, tape.n_params, smem);
   __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1041,12 +1042,10 @@ cudaError_t launch_fit_z(const DevGrid<T>& g, const DevTape& tape, const Cols& c
   const int lists = MODE == SPHERES || MODE == SMOOTH ? (NT / 32) * tape.n_ops * int(sizeof(unsigned)) : 0;
   const int sm = ((tape.bytes_len + 15) / 16) * 16 + lists;
   auto run = [&](auto kernel) {
-    if (sm > 40 * 1024) {
-      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-      if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_dynamic_smem(kernel, sm);
+    if (e != cudaSuccess) return e;
     kernel<<<unsigned(blocks), NT, sm, s>>>(g, tape, cols, normals, intercepts, valid, sides, depth);
-    return cudaSuccess;
+    return cudaGetLastError();  // the resolve pass must not follow a fit that did not run
   };
   if constexpr (sizeof(T) == 4) {
     if (mx) return run(plic_fit_z_kernel<T, true, MODE>);
@@ -1075,12 +1074,9 @@ cudaError_t launch_plic(const DevGrid<T>& g, const DevTape& body, const Cols& co
     plic_resolve_kernel<T><<<rb, NT, 0, s>>>(g, static_cast<T*>(cols.ff), sides, total);
   } else {  // 2D works in tiles
     const int sm = CentroidSmem::of(tape).bytes;
-    if (sm > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(plic_fit_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-      if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(plic_fit_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-      if (e != cudaSuccess) return e;
-    }
+    cudaError_t e = allow_dynamic_smem(plic_fit_kernel<T, true>, sm);
+    if (e == cudaSuccess) e = allow_dynamic_smem(plic_fit_kernel<T, false>, sm);
+    if (e != cudaSuccess) return e;
     if (mixed && sizeof(T) == 4) {
       plic_fit_kernel<T, true><<<blocks_for(total, 16), NT, sm, s>>>(g, tape, cols, normals, intercepts, valid);
       plic_face_kernel<T, true><<<blocks_for(total, 16), NT, 0, s>>>(g, cols, normals, intercepts, valid);
@@ -1119,12 +1115,10 @@ cudaError_t launch_volume_z(const DevGrid<T>& g, const DevTape& tape, const Tape
   const int lists = MODE == SPHERES || MODE == SMOOTH ? (NT / 32) * tape.n_ops * int(sizeof(unsigned)) : 0;
   const int sm = ((tape.bytes_len + 15) / 16) * 16 + lists;
   auto run = [&](auto kernel) {
-    if (sm > 40 * 1024) {
-      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-      if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_dynamic_smem(kernel, sm);
+    if (e != cudaSuccess) return e;
     kernel<<<*nb, NT, sm, s>>>(g, tape, partial, T(thr), T(beyond), group);
-    return cudaSuccess;
+    return cudaGetLastError();
   };
   if constexpr (sizeof(T) == 4) {
     if (mx) return run(calc_volume_z_kernel<T, true, MODE>);
@@ -1149,12 +1143,9 @@ cudaError_t launch_calc_volume(const DevGrid<T>& g, const DevTape& body, const T
     if (e != cudaSuccess) return e;
   } else {
     const int sm = CentroidSmem::of(tape).bytes;
-    if (sm > 48 * 1024) {
-      e = cudaFuncSetAttribute(calc_volume_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-      if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(calc_volume_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-      if (e != cudaSuccess) return e;
-    }
+    e = allow_dynamic_smem(calc_volume_kernel<T, true>, sm);
+    if (e == cudaSuccess) e = allow_dynamic_smem(calc_volume_kernel<T, false>, sm);
+    if (e != cudaSuccess) return e;
     if (mixed && sizeof(T) == 4) calc_volume_kernel<T, true><<<nb, NT, sm, s>>>(g, tape, partial);
     else calc_volume_kernel<T, false><<<nb, NT, sm, s>>>(g, tape, partial);
   }
