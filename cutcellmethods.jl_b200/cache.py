@@ -18,6 +18,7 @@ src/marching_cubes/cache.jl, src/plic/cache.jl):
 from __future__ import annotations
 
 import ctypes as C
+import threading
 
 import numpy as np
 import torch
@@ -333,7 +334,17 @@ def kinds(cache):
     return cache.cells.kind
 
 
+# calc_volume's and monte_carlo_volume's hidden handles, one per device and precision, each with the lock that
+# lets one call at a time use its tape staging, its scratch and its result (a ctypes call releases the GIL)
 _vol_handles = {}
+_vol_handles_lock = threading.Lock()
+
+
+def _vol_handle(dev, prec):
+    with _vol_handles_lock:
+        if (dev, prec) not in _vol_handles:
+            _vol_handles[(dev, prec)] = (_Handle(dev, _lib.CC_PLIC, 3, prec, (1, 1, 1)), threading.Lock())
+        return _vol_handles[(dev, prec)]
 
 
 def calc_volume(geo, grid: CartesianGrid, dtype=torch.float64, device=None, precision: str = "plain"):
@@ -344,14 +355,12 @@ def calc_volume(geo, grid: CartesianGrid, dtype=torch.float64, device=None, prec
     device = torch.device(device)
     dev = device.index if device.index is not None else torch.cuda.current_device()
     prec = _prec(dtype, precision)
-    key = (dev, prec)
-    if key not in _vol_handles:
-        _vol_handles[key] = _Handle(dev, _lib.CC_PLIC, 3, prec, (1, 1, 1))
-    h = _vol_handles[key]
+    h, lock = _vol_handle(dev, prec)
     tp = _TapeRef(as_tape(geo, grid.dim))
     out = C.c_double(0.0)
     gs = grid_struct(grid)
-    _check(h.lib.cc_calc_volume(h.h, C.byref(gs), C.byref(tp.s), C.byref(out), _stream(device)))
+    with lock:
+        _check(h.lib.cc_calc_volume(h.h, C.byref(gs), C.byref(tp.s), C.byref(out), _stream(device)))
     return out.value
 
 
@@ -362,16 +371,14 @@ def monte_carlo_volume(geo, lo, hi, n_points: int, seed: int = 0, device=None):
         device = torch.device("cuda", torch.cuda.current_device())
     device = torch.device(device)
     dev = device.index if device.index is not None else torch.cuda.current_device()
-    key = (dev, _lib.CC_F64)
-    if key not in _vol_handles:
-        _vol_handles[key] = _Handle(dev, _lib.CC_PLIC, 3, _lib.CC_F64, (1, 1, 1))
-    h = _vol_handles[key]
+    h, lock = _vol_handle(dev, _lib.CC_F64)
     tp = _TapeRef(as_tape(geo, 3))
     l = (C.c_double * 3)(*lo)
     u = (C.c_double * 3)(*hi)
     inside, vol = C.c_int64(0), C.c_double(0.0)
-    _check(h.lib.cc_monte_carlo_volume(h.h, C.byref(tp.s), l, u, n_points, seed, C.byref(inside), C.byref(vol),
-                                       _stream(device)))
+    with lock:
+        _check(h.lib.cc_monte_carlo_volume(h.h, C.byref(tp.s), l, u, n_points, seed, C.byref(inside), C.byref(vol),
+                                           _stream(device)))
     return vol.value, inside.value
 
 

@@ -208,7 +208,7 @@ struct cc_handle {
   double* vol_scratch = nullptr;  // calc_volume partials + result
   unsigned long long* rep_scratch = nullptr;  // report counters + the complement of the min's bits
   // pinned, for results read back: the report's, then calc_volume's and generate_mesh's own words (threads may
-  // be in different ones of them at once)
+  // be in different ones of them at once; two calls of one of them on one handle are the caller's to keep apart)
   unsigned long long* rep_host = nullptr;
   unsigned long long* vol_host() const { return rep_host + 8; }
   unsigned long long* mesh_host() const { return rep_host + 16; }
