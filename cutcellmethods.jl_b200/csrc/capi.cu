@@ -156,10 +156,6 @@ DevTable TableLayout::at(const unsigned char* dev) const {
 }  // namespace cci
 
 
-namespace {
-
-}  // namespace
-
 namespace cci {
 
 // Pack a validated tape for the device into `out` (capacity tape_pack_capacity()): the ops,
@@ -486,11 +482,11 @@ static cc_status mc_common(cc_handle* h, const cc_grid* g, const cc_optape* body
     if (body && (st = upload_tape<double>(h, body, 3, s, &tape, true)) != CC_OK) return st;
     e = cci::launch_mc<double>(dev_grid<double>(g), tape, static_cast<const double*>(phi_in),
                                static_cast<double*>(phi_out), cols_of(cells), h->tb, h->cut_list, h->cut_count, s,
-                               true, false, body != nullptr);
+                               false, body != nullptr);
   } else {
     if (body && (st = upload_tape<float>(h, body, 3, s, &tape, true)) != CC_OK) return st;
     e = cci::launch_mc<float>(dev_grid<float>(g), tape, static_cast<const float*>(phi_in),
-                              static_cast<float*>(phi_out), cols_of(cells), h->tb, h->cut_list, h->cut_count, s, true,
+                              static_cast<float*>(phi_out), cols_of(cells), h->tb, h->cut_list, h->cut_count, s,
                               h->prec == CC_MIXED, body != nullptr);
   }
   if (e != cudaSuccess) return cuda_fail(e, "marching cubes launch");

@@ -485,11 +485,13 @@ __device__ __forceinline__ STape<T> load_tape(const unsigned char* __restrict__ 
 //    the largest value over the box of every earlier sphere's minimum -- then the smooth-min step
 //    sees |top - v| >= k, h = 0, and returns the running value unchanged, bit for bit.
 // The bounds carry a margin of 16 eps(T) times the magnitudes involved, so T's rounding of the
-// evaluation can not cross them. All threads call this; it returns the kept op count and writes
-// the kept ops (the first one's combine made PUSH) to `out`. `ls`, `us`: n_ops doubles each.
-template <class T, int D>
-__device__ int prune_union(const STape<T>& t, int mode, const double lo[D], const double hi[D], double* ls, double* us,
+// evaluation can not cross them. This is the 2D passes' form, by a CTA of at least n_ops threads (prune_warp
+// is the 3D passes'). All threads call it; it returns the kept op count and writes the kept ops (the
+// first one's combine made PUSH) to `out`. `ls`, `us`: n_ops doubles each.
+template <class T>
+__device__ int prune_union(const STape<T>& t, int mode, const double lo[2], const double hi[2], double* ls, double* us,
                            cc_op* out, int* count) {
+  constexpr int D = 2;
   const int n = t.n_ops;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const T* p = t.p + t.ops[i].poff;
@@ -510,110 +512,81 @@ __device__ int prune_union(const STape<T>& t, int mode, const double lo[D], cons
     us[i] = sqrt(dmax2) - r + margin;
   }
   __syncthreads();
-  if (n <= int(blockDim.x) && blockDim.x <= 1024) {
-    // one op per thread: block reductions and scans, then an order-preserving compaction
-    __shared__ double s_val[32];
-    __shared__ int s_idx[32];
-    __shared__ int s_cnt[32];
-    const int i = threadIdx.x, lane = i & 31, w = i >> 5, nw = (blockDim.x + 31) >> 5;
-    const double u = i < n ? us[i] : 1.0e300;
-    bool keep = false;
-    if (mode == 1) {
-      // the smallest upper bound, its op, and the smallest of the others
-      double v = u;
-      int vi = i;
+  // one op per thread: block reductions and scans, then an order-preserving compaction
+  __shared__ double s_val[32];
+  __shared__ int s_idx[32];
+  __shared__ int s_cnt[32];
+  const int i = threadIdx.x, lane = i & 31, w = i >> 5, nw = (blockDim.x + 31) >> 5;
+  const double u = i < n ? us[i] : 1.0e300;
+  bool keep = false;
+  if (mode == 1) {
+    // the smallest upper bound, its op, and the smallest of the others
+    double v = u;
+    int vi = i;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ov = __shfl_xor_sync(0xffffffffu, v, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, vi, o);
-        if (ov < v || (ov == v && oi < vi)) { v = ov; vi = oi; }
-      }
-      if (lane == 0) { s_val[w] = v; s_idx[w] = vi; }
-      __syncthreads();
-      double mn = s_val[0];
-      int jm = s_idx[0];
-      for (int q = 1; q < nw; ++q)
-        if (s_val[q] < mn || (s_val[q] == mn && s_idx[q] < jm)) { mn = s_val[q]; jm = s_idx[q]; }
-      __syncthreads();
-      double v2 = i == jm ? 1.0e300 : u;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ov = __shfl_xor_sync(0xffffffffu, v2, o);
-        v2 = ov < v2 ? ov : v2;
-      }
-      if (lane == 0) s_val[w] = v2;
-      __syncthreads();
-      double mn2 = s_val[0];
-      for (int q = 1; q < nw; ++q) mn2 = s_val[q] < mn2 ? s_val[q] : mn2;
-      keep = i < n && !(ls[i] > (i == jm ? mn2 : mn));
-    } else {
-      // the exclusive prefix minimum of the upper bounds
-      double v = u;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const double ov = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v = ov < v ? ov : v;
-      }
-      if (lane == 31) s_val[w] = v;
-      __syncthreads();
-      double before = 1.0e300;  // the minimum over the earlier warps
-      for (int q = 0; q < w; ++q) before = s_val[q] < before ? s_val[q] : before;
-      double up = __shfl_up_sync(0xffffffffu, v, 1);
-      if (lane == 0) up = 1.0e300;
-      const double prefix = up < before ? up : before;  // min over ops 0..i-1
-      if (i < n) {
-        if (i == 0) keep = true;
-        else {
-          const double k = t.p[t.ops[i].kparam];
-          const double kmargin = 16.0 * double(Eps<T>::v()) * (fabs(k) + fabs(prefix) + fabs(ls[i]) + 1.0);
-          keep = !(ls[i] >= prefix + k + kmargin);
-        }
-      }
-      __syncthreads();
+    for (int o = 16; o > 0; o >>= 1) {
+      const double ov = __shfl_xor_sync(0xffffffffu, v, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, vi, o);
+      if (ov < v || (ov == v && oi < vi)) { v = ov; vi = oi; }
     }
-    const unsigned b = __ballot_sync(0xffffffffu, keep);
-    if (lane == 0) s_cnt[w] = __popc(b);
+    if (lane == 0) { s_val[w] = v; s_idx[w] = vi; }
     __syncthreads();
-    int pos = __popc(b & ((1u << lane) - 1u));
-    int total = 0;
-    for (int q = 0; q < nw; ++q) {
-      if (q < w) pos += s_cnt[q];
-      total += s_cnt[q];
-    }
-    if (keep) {
-      cc_op op = t.ops[i];
-      if (pos == 0) op.combine = CC_COMB_PUSH;
-      out[pos] = op;
-    }
-    if (i == 0) *count = total;
+    double mn = s_val[0];
+    int jm = s_idx[0];
+    for (int q = 1; q < nw; ++q)
+      if (s_val[q] < mn || (s_val[q] == mn && s_idx[q] < jm)) { mn = s_val[q]; jm = s_idx[q]; }
     __syncthreads();
-    return *count;
-  }
-  if (threadIdx.x == 0) {
-    int m = 0;
-    if (mode == 1) {
-      int jm = 0;
-      for (int j = 1; j < n; ++j) if (us[j] < us[jm]) jm = j;
-      double u2 = 1.0e300;
-      for (int j = 0; j < n; ++j) if (j != jm && us[j] < u2) u2 = us[j];
-      for (int i = 0; i < n; ++i) {
-        if (ls[i] > (i == jm ? u2 : us[jm])) continue;
-        cc_op op = t.ops[i];
-        if (m == 0) op.combine = CC_COMB_PUSH;
-        out[m++] = op;
-      }
-    } else {
-      double prefix = us[0];
-      out[m++] = t.ops[0];
-      for (int i = 1; i < n; ++i) {
+    double v2 = i == jm ? 1.0e300 : u;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double ov = __shfl_xor_sync(0xffffffffu, v2, o);
+      v2 = ov < v2 ? ov : v2;
+    }
+    if (lane == 0) s_val[w] = v2;
+    __syncthreads();
+    double mn2 = s_val[0];
+    for (int q = 1; q < nw; ++q) mn2 = s_val[q] < mn2 ? s_val[q] : mn2;
+    keep = i < n && !(ls[i] > (i == jm ? mn2 : mn));
+  } else {
+    // the exclusive prefix minimum of the upper bounds
+    double v = u;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double ov = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v = ov < v ? ov : v;
+    }
+    if (lane == 31) s_val[w] = v;
+    __syncthreads();
+    double before = 1.0e300;  // the minimum over the earlier warps
+    for (int q = 0; q < w; ++q) before = s_val[q] < before ? s_val[q] : before;
+    double up = __shfl_up_sync(0xffffffffu, v, 1);
+    if (lane == 0) up = 1.0e300;
+    const double prefix = up < before ? up : before;  // min over ops 0..i-1
+    if (i < n) {
+      if (i == 0) keep = true;
+      else {
         const double k = t.p[t.ops[i].kparam];
         const double kmargin = 16.0 * double(Eps<T>::v()) * (fabs(k) + fabs(prefix) + fabs(ls[i]) + 1.0);
-        if (!(ls[i] >= prefix + k + kmargin)) out[m++] = t.ops[i];
-        if (us[i] < prefix) prefix = us[i];
+        keep = !(ls[i] >= prefix + k + kmargin);
       }
     }
-    *count = m;
+    __syncthreads();
   }
+  const unsigned b = __ballot_sync(0xffffffffu, keep);
+  if (lane == 0) s_cnt[w] = __popc(b);
+  __syncthreads();
+  int pos = __popc(b & ((1u << lane) - 1u));
+  int total = 0;
+  for (int q = 0; q < nw; ++q) {
+    if (q < w) pos += s_cnt[q];
+    total += s_cnt[q];
+  }
+  if (keep) {
+    cc_op op = t.ops[i];
+    if (pos == 0) op.combine = CC_COMB_PUSH;
+    out[pos] = op;
+  }
+  if (i == 0) *count = total;
   __syncthreads();
   return *count;
 }
@@ -771,9 +744,8 @@ __device__ __forceinline__ Dual<T, 3> tape_eval_select(const STape<T>& t, const 
 // input). Bounds are formed in Float32 whatever T is; the margin, 2^-18 of every magnitude involved
 // (`mag`: the grid's coordinates, plus the sphere's own), is at least eight times their rounding and
 // that of the coordinates and of T's evaluation, in the range that the host checks (in_bounds_range); `lo`, `hi` and `mag`
-// are as bound_f32 gives them, and so are low and up. A NaN or infinite bound keeps its sphere. Writes the
-// kept spheres in op order, as indices (INDEX) or poff | kparam << 16, to `out` (n_ops entries) and returns their number;
-// low and up receive the smallest lower and upper bound over the spheres.
+// are as bound_f32 gives them. A NaN or infinite bound keeps its sphere. Writes the kept spheres in op order, as
+// indices (INDEX) or poff | kparam << 16, to `out` (n_ops entries) and returns their number.
 __device__ __forceinline__ float sqrt_approx(float x) {
   float r;
   asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -787,7 +759,7 @@ __device__ __forceinline__ float bound_f32(T v, double scale) {
 }
 template <class T, bool INDEX = false>
 __device__ __forceinline__ int prune_warp(const STape<T>& t, int mode, double scale, const float lo[3], const float hi[3],
-                                          float mag, unsigned* out, float& low, float& up) {
+                                          float mag, unsigned* out) {
   const int lane = threadIdx.x & 31, n = t.n_ops;
   const float big = __int_as_float(0x7f800000);
   auto bounds = [&](int i, float& l, float& u) {
@@ -815,7 +787,6 @@ __device__ __forceinline__ int prune_warp(const STape<T>& t, int mode, double sc
   };
   int kept = 0;
   float running = big;  // mode 1: the least upper bound of all; mode 2: of the spheres so far
-  low = big;
   float l0 = big, u0 = big;
   if (mode == 1) {
     for (int i = lane; i < n; i += 32) {
@@ -823,7 +794,6 @@ __device__ __forceinline__ int prune_warp(const STape<T>& t, int mode, double sc
       bounds(i, l, u);
       if (i < 32) { l0 = l; u0 = u; }
       running = fminf(running, u);
-      low = fminf(low, l);
     }
     running = warp_min(running);
   }
@@ -836,7 +806,6 @@ __device__ __forceinline__ int prune_warp(const STape<T>& t, int mode, double sc
       keep = i < n && !(l > running);
     } else {
       if (i >= n) { l = big; u = big; }
-      low = fminf(low, l);
       float before = u;  // inclusive prefix minimum over the lanes, then made exclusive
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -861,8 +830,6 @@ __device__ __forceinline__ int prune_warp(const STape<T>& t, int mode, double sc
     kept += __popc(b);
   }
   __syncwarp();
-  low = warp_min(low);
-  up = running;
   return kept;
 }
 

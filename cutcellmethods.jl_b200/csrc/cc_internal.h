@@ -96,11 +96,11 @@ struct Cols {
 // every cell. Returns the CUDA launch status.
 // `cut_list` (one slot per cell) and `cut_count` are scratch: the fill pass lists the cut band
 // there and the cut pass reads it back.
-// With count_zeroed, *cut_count is 0 already in stream order. With with_cut false only the fill pass runs (the cut band is listed, not built).
+// With count_zeroed, *cut_count is 0 already in stream order.
 template <class T>
 cudaError_t launch_mc(const DevGrid<T>& g, const DevTape& tape, const T* phi_in, T* phi_out,
                       const Cols& cols, const DevTable& tb, unsigned* cut_list, unsigned* cut_count,
-                      cudaStream_t s, bool with_cut = true, bool mixed = false, bool count_zeroed = false);
+                      cudaStream_t s, bool mixed = false, bool count_zeroed = false);
 // The mbarrier poll limit of the learned kernels (cc_set_wait_limit): set returns the old value; a
 // negative argument restores the default.
 long long set_wait_limit(long long polls);

@@ -300,7 +300,7 @@ cc_status cc_mc_update_learned(cc_handle* h, const cc_grid* g, const cc_optape* 
     if ((st = cci::upload_body_f64(h, body, 3, s, &tape)) != CC_OK) return st;
     const cci::DevGrid<double> dg2 = grid_of<double>(g);
     e = cci::launch_mc<double>(dg2, tape, nullptr, static_cast<double*>(phi), cols_of(cells), h->tb, h->cut_list,
-                               h->cut_count, s, true, false);
+                               h->cut_count, s);
     if (e == cudaSuccess)
       e = cci::launch_mc_correct<double>(dg2, static_cast<const double*>(phi), cols_of(cells), h->cut_list, h->cut_count,
                                          m->P, bound, m->fallback, m->err, s);
@@ -309,7 +309,7 @@ cc_status cc_mc_update_learned(cc_handle* h, const cc_grid* g, const cc_optape* 
     if ((st = cci::upload_body_f32(h, body, 3, s, &tape)) != CC_OK) return st;
     const cci::DevGrid<float> dg2 = grid_of<float>(g);
     e = cci::launch_mc<float>(dg2, tape, nullptr, static_cast<float*>(phi), cols_of(cells), h->tb, h->cut_list,
-                              h->cut_count, s, true, false);
+                              h->cut_count, s);
     if (e == cudaSuccess)
       e = cci::launch_mc_correct<float>(dg2, static_cast<const float*>(phi), cols_of(cells), h->cut_list, h->cut_count,
                                         m->P, bound, m->fallback, m->err, s);

@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(Tile<T>::NT, Tile<T>::MINB) mc_fill_kernel(con
       __syncthreads();
       if (tid < 32) {
         const long long first[3] = {i0, j0, k0}, last[3] = {i0 + TX < n0 ? i0 + TX : n0, j0 + TY < n1 ? j0 + TY : n1, k1};
-        float lo[3], hi[3], mag = 0.0f, low, up;
+        float lo[3], hi[3], mag = 0.0f;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
           lo[a] = bound_f32(node_coord(A.g.x0[a], A.g.d[a], first[a]), A.tape.scale);
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(Tile<T>::NT, Tile<T>::MINB) mc_fill_kernel(con
           mag += fabsf(bound_f32(A.g.x0[a], A.tape.scale)) + float(A.g.n[a]) * bound_f32(A.g.d[a], A.tape.scale);
         }
         unsigned* list = reinterpret_cast<unsigned*>(kept + n);
-        const int m = prune_warp<T, true>(tape, A.tape.prunable, A.tape.scale, lo, hi, mag, list, low, up);
+        const int m = prune_warp<T, true>(tape, A.tape.prunable, A.tape.scale, lo, hi, mag, list);
         for (int q = tid; q < m; q += 32) {
           cc_op op = tape.ops[list[q]];
           if (q == 0) op.combine = CC_COMB_PUSH;
@@ -408,10 +408,10 @@ __global__ void __launch_bounds__(Tile<T>::NT, Tile<T>::MINB) mc_fill_kernel(con
               reinterpret_cast<const uint32_t*>(sbase + col_offset<T>(col) + r * col_bytes<T>(col))[w];
         }
       }
-      // the rest row by row, a warp taking the rows it staged itself: a column's part of a row is
-      // contiguous, so lane-strided elements are full-width stores whatever the row's alignment. (A CTA
-      // stepping through every row and column with all its threads ran mostly idle: 301 x 187 x 130
-      // mixed: fill 581 -> 226 us; 203^3 Float64: 1126 -> 434 us.) Most grids have none.
+      // the rest row by row, a warp per row (at Float64 other warps staged it: the barrier above stands
+      // between). A column's part of a row is contiguous, so lane-strided elements are full-width stores
+      // whatever the row's alignment. (All threads stepping through every row and column were mostly idle:
+      // 301 x 187 x 130 mixed: fill 581 -> 226 us; 203^3 Float64: 1126 -> 434 us.) Most grids have none.
       if (A.thread_cols) {
         const int lane = tid & 31;
         for (int r = tid >> 5; r < rows; r += NT / 32) {
@@ -655,7 +655,7 @@ cudaError_t launch_fill(const McArgs<T>& a, const ColumnMaps& maps, unsigned blo
 template <class T>
 cudaError_t launch_mc(const DevGrid<T>& g, const DevTape& tape, const T* phi_in, T* phi_out,
                       const Cols& cols, const DevTable& tb, unsigned* cut_list, unsigned* cut_count,
-                      cudaStream_t s, bool with_cut, bool mixed, bool count_zeroed) {
+                      cudaStream_t s, bool mixed, bool count_zeroed) {
   using TL = Tile<T>;
   McArgs<T> a;
   a.g = g;
@@ -690,27 +690,25 @@ cudaError_t launch_mc(const DevGrid<T>& g, const DevTape& tape, const T* phi_in,
   if (pruned) {
     e = launch_fill<T, true, true>(a, maps, unsigned(blocks), sm, s);
     if (e != cudaSuccess) return e;
-    if (with_cut && mx) mc_cut_kernel<T, true, true><<<cut_blocks, CUT_NT, 0, s>>>(a);
-    else if (with_cut) mc_cut_kernel<T, true, false><<<cut_blocks, CUT_NT, 0, s>>>(a);
+    if (mx) mc_cut_kernel<T, true, true><<<cut_blocks, CUT_NT, 0, s>>>(a);
+    else mc_cut_kernel<T, true, false><<<cut_blocks, CUT_NT, 0, s>>>(a);
   } else if (sample) {
     e = launch_fill<T, true, false>(a, maps, unsigned(blocks), sm, s);
     if (e != cudaSuccess) return e;
-    if (with_cut && mx) mc_cut_kernel<T, true, true><<<cut_blocks, CUT_NT, 0, s>>>(a);
-    else if (with_cut) mc_cut_kernel<T, true, false><<<cut_blocks, CUT_NT, 0, s>>>(a);
+    if (mx) mc_cut_kernel<T, true, true><<<cut_blocks, CUT_NT, 0, s>>>(a);
+    else mc_cut_kernel<T, true, false><<<cut_blocks, CUT_NT, 0, s>>>(a);
   } else {
     e = launch_fill<T, false, false>(a, maps, unsigned(blocks), sm, s);
     if (e != cudaSuccess) return e;
-    if (with_cut && mx) mc_cut_kernel<T, false, true><<<cut_blocks, CUT_NT, 0, s>>>(a);
-    else if (with_cut) mc_cut_kernel<T, false, false><<<cut_blocks, CUT_NT, 0, s>>>(a);
+    if (mx) mc_cut_kernel<T, false, true><<<cut_blocks, CUT_NT, 0, s>>>(a);
+    else mc_cut_kernel<T, false, false><<<cut_blocks, CUT_NT, 0, s>>>(a);
   }
   return cudaGetLastError();
 }
 
 template cudaError_t launch_mc<float>(const DevGrid<float>&, const DevTape&, const float*, float*,
-                                      const Cols&, const DevTable&, unsigned*, unsigned*, cudaStream_t, bool, bool,
-                                      bool);
+                                      const Cols&, const DevTable&, unsigned*, unsigned*, cudaStream_t, bool, bool);
 template cudaError_t launch_mc<double>(const DevGrid<double>&, const DevTape&, const double*, double*,
-                                       const Cols&, const DevTable&, unsigned*, unsigned*, cudaStream_t, bool, bool,
-                                       bool);
+                                       const Cols&, const DevTable&, unsigned*, unsigned*, cudaStream_t, bool, bool);
 
 }  // namespace cci

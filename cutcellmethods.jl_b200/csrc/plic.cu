@@ -59,6 +59,7 @@ __device__ __forceinline__ PlaneFit<T, 2> cell_plane(const STape<T>& t, const De
 // tile's centroids when the body is a union of spheres.
 constexpr int PX = 32, PY = 8;
 static_assert(PX * PY == NT, "one cell per thread");
+static_assert(NT >= CC_TAPE_MAX_OPS, "prune_union: an op per thread");
 
 // Tile t's first cell, tiles numbered x fastest, from 32-bit quotients (a grid has far fewer
 // than 2^32 tiles: that would be 2^40 cells).
@@ -97,7 +98,7 @@ __device__ __forceinline__ STape<T> tile_tape(const STape<T>& t, const DevTape& 
     hi[a] = double(g.x0[a]) + (double(last) + 0.5) * double(g.d[a]);
   }
   cc_op* ops = reinterpret_cast<cc_op*>(smem + L.ops_off);
-  const int m = prune_union<T, 2>(t, tape.prunable, lo, hi, reinterpret_cast<double*>(smem + L.ls_off),
+  const int m = prune_union<T>(t, tape.prunable, lo, hi, reinterpret_cast<double*>(smem + L.ls_off),
                                   reinterpret_cast<double*>(smem + L.us_off), ops, count);
   STape<T> u = t;
   u.ops = ops;
@@ -381,8 +382,8 @@ struct OneSphere {  // sphere_at's arithmetic, the part that z does not change f
   }
 };
 
-// cell_plane (src/plic/plic.jl:72-88) from the body's dual at the centroid, with the cell's side
-// (cell_side). Where plane_side says that a valid plane misses the cell, gvf3 returns 1 or 0: its
+// cell_plane (src/plic/plic.jl:72-88) from the body's dual at the centroid, with the cell's side: plane_side's
+// of a valid plane, else closed (-1) or open (1) by the value's sign. Where plane_side says that a valid plane misses the cell, gvf3 returns 1 or 0: its
 // alpha is then beyond s or below 0 by far more than the few roundings of its sums.
 template <class T, bool MX>
 __device__ __forceinline__ PlaneFit<T, 3> plane_of(const Dual<T, 3>& r, T h, int& side) {
@@ -473,8 +474,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : (MODE == SPHERES || M
   int m = 0;
   if constexpr (MODE == SPHERES || MODE == SMOOTH) {
     const RowBox<T> box(g, tape.scale, i0, ni, j, k0, nk);
-    float low, up;
-    m = prune_warp<T>(t, MODE, tape.scale, box.lo, box.hi, box.mag, list, low, up);
+    m = prune_warp<T>(t, MODE, tape.scale, box.lo, box.hi, box.mag, list);
   }
   const bool in = lane < ni;
   const T x = centroid_coord(g.x0[0], g.d[0], i0 + lane), y = centroid_coord(g.x0[1], g.d[1], j);
@@ -830,14 +830,14 @@ __global__ void __launch_bounds__(NT) calc_volume_z_kernel(const DevGrid<T> g, c
       }
       int m = 0;
       if constexpr (MODE == SPHERES || MODE == SMOOTH) {
-        float lo[3], hi[3], mag = 0.0f, low, up;
+        float lo[3], hi[3], mag = 0.0f;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
           lo[a] = bound_f32(g.x0[a] + (T(c0[a]) + T(0.5)) * g.d[a], tape.scale);
           hi[a] = bound_f32(g.x0[a] + (T(c0[a] + ce[a] - 1) + T(0.5)) * g.d[a], tape.scale);
           mag += fabsf(bound_f32(g.x0[a], tape.scale)) + float(g.n[a]) * bound_f32(g.d[a], tape.scale);
         }
-        m = prune_warp<T>(t, MODE, tape.scale, lo, hi, mag, list, low, up);
+        m = prune_warp<T>(t, MODE, tape.scale, lo, hi, mag, list);
       }
       // cells near enough to need their plane are listed, then taken on full warps
       const bool in = lane % VX < ce[0] && lane / VX < ce[1];
