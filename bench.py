@@ -535,12 +535,12 @@ def sizes_block(args, dev, cc, sizes=(256, 200, 500)):
 
 def traffic_per_update(n):
     """DRAM bytes of one Float32 update of the CSG workload, from one ncu capture of the fill and
-    cut-band kernels at 256^3 (fill 1.7377 GB written + 3.9 MB read; cut 21.3 MB for 99,771 cut
+    cut-band kernels at 256^3 (fill 1.7249 GB written + 0.6 MB read; cut 19.0 MB for 99,771 cut
     cells), scaled by cells (x8 per doubling of n for the fill, x4 for the cut band's surface)."""
     if n < 64:
         return None
     s = n / 256.0
-    return (1.7377e9 + 3.9e6) * s ** 3 + 21.3e6 * s ** 2
+    return (1.7249e9 + 0.6e6) * s ** 3 + 19.0e6 * s ** 2
 
 
 # Per-cell counts of the PLIC Float32 update (fit + resolve pass) on the 64-sphere union. Warp
@@ -566,7 +566,7 @@ def plic_rooflines(cells, ms, peak_gbs, bytes_per_cell=46):
     return {"hbm_frac": hbm, "fp32_pipe_frac": fp32, "issue_frac": issue,
             "bound": max((("hbm", hbm), ("fp32 pipe", fp32), ("instruction issue", issue)), key=lambda x: x[1])[0],
             "fp32_flops_per_cell": PLIC_F32_FLOPS_PER_CELL, "warp_instructions_per_cell": PLIC_F32_WARP_INSTS_PER_CELL,
-            "counts_source": "ncu: instructions at 512^3, flops at 256^3 scaled (profiles/plic_fit_resolve_f32.md)"}
+            "counts_source": "ncu: instructions at 512^3, flops at 256^3 scaled"}
 
 
 def plic_block(args, dev, cc):

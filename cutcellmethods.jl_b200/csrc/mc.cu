@@ -577,6 +577,7 @@ long long device_sms() {
 //   Float64, all by TMA              512^3 4744 4397 4238 4090 4225    256^3 579 555 540 531 558
 //                                    192 x 160 x 129 field 164 152 154 150 148    -> 11
 //   Float64, some by the threads     404^3 2347 2379 2408 2463 2585    -> 31
+//     (updates at most 31, 19 and 11: 301^3 1285 1296 1323, 203^3 437 441 442, 330 x 250 x 90 324 333 334)
 int deepest_pencil(bool f64, bool all_tma) { return f64 ? (all_tma ? 11 : KZ) : (all_tma ? 19 : 15); }
 
 int pencil_slices(long long n0, long long n1, long long n2, bool f64, int deepest) {

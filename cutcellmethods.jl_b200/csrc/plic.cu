@@ -444,13 +444,14 @@ __device__ __forceinline__ void clip_crossed(const CrossedCell<T>* cells, int n,
 // that each store covers whole sectors. A cell's faces are written here too, one-sided: of a cell that
 // its plane misses, all open or all closed; a crossed cell's are clipped from a list, full warps at a
 // time. plic_resolve_kernel then joins the two sides. (A face pass that read every cell's side and
-// resolved all six faces through shared memory took as long as the fit.) Near both its bounds: 85% of
-// the issue slots and 4.6 TB/s of stores. Boxes of 8 x 4 and 16 x 2 columns keep fewer spheres (1.3 and
-// 1.6 instead of 2.0 at 512^3) but their stores cost more: 1.44 and 1.41 against 1.33 ms. CTAs per SM: 4
-// at Float32 (3: 1.36 ms), at Float64 2 with spheres (3: 2.46 against 2.38 ms), else 3 (CSG body at
-// 150 x 97 x 131: 101 against 111 us).
-// Update at 512^3, 64 spheres, kernels, by that change: Float32 2.50 -> 1.43 ms, Float64 3.92 -> 2.50, mixed 2.75 -> 1.55;
-// a smooth blob at 256^3 714 -> 455 us; a CSG body at 150 x 97 x 131, Float64, 281 -> 112 us.
+// resolved all six faces through shared memory took as long as the fit.) Near both its bounds: 5.6 TB/s
+// of stores (512^3 Float32, 64 spheres: 6.26 GB in 1.11 ms) and 84% of the issue slots (256^3). Boxes of 8 x 4
+// and 16 x 2 columns keep fewer spheres (1.3 and 1.6 instead of 2.0 at 512^3), but their stores cost 8% and 6% more.
+// CTAs per SM, updates at 512^3: at Float32 4 (3: 2% slower; mixed, whose SPHERES and SMOOTH forms spill a
+// little there, 4 against 3: spheres 1385 and 1413 us, CSG body 2507 and 2538, smooth blob 2558 and 2531), at Float64 2
+// with spheres (3: 3% slower), else 3 (2: 10% slower, CSG body at 150 x 97 x 131).
+// Updates, before (a fit on duals pruned per CTA, a pass over every face) and now: 512^3, 64 spheres, Float32 3.27 ->
+// 1.22 ms, Float64 5.10 -> 2.38, mixed 3.61 -> 1.39; a smooth blob at 256^3 Float32 now 427 us.
 template <class T, bool MX, int MODE>
 __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : (MODE == SPHERES || MODE == SMOOTH ? 2 : 3))
     plic_fit_z_kernel(const DevGrid<T> g, const DevTape tape, const Cols cols, T* __restrict__ normals,
