@@ -325,7 +325,8 @@ struct cc_batch {
   int max_tape = 0;
   std::vector<int> tape_off;
   unsigned long long* counter = nullptr;
-  long long total_tiles = 0;
+  long long total_tiles = 0;   // of the work list as it is laid out: tiles, or strips (warp_tiles)
+  long long config_tiles = -1;  // tiles and leaf chunks of the configuration's own sizes; -1 before a layout
   cudaStream_t stream = nullptr;
   cudaEvent_t in_ready = nullptr, done = nullptr;
   bool pending = false;
@@ -416,7 +417,7 @@ cc_status build_layout(cc_batch* b) {
   std::vector<BatchItem> dev(b->items.size());
   size_t off = 0;
   int max_tape = 0;
-  long long tiles = 0;
+  long long tiles = 0, config_tiles = 0;
   const int ty = b->cfg.tile_y;
   // sizes first, so the staging buffer is grown once
   std::vector<size_t> sz(b->items.size());
@@ -471,6 +472,7 @@ cc_status build_layout(cc_batch* b) {
       if (txs > 0x7fffffffLL) return fail(CC_TOO_LARGE, "grid too wide for the batch's tiles");
       d.tiles_x = int(txs);
       tiles += txs * tys;
+      config_tiles += (d.n0 + b->cfg.tile_x - 1) / b->cfg.tile_x * tys;
     } else {
       d.n0 = h.t.nleaves;
       d.x0[0] = h.t.x0[0]; d.x0[1] = h.t.x0[1];
@@ -478,6 +480,7 @@ cc_status build_layout(cc_batch* b) {
       d.level = h.t.level;
       d.coord = h.t.coord;
       tiles += (d.n0 + nt - 1) / nt;
+      config_tiles += (d.n0 + b->cfg.threads - 1) / b->cfg.threads;
     }
   }
   b->tapes_bytes = off;
@@ -496,6 +499,7 @@ cc_status build_layout(cc_batch* b) {
     const cudaError_t e = cudaMemcpy(b->items_dev, dev.data(), ib, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_fail(e, "batch items");
   }
+  b->config_tiles = config_tiles;
   b->layout_ok = true;
   return CC_OK;
 }
@@ -588,6 +592,7 @@ cc_status add_item(cc_batch* b, HostItem&& it, const cc_optape* body, int32_t* i
   if (st != CC_OK) return st;
   b->items.push_back(std::move(it));
   b->layout_ok = false;
+  b->config_tiles = -1;
   b->graph_ok = false;
   if (item) *item = int32_t(b->items.size() - 1);
   return CC_OK;
@@ -695,9 +700,10 @@ cc_status cc_batch_set_config(cc_batch* b, const cc_batch_config* cfg) {
   cc_status st = check_config(cfg);
   if (st != CC_OK) return st;
   if ((st = wait_pending(b)) != CC_OK) return st;
-  const bool layout = cfg->tile_x != b->cfg.tile_x || cfg->tile_y != b->cfg.tile_y || cfg->threads != b->cfg.threads ||
-                      (cfg->band_percent > 0) != (b->cfg.band_percent > 0);  // strips or tiles (warp_tiles)
+  const bool tiles = cfg->tile_x != b->cfg.tile_x || cfg->tile_y != b->cfg.tile_y || cfg->threads != b->cfg.threads;
+  const bool layout = tiles || (cfg->band_percent > 0) != (b->cfg.band_percent > 0);  // strips or tiles (warp_tiles)
   b->cfg = *cfg;
+  if (tiles) b->config_tiles = -1;
   if (layout) b->layout_ok = false;
   b->graph_ok = false;
   return CC_OK;
@@ -712,7 +718,7 @@ cc_status cc_batch_get_config(const cc_batch* b, cc_batch_config* cfg) {
 cc_status cc_batch_info(const cc_batch* b, int64_t* n_items, int64_t* total_tiles) {
   if (!b) return fail(CC_BAD_ARG, "null batch");
   if (n_items) *n_items = int64_t(b->items.size());
-  if (total_tiles) *total_tiles = b->layout_ok ? b->total_tiles : -1;
+  if (total_tiles) *total_tiles = b->config_tiles;
   return CC_OK;
 }
 

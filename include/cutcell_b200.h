@@ -375,7 +375,8 @@ cc_status cc_batch_add_ms_tree(cc_batch* b, const cc_tree* t, const cc_optape* b
 cc_status cc_batch_set_body(cc_batch* b, int32_t item, const cc_optape* body);
 cc_status cc_batch_set_config(cc_batch* b, const cc_batch_config* cfg);
 cc_status cc_batch_get_config(const cc_batch* b, cc_batch_config* cfg);
-/* Items, and the work list's tiles for the current configuration (-1 before the first run). */
+/* Items, and the work list's tiles for the current configuration (-1 before the first run): tiles of tile_x x
+ * tile_y cells and chunks of `threads` leaves, also where warps take them in strips of 32 cells. */
 cc_status cc_batch_info(const cc_batch* b, int64_t* n_items, int64_t* total_tiles);
 /* Run every update, ordered after the work already on `stream` and before what follows it. */
 cc_status cc_batch_run(cc_batch* b, void* stream);
