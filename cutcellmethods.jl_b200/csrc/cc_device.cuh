@@ -757,19 +757,34 @@ __device__ __forceinline__ float bound_f32(T v, double scale) {
   if constexpr (sizeof(T) == 8) return float(v * scale);
   else return v;
 }
+// A sphere's centre and radius, the same. The scale is 1 almost always, and multiplying by it all the same
+// cost calc_volume at 512^3 Float64 1% more than the test does (245 us without either, 250 with, 253).
+template <class T>
+__device__ __forceinline__ void bound_sphere(const T* __restrict__ p, double scale, float o[4]) {
+  T c[4];
+  ldq(p, c);
+  if constexpr (sizeof(T) == 8) {
+    if (scale != 1.0) {
+#pragma unroll
+      for (int a = 0; a < 4; ++a) c[a] = c[a] * scale;
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < 4; ++a) o[a] = float(c[a]);
+}
 template <class T, bool INDEX = false>
 __device__ __forceinline__ int prune_warp(const STape<T>& t, int mode, double scale, const float lo[3], const float hi[3],
                                           float mag, unsigned* out) {
   const int lane = threadIdx.x & 31, n = t.n_ops;
   const float big = __int_as_float(0x7f800000);
   auto bounds = [&](int i, float& l, float& u) {
-    T c[4];
-    ldq(t.p + t.ops[i].poff, c);
-    const float r = bound_f32(c[3], scale);
+    float c[4];
+    bound_sphere(t.p + t.ops[i].poff, scale, c);
+    const float r = c[3];
     float dmin2 = 0.0f, dmax2 = 0.0f, m = mag + fabsf(r);
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      const float ca = bound_f32(c[a], scale);
+      const float ca = c[a];
       const float below = lo[a] - ca, above = ca - hi[a];
       const float dn = fmaxf(fmaxf(below, above), 0.0f), dx = fmaxf(fabsf(below), fabsf(above));
       dmin2 += dn * dn;

@@ -48,17 +48,17 @@ struct DevTape {
 };
 
 // The tape as prune_warp may bound it over a grid, in every 3D pass that prunes. Its bounds are Float32 and
-// square distances, so Float64 lengths are first taken times `scale` (exact). A union of spheres stays prunable
-// while T's own squares are normal over the grid: `mag`, the size of its coordinates, within 2^-48..2^60 at
-// Float32 (below, the roots of T's squares err by up to 2^-73, near the bounds' margin of 2^-18 mag; above, squares
-// overflow) and within 2^-480..2^480 at Float64. Outside, it is evaluated whole like any other body.
+// square distances, which holds while `mag`, the size of the grid's coordinates, is within 2^-48..2^60: below, the
+// roots of Float32 squares err by up to 2^-73, near the bounds' margin of 2^-18 mag; above, they overflow. Float64
+// lengths outside are first taken times `scale`, which is exact and brings mag near 1, as far as Float64's own
+// squares are normal. A union of spheres on any other grid is evaluated whole like any other body.
 template <class T>
 DevTape in_bounds_range(DevTape tape, const DevGrid<T>& g) {
   double mag = 0;
   for (int a = 0; a < 3; ++a) mag += std::fabs(double(g.x0[a])) + double(g.n[a]) * double(g.d[a]);
-  const bool f64 = sizeof(T) == 8;
-  if (!(mag >= (f64 ? 0x1p-480 : 0x1p-48) && mag <= (f64 ? 0x1p480 : 0x1p60))) tape.prunable = 0;
-  else if (f64) tape.scale = std::ldexp(1.0, -std::ilogb(mag));
+  if (mag >= 0x1p-48 && mag <= 0x1p60) return tape;
+  if (sizeof(T) == 8 && mag >= 0x1p-480 && mag <= 0x1p480) tape.scale = std::ldexp(1.0, -std::ilogb(mag));
+  else tape.prunable = 0;
   return tape;
 }
 

@@ -794,17 +794,17 @@ __global__ void __launch_bounds__(NT) calc_volume_z_kernel(const DevGrid<T> g, c
       }
       if constexpr (MODE == SPHERES) {
         float least = __int_as_float(0x7f800000);
-        bool known = true;
+        float probe = 0.0f;  // not a number once any distance is infinite or not one
         const float b[3] = {bound_f32(x[0], tape.scale), bound_f32(x[1], tape.scale), bound_f32(x[2], tape.scale)};
         for (int i = lane % share; i < t.n_ops; i += share) {
-          T c[4];
-          ldq(t.p + t.ops[i].poff, c);
-          const float d0 = b[0] - bound_f32(c[0], tape.scale), d1 = b[1] - bound_f32(c[1], tape.scale), d2 = b[2] - bound_f32(c[2], tape.scale);
-          const float u = sqrt_approx(d0 * d0 + d1 * d1 + d2 * d2) - bound_f32(c[3], tape.scale);
-          known = known && u - u == 0.0f;
+          float c[4];
+          bound_sphere(t.p + t.ops[i].poff, tape.scale, c);
+          const float d0 = b[0] - c[0], d1 = b[1] - c[1], d2 = b[2] - c[2];
+          const float u = sqrt_approx(d0 * d0 + d1 * d1 + d2 * d2) - c[3];
+          probe = __fmaf_rn(u, 0.0f, probe);
           least = fminf(least, u);
         }
-        v = known ? T(least) : qnan<T>();  // times the scale, as `beyond` is
+        v = probe == 0.0f ? T(least) : qnan<T>();  // times the scale, as `beyond` is
       } else {
         v = tape_eval<T, 3, T>(t, x);
       }
