@@ -210,6 +210,13 @@ int tape_select(const cc_optape* t) {
   return 1;
 }
 
+int tape_cost(const cc_optape* t) {
+  int c = 0;
+  for (int i = 0; i < t->n_ops; ++i)
+    c += (t->ops[i].opcode == CC_OP_TRIG || t->ops[i].opcode == CC_OP_STAR ? COSTLY : 1) + (t->ops[i].combine == CC_COMB_SMIN ? 1 : 0);
+  return c;
+}
+
 // A combinator takes one operand's value or a smooth blend whose gradient is a convex combination, so a
 // body's bounds are its primitives' largest. A sphere's and a box's gradient has length 1 (or none,
 // inside a box), a torus's at most its matrix's (Frobenius) norm, a plane's its normal's.
@@ -303,6 +310,7 @@ cc_status upload_tape(cc_handle* h, const cc_optape* t, int dim, cudaStream_t s,
   out->bytes_len = int(bytes);
   out->prunable = cci::tape_prunable(t);
   out->select = cci::tape_select(t);
+  out->cost = cci::tape_cost(t);
   return CC_OK;
 }
 

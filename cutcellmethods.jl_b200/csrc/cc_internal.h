@@ -42,9 +42,10 @@ struct DevTape {
   int n_params;
   int bytes_len;
   int prunable = 0;  // 1: a union (MIN) of spheres, 2: a smooth union (SMIN) of spheres; see prune_union, prune_warp
+  int cost = 0;      // of one evaluation, in plain primitives (tape_cost)
   int select = 0;    // no smooth minimum: value and gradient are one primitive's (tape_eval_select)
   int slab = 8;      // the 3D PLIC fit's pruning slab in cell layers (prune_slab)
-  double scale = 1;  // a power of two that brings the grid's lengths near 1 (in_bounds_range)
+  double scale = 1;  // a power of two that brings the grid's lengths into Float32's range (in_bounds_range)
 };
 
 // The tape as prune_warp may bound it over a grid, in every 3D pass that prunes. Its bounds are Float32 and
@@ -157,6 +158,10 @@ size_t pack_tape(const cc_optape* t, int dim, unsigned char* out, int* n_params)
 size_t tape_pack_capacity();
 int tape_prunable(const cc_optape* t);
 int tape_select(const cc_optape* t);
+// The cost of evaluating a tape once, in spheres: a smooth minimum counts as another one, a primitive of sines,
+// cosines or an angle as COSTLY.
+constexpr int COSTLY = 1 << 16;
+int tape_cost(const cc_optape* t);
 
 // Release the contour a marching-squares handle holds (ms_mesh.cu).
 void free_ms_mesh(cc_handle* h);

@@ -3,7 +3,7 @@
 //
 // Grid: a warp per strip of 32 cells by a few rows samples its nodes from the op-tape and builds its cells
 // from them (the reference's _sample_nodes_kernel!, src/marching_squares/cache.jl:67-70, and
-// _nodal_cells_kernel!, :75-78, in one pass). Tree: one thread per leaf samples its four lattice corners
+// _nodal_cells_kernel!, :75-78, in one pass), or, where that does not pay (strips_pay), two passes. Tree: one thread per leaf samples its four lattice corners
 // and builds its moments from exactly those (_leaf_cells_kernel!, :129-137).
 #include <cstdint>
 #include <type_traits>
@@ -25,8 +25,8 @@ constexpr int NT = 256;
 constexpr int GRID_NT = 128;  // four warps, each with its own strips
 
 // SAMPLE: phi is written from the tape; else it holds the nodal values. I: the grid's index type. A strip per
-// warp, strips numbered x fastest. Sampling and cells used to be two kernels with phi in between: 2000 x 1500
-// Float32 43 -> 32 us; 200 x 200 Float64, bound by one cut cell's latency, 6.3 -> 6.5 us with one launch less.
+// warp, strips numbered x fastest. Against the two passes (strips_pay): 2000 x 1500 Float32, one circle, 43 -> 32 us;
+// 200 x 200 Float64, bound by one cut cell's latency, 6.3 -> 6.5 us with one launch less.
 template <class T, bool MX, bool SAMPLE, class I>
 __global__ void __launch_bounds__(GRID_NT, sizeof(T) == 4 ? 8 : 4) ms_grid_kernel(const DevGrid<T> g, const DevTape tape, T* phi, const Cols cols,
                                                           int ty) {
@@ -45,6 +45,52 @@ __global__ void __launch_bounds__(GRID_NT, sizeof(T) == 4 ? 8 : 4) ms_grid_kerne
     const unsigned long long sy = nsx * nsy < (1ull << 32) ? unsigned(s) / unsigned(nsx) : s / nsx;
     ms_strip<T, MX, SAMPLE, I>(t, g.x0[0], g.x0[1], g.d[0], g.d[1], n0, n1, I((s - sy * nsx) * STRIP), I(sy * ty), ty,
                                own, phi, cols);
+  }
+}
+
+// (i, j) of item v of an n0-wide box: a 32-bit quotient where the box has fewer than 2^32 items
+// (every grid that fits a device), else 64-bit.
+__device__ __forceinline__ void split2(long long v, long long n0, bool small, long long& i, long long& j) {
+  if (small) {
+    const unsigned q = unsigned(v) / unsigned(n0);
+    j = q;
+    i = (long long)(unsigned(v) - q * unsigned(n0));
+  } else {
+    j = v / n0;
+    i = v - j * n0;
+  }
+}
+
+// The two passes by nodes and by cells, a thread each, where strips do not pay (strips_pay).
+template <class T>
+__global__ void __launch_bounds__(NT) ms_sample_kernel(const DevGrid<T> g, const DevTape tape, T* phi) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const STape<T> t = load_tape<T>(tape.bytes, tape.n_ops, tape.n_params, smem);
+  __syncthreads();
+  const long long nx = g.n[0] + 1, ny = g.n[1] + 1, total = nx * ny;
+  const bool small = total + (long long)gridDim.x * NT < (1LL << 32);
+  for (long long v = blockIdx.x * (long long)NT + threadIdx.x; v < total; v += (long long)gridDim.x * NT) {
+    long long i, j;
+    split2(v, nx, small, i, j);
+    const T x[2] = {node_coord(g.x0[0], g.d[0], i), node_coord(g.x0[1], g.d[1], j)};
+    phi[v] = tape_eval<T, 2, T>(t, x);
+  }
+}
+
+template <class T, bool MX>
+__global__ void __launch_bounds__(NT) ms_cells_kernel(const DevGrid<T> g, const T* __restrict__ phi, const Cols cols) {
+  const long long n0 = g.n[0], n1 = g.n[1], nx = n0 + 1, total = n0 * n1;
+  const T cs[2] = {g.d[0], g.d[1]};
+  const bool small = total + (long long)gridDim.x * NT < (1LL << 32);
+  for (long long ci = blockIdx.x * (long long)NT + threadIdx.x; ci < total; ci += (long long)gridDim.x * NT) {
+    long long i, j;
+    split2(ci, n0, small, i, j);
+    const T xa = node_coord(g.x0[0], g.d[0], i), xb = node_coord(g.x0[0], g.d[0], i + 1);
+    const T ya = node_coord(g.x0[1], g.d[1], j), yb = node_coord(g.x0[1], g.d[1], j + 1);
+    const T nd[4][2] = {{xa, ya}, {xb, ya}, {xb, yb}, {xa, yb}};
+    const long long b = i + nx * j;
+    const T ph[4] = {phi[b], phi[b + 1], phi[b + nx + 1], phi[b + nx]};
+    ms_cell<T, MX>(nd, ph, cs, cols, ci);
   }
 }
 
@@ -71,9 +117,44 @@ int grid_blocks(long long work) {
 
 namespace cci {
 
+namespace {
+template <class T>
+bool strips_pay(const DevGrid<T>& g, const DevTape& tape, bool sample) {
+  // Strips fuse the two passes and store whole sectors, but sample an extra node row and column each, evaluate
+  // nodes in groups per lane, and idle the lanes beyond a narrow grid's end. Two passes / strips, us:
+  //   one circle: Float32 500^2 21 / 18, 1000^2 22 / 19, 4096^2 231 / 152; Float64 21 / 18, 37 / 33, 422 / 297; 1 x 40000
+  //     (whole calls) Float32 35 / 41, Float64 37 / 49, 33 x 20000 4% and 8% slower, 40 x 20000 level
+  //   union of 8: Float32 1000^2 34 / 26, 4096^2 412 / 269, 100 x 20000 57 / 50; Float64 55 / 55, 674 / 546, 91 / 97
+  //   of 20: Float32 500^2 25 / 31, 1000^2 56 / 48, 4096^2 724 / 540; Float64 1400^2 145 / 159, 3000^2 602 / 600
+  //   of 100: Float32 500^2 62 / 123, 1000^2 185 / 184, 2047 x 1500 530 / 479; Float64 4096^2 3909 / 4762
+  //   a star curve, 1400^2: Float32 48 / 50, Float64 91 / 106
+  //   given values (whole calls), 1000^2, 2047 x 1500, 4096^2: Float32 41 / 42, 63 / 67, 224 / 219, Float64 57 / 59, 107 / 109, 436 / 391
+  const long long cells = g.n[0] * g.n[1], lanes = (g.n[0] + STRIP - 1) / STRIP * STRIP;
+  const bool full = 10 * g.n[0] >= 9 * lanes;
+  if (!sample) return full && cells >= 6000000;
+  if (tape.cost <= 2) return cells <= 16384 || 10 * g.n[0] >= 6 * lanes;
+  if (tape.cost >= COSTLY || cells < 1000000) return false;
+  if (sizeof(T) == 4) return tape.cost <= 8 ? 4 * g.n[0] >= 3 * lanes : full && (tape.cost <= 20 || cells >= 3000000);
+  return full && (tape.cost <= 8 || (tape.cost <= 20 && cells >= 9000000));
+}
+}  // namespace
+
 template <class T>
 cudaError_t launch_ms(const DevGrid<T>& g, const DevTape& tape, const T* phi_in, T* phi_out,
                       const Cols& cols, cudaStream_t s, bool mixed) {
+  if (!strips_pay<T>(g, tape, phi_in == nullptr)) {
+    const T* phi = phi_in;
+    if (!phi_in) {
+      const int sm = ((tape.bytes_len + 15) / 16) * 16;
+      const cudaError_t e = allow_dynamic_smem(ms_sample_kernel<T>, sm);
+      if (e != cudaSuccess) return e;
+      ms_sample_kernel<T><<<grid_blocks((g.n[0] + 1) * (g.n[1] + 1)), NT, sm, s>>>(g, tape, phi_out);
+      phi = phi_out;
+    }
+    if (mixed && sizeof(T) == 4) ms_cells_kernel<T, true><<<grid_blocks(g.n[0] * g.n[1]), NT, 0, s>>>(g, phi, cols);
+    else ms_cells_kernel<T, false><<<grid_blocks(g.n[0] * g.n[1]), NT, 0, s>>>(g, phi, cols);
+    return cudaGetLastError();
+  }
   // eight rows per strip, fewer while that leaves SMs without warps (the strip's one extra node row
   // then costs more, latency less)
   int ty = 8;
