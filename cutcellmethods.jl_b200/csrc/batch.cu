@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(256) ms_batch_kernel(const BatchArgs A) {
 }
 
 // The same work list with a warp, not a CTA, per tile: for tiles of whole 32-cell strips, without band
-// compaction, while a warp's tape and strip fit its share of shared memory (warp_tiles). The work list then
+// compaction, while a warp's tape and strip fit its share of shared memory (warps_can), where it pays (warps_pay). The work list then
 // holds strips of 32 x tile_y cells, whatever tile_x, and chunks of 32 leaves. 35% of the CTA kernel's instructions. What
 // bounds it is where the stores go: with each warp popping for itself the tiles in flight were spread so
 // far that their half-written sectors left L2 (DRAM reads of 165-300 MB, 700-900 us); side by side in a CTA
@@ -325,7 +325,8 @@ struct cc_batch {
   int max_tape = 0;
   std::vector<int> tape_off;
   unsigned long long* counter = nullptr;
-  long long total_tiles = 0;   // of the work list as it is laid out: tiles, or strips (warp_tiles)
+  bool warp_tiles = false;     // laid out as strips, a warp each (warps_can, warps_pay)
+  long long total_tiles = 0;   // of the work list as it is laid out: tiles, or strips
   long long config_tiles = -1;  // tiles and leaf chunks of the configuration's own sizes; -1 before a layout
   cudaStream_t stream = nullptr;
   cudaEvent_t in_ready = nullptr, done = nullptr;
@@ -396,13 +397,56 @@ int smem_of(const cc_batch* b) {
   return tape_smem_of(b) + (nodes + 15) / 16 * 16 + list;
 }
 
-// Whether the current config runs a warp per tile: whole strips, no band compaction, and at most 64 KB of
+// Whether the current config can run a warp per tile: whole strips, no band compaction, and at most 64 KB of
 // tapes and strips per CTA (then at least three CTAs of eight warps fit an SM).
 int warp_smem_of(const cc_batch* b) {
   return tape_smem_of(b) + (b->prec == CC_F64 ? strip_bytes<double>(b->cfg.tile_y) : strip_bytes<float>(b->cfg.tile_y));
 }
-bool warp_tiles(const cc_batch* b) {
+bool warps_can(const cc_batch* b) {
   return b->cfg.tile_x % STRIP == 0 && b->cfg.band_percent == 0 && (b->cfg.threads / 32) * warp_smem_of(b) <= 64 * 1024;
+}
+// Whether they also pay. A warp works through its strip's nodes 32 lanes at a time where a CTA takes a tile's at
+// once, so few strips leave the chip waiting for them. Compared is the longest chain of node evaluations either
+// way: rounds of resident CTAs times evaluations per thread. Strips are quicker where the CTA kernel's chain is at
+// least half of theirs (at Float64 in tiles of one strip 0.4), by up to 3 times (three grids of 2000^2, a union of
+// 100, 32 x 8 tiles, 2 CTAs an SM: CTAs 7012 us, strips 2390), and slower below, by up to 2.9 (20 grids of 64^2, the
+// same body, the default shape: 138 and 351 us). Curves of sines, cosines and angles run slower in strips except where
+// the chain favours them and a tile is one strip (a star curve, 2000^2, Float64: 32 x 4 tiles 266 and 225 us,
+// 64 x 8 tiles 189 and 234).
+bool warps_pay(const cc_batch* b) {
+  const bool f64 = b->prec == CC_F64;
+  const long long tx = b->cfg.tile_x, ty = b->cfg.tile_y, nt = b->cfg.threads, ch = b->cfg.chunk, wp = nt / 32;
+  const int nb = f64 ? 3 : 5;  // ms_strip's nodes per lane and pass
+  long long strips = 0, tiles = 0, strip_evals = 0, tile_evals = 0, costly = 0;
+  for (const HostItem& h : b->items) {
+    long long s, t, se = 4, te = 4;
+    if (h.kind == 0) {
+      const long long rows = (h.g.n[1] + ty - 1) / ty, high = (h.g.n[1] < ty ? h.g.n[1] : ty) + 1;
+      s = (h.g.n[0] + STRIP - 1) / STRIP * rows;
+      t = (h.g.n[0] + tx - 1) / tx * rows;
+      se = (STRIP_X * high + 32 * nb - 1) / (32 * nb) * nb;
+      // a tile wider than its grid takes the time of a full one, but a grid of a few columns or rows
+      te = h.g.n[0] > 16 && h.g.n[1] >= ty ? ((tx + 1) * (ty + 1) + nt - 1) / nt : (((h.g.n[0] < tx ? h.g.n[0] : tx) + 1) * high + nt - 1) / nt;
+    } else {
+      s = (h.t.nleaves + 31) / 32;
+      t = (h.t.nleaves + nt - 1) / nt;
+    }
+    strips += s;
+    tiles += t;
+    strip_evals = se > strip_evals ? se : strip_evals;
+    tile_evals = te > tile_evals ? te : tile_evals;
+    const cc_optape body = tape_of(h);
+    if (cci::tape_cost(&body) >= cci::COSTLY && h.kind == 0) costly += s;
+  }
+  if (strips == 0) return false;
+  auto rounds = [&](long long work, long long per_pop, long long ctas) {
+    const long long pops = (work + per_pop - 1) / per_pop;
+    return (pops + 148 * ctas - 1) / (148 * ctas) * ch;
+  };
+  const long long most = (f64 ? 16 : 24) / wp, ctas = b->cfg.ctas_per_sm < most ? b->cfg.ctas_per_sm : (most > 0 ? most : 1);
+  const double chain = double(rounds(tiles, ch, b->cfg.ctas_per_sm) * tile_evals) / double(rounds(strips, ch * wp, ctas) * strip_evals);
+  if (2 * costly > strips) return tx == STRIP && chain >= (f64 ? 0.6 : 1.0);
+  return chain >= (f64 && tx == STRIP ? 0.4 : 0.5);
 }
 
 // Pack every body into the staging buffer and lay the work list out for the current config.
@@ -431,7 +475,8 @@ cc_status build_layout(cc_batch* b) {
   }
   if (off > 0x7fffffffULL) return fail(CC_TOO_LARGE, "the batch's op-tapes exceed 2 GiB");
   b->max_tape = max_tape;
-  const int tx = warp_tiles(b) ? STRIP : b->cfg.tile_x, nt = warp_tiles(b) ? 32 : b->cfg.threads;  // nt: leaves per chunk
+  b->warp_tiles = warps_can(b) && warps_pay(b);
+  const int tx = b->warp_tiles ? STRIP : b->cfg.tile_x, nt = b->warp_tiles ? 32 : b->cfg.threads;  // nt: leaves per chunk
   if (off > b->tapes_host_cap) {
     if (b->tapes_host) cudaFreeHost(b->tapes_host);
     b->tapes_host = nullptr;
@@ -521,7 +566,7 @@ cudaError_t issue(cc_batch* b, cudaStream_t s) {
   a.tape_smem = tape_smem_of(b);
   a.warp_smem = warp_smem_of(b);
   a.band = b->cfg.band_percent;
-  const bool warps = warp_tiles(b);
+  const bool warps = b->warp_tiles;
   const int sm = warps ? (b->cfg.threads / 32) * a.warp_smem : smem_of(b);
   const int grid = 148 * b->cfg.ctas_per_sm;
   const int nt = b->cfg.threads;
@@ -546,7 +591,7 @@ cudaError_t issue(cc_batch* b, cudaStream_t s) {
 // The kernel's dynamic shared-memory limit for the current layout (set outside any capture).
 cudaError_t prepare_kernel(const cc_batch* b) {
   const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  if (warp_tiles(b)) {
+  if (b->warp_tiles) {
     const int wsm = (b->cfg.threads / 32) * warp_smem_of(b);
     if (b->prec == CC_F64) return cudaFuncSetAttribute(ms_batch_warp_kernel<double, false>, at, wsm);
     if (b->prec == CC_MIXED) return cudaFuncSetAttribute(ms_batch_warp_kernel<float, true>, at, wsm);
@@ -701,7 +746,9 @@ cc_status cc_batch_set_config(cc_batch* b, const cc_batch_config* cfg) {
   if (st != CC_OK) return st;
   if ((st = wait_pending(b)) != CC_OK) return st;
   const bool tiles = cfg->tile_x != b->cfg.tile_x || cfg->tile_y != b->cfg.tile_y || cfg->threads != b->cfg.threads;
-  const bool layout = tiles || (cfg->band_percent > 0) != (b->cfg.band_percent > 0);  // strips or tiles (warp_tiles)
+  // strips or tiles: the rule takes these too (warps_can, warps_pay)
+  const bool layout = tiles || (cfg->band_percent > 0) != (b->cfg.band_percent > 0) || cfg->ctas_per_sm != b->cfg.ctas_per_sm ||
+                      cfg->chunk != b->cfg.chunk;
   b->cfg = *cfg;
   if (tiles) b->config_tiles = -1;
   if (layout) b->layout_ok = false;
