@@ -606,7 +606,8 @@ __global__ void __launch_bounds__(NT) plic_resolve_kernel(const DevGrid<T> g, T*
       for (int d = 0; d < 2; ++d) {
         const long long at = c + step[d + 1];
         const int r = int(at & 15);  // the same for every lane
-        if (c >= total - step[d + 1]) {  // no cell beyond: not the padding's bytes, which would list them all
+        // no cell beyond: the padding's bytes would list them all (400 x 400 x 1 without a body: 41 -> 36 us a call)
+        if (c >= total - step[d + 1]) {
 #pragma unroll
           for (int q = 0; q < 4; ++q) yz[d][q] = o[q];
         } else if (r == 0) {
