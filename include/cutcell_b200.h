@@ -194,6 +194,8 @@ typedef struct {
 } cc_mc_tile;
 
 /* ---- handle -------------------------------------------------------------- */
+/* A handle holds one staging buffer and one set of scratch and results: calls on one handle from several
+ * threads are the caller's to keep apart (a handle each, or a lock). */
 typedef struct cc_handle cc_handle;
 
 /* Create the library-side state for one cache (the reference's
