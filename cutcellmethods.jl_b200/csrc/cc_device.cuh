@@ -751,35 +751,28 @@ __device__ __forceinline__ float sqrt_approx(float x) {
   asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
-// A length as the bounds take it: Float64 ones times the tape's power of two.
-template <class T>
+// A length, or a sphere's centre and radius, as the bounds take them: Float64 ones times the tape's power of two,
+// which is 1 without SCALED.
+template <class T, bool SCALED>
 __device__ __forceinline__ float bound_f32(T v, double scale) {
-  if constexpr (sizeof(T) == 8) return float(v * scale);
-  else return v;
+  if constexpr (sizeof(T) == 8 && SCALED) return float(v * scale);
+  else return float(v);
 }
-// A sphere's centre and radius, the same. The scale is 1 almost always, and multiplying by it all the same
-// cost calc_volume at 512^3 Float64 1% more than the test does (245 us without either, 250 with, 253).
-template <class T>
+template <class T, bool SCALED>
 __device__ __forceinline__ void bound_sphere(const T* __restrict__ p, double scale, float o[4]) {
   T c[4];
   ldq(p, c);
-  if constexpr (sizeof(T) == 8) {
-    if (scale != 1.0) {
 #pragma unroll
-      for (int a = 0; a < 4; ++a) c[a] = c[a] * scale;
-    }
-  }
-#pragma unroll
-  for (int a = 0; a < 4; ++a) o[a] = float(c[a]);
+  for (int a = 0; a < 4; ++a) o[a] = bound_f32<T, SCALED>(c[a], scale);
 }
-template <class T, bool INDEX = false>
+template <class T, bool INDEX = false, bool SCALED = true>
 __device__ __forceinline__ int prune_warp(const STape<T>& t, int mode, double scale, const float lo[3], const float hi[3],
                                           float mag, unsigned* out) {
   const int lane = threadIdx.x & 31, n = t.n_ops;
   const float big = __int_as_float(0x7f800000);
   auto bounds = [&](int i, float& l, float& u) {
     float c[4];
-    bound_sphere(t.p + t.ops[i].poff, scale, c);
+    bound_sphere<T, SCALED>(t.p + t.ops[i].poff, scale, c);
     const float r = c[3];
     float dmin2 = 0.0f, dmax2 = 0.0f, m = mag + fabsf(r);
 #pragma unroll
@@ -831,7 +824,7 @@ __device__ __forceinline__ int prune_warp(const STape<T>& t, int mode, double sc
       before = __shfl_up_sync(0xffffffffu, before, 1);
       before = fminf(lane == 0 ? big : before, running);
       if (i < n) {
-        const float k = bound_f32(t.p[t.ops[i].kparam], scale);
+        const float k = bound_f32<T, SCALED>(t.p[t.ops[i].kparam], scale);
         const float km = 0x1p-18f * (fabsf(k) + fabsf(before) + fabsf(l) + mag);
         keep = i == 0 || !(l >= before + k + km);
       }

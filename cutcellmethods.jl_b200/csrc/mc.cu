@@ -205,9 +205,9 @@ __global__ void __launch_bounds__(Tile<T>::NT, Tile<T>::MINB) mc_fill_kernel(con
         float lo[3], hi[3], mag = 0.0f;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-          lo[a] = bound_f32(node_coord(A.g.x0[a], A.g.d[a], first[a]), A.tape.scale);
-          hi[a] = bound_f32(node_coord(A.g.x0[a], A.g.d[a], last[a]), A.tape.scale);
-          mag += fabsf(bound_f32(A.g.x0[a], A.tape.scale)) + float(A.g.n[a]) * bound_f32(A.g.d[a], A.tape.scale);
+          lo[a] = bound_f32<T, true>(node_coord(A.g.x0[a], A.g.d[a], first[a]), A.tape.scale);
+          hi[a] = bound_f32<T, true>(node_coord(A.g.x0[a], A.g.d[a], last[a]), A.tape.scale);
+          mag += fabsf(bound_f32<T, true>(A.g.x0[a], A.tape.scale)) + float(A.g.n[a]) * bound_f32<T, true>(A.g.d[a], A.tape.scale);
         }
         unsigned* list = reinterpret_cast<unsigned*>(kept + n);
         const int m = prune_warp<T, true>(tape, A.tape.prunable, A.tape.scale, lo, hi, mag, list);

@@ -274,9 +274,9 @@ struct RowBox {
     mag = 0.0f;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      lo[a] = bound_f32(g.x0[a] + (T(first[a]) + T(0.5)) * g.d[a], scale);
-      hi[a] = bound_f32(g.x0[a] + (T(last[a]) + T(0.5)) * g.d[a], scale);
-      mag += fabsf(bound_f32(g.x0[a], scale)) + float(g.n[a]) * bound_f32(g.d[a], scale);
+      lo[a] = bound_f32<T, true>(g.x0[a] + (T(first[a]) + T(0.5)) * g.d[a], scale);
+      hi[a] = bound_f32<T, true>(g.x0[a] + (T(last[a]) + T(0.5)) * g.d[a], scale);
+      mag += fabsf(bound_f32<T, true>(g.x0[a], scale)) + float(g.n[a]) * bound_f32<T, true>(g.d[a], scale);
     }
   }
 };
@@ -757,7 +757,9 @@ __global__ void __launch_bounds__(NT) calc_volume_kernel(const DevGrid<T> g, con
 // on all lanes, and listing the near cells, took the 256^3 time from 244 to 103 us.
 constexpr int VX = 8, VY = 4, VZ = 8;
 
-template <class T, bool MX, int MODE>
+// SCALED: lengths are brought into Float32's range first (in_bounds_range); its own instantiation, since the
+// multiplications made 512^3 Float64 3% slower.
+template <class T, bool MX, int MODE, bool SCALED>
 __global__ void __launch_bounds__(NT) calc_volume_z_kernel(const DevGrid<T> g, const DevTape tape, double* partial,
                                                            T thr, T beyond, int group) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -799,10 +801,10 @@ __global__ void __launch_bounds__(NT) calc_volume_z_kernel(const DevGrid<T> g, c
       if constexpr (MODE == SPHERES) {
         float least = __int_as_float(0x7f800000);
         float probe = 0.0f;  // not a number once any distance is infinite or not one
-        const float b[3] = {bound_f32(x[0], tape.scale), bound_f32(x[1], tape.scale), bound_f32(x[2], tape.scale)};
+        const float b[3] = {bound_f32<T, SCALED>(x[0], tape.scale), bound_f32<T, SCALED>(x[1], tape.scale), bound_f32<T, SCALED>(x[2], tape.scale)};
         for (int i = lane % share; i < t.n_ops; i += share) {
           float c[4];
-          bound_sphere(t.p + t.ops[i].poff, tape.scale, c);
+          bound_sphere<T, SCALED>(t.p + t.ops[i].poff, tape.scale, c);
           const float d0 = b[0] - c[0], d1 = b[1] - c[1], d2 = b[2] - c[2];
           const float u = sqrt_approx(d0 * d0 + d1 * d1 + d2 * d2) - c[3];
           probe = __fmaf_rn(u, 0.0f, probe);
@@ -838,11 +840,11 @@ __global__ void __launch_bounds__(NT) calc_volume_z_kernel(const DevGrid<T> g, c
         float lo[3], hi[3], mag = 0.0f;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-          lo[a] = bound_f32(g.x0[a] + (T(c0[a]) + T(0.5)) * g.d[a], tape.scale);
-          hi[a] = bound_f32(g.x0[a] + (T(c0[a] + ce[a] - 1) + T(0.5)) * g.d[a], tape.scale);
-          mag += fabsf(bound_f32(g.x0[a], tape.scale)) + float(g.n[a]) * bound_f32(g.d[a], tape.scale);
+          lo[a] = bound_f32<T, SCALED>(g.x0[a] + (T(c0[a]) + T(0.5)) * g.d[a], tape.scale);
+          hi[a] = bound_f32<T, SCALED>(g.x0[a] + (T(c0[a] + ce[a] - 1) + T(0.5)) * g.d[a], tape.scale);
+          mag += fabsf(bound_f32<T, SCALED>(g.x0[a], tape.scale)) + float(g.n[a]) * bound_f32<T, SCALED>(g.d[a], tape.scale);
         }
-        m = prune_warp<T>(t, MODE, tape.scale, lo, hi, mag, list);
+        m = prune_warp<T, false, SCALED>(t, MODE, tape.scale, lo, hi, mag, list);
       }
       // cells near enough to need their plane are listed, then taken on full warps
       const bool in = lane % VX < ce[0] && lane / VX < ce[1];
@@ -1126,9 +1128,11 @@ cudaError_t launch_volume_z(const DevGrid<T>& g, const DevTape& tape, const Tape
     return cudaGetLastError();
   };
   if constexpr (sizeof(T) == 4) {
-    if (mx) return run(calc_volume_z_kernel<T, true, MODE>);
+    if (mx) return run(calc_volume_z_kernel<T, true, MODE, false>);
+  } else if constexpr (MODE == SPHERES || MODE == SMOOTH) {
+    if (tape.scale != 1.0) return run(calc_volume_z_kernel<T, false, MODE, true>);
   }
-  return run(calc_volume_z_kernel<T, false, MODE>);
+  return run(calc_volume_z_kernel<T, false, MODE, false>);
 }
 
 }  // namespace
